@@ -1,0 +1,300 @@
+"""The work that is timed when the library is made faster, as its users call it.
+
+Decode side: a runtime holds the 2-bit linears of a layer and runs them for T tokens at a time: one token per step for a
+single request, a handful for speculative decoding, tens for continuous batching, hundreds and thousands for prefill.
+Encode side: a quantizer takes weight matrices to trellis codes, with or without a Hessian, and prepares the Hessian.
+Widths are those of the repository's benchmark configurations and tests (hidden 12288, intermediate 28672, K/V 1024).
+
+A case is a dict with a "kind":
+  linear   one linear: input transform, product, output transform               n_in, n_out, tokens
+  qkv      RMSNorm + input transform, q projection, FP8 k and v projections     hidden, kv, tokens
+  mlp      RMSNorm + input transform, gate|up, SiLU, down, residual add         hidden, inter, tokens
+  encode   fp32 matrix -> tiles -> two-pass Viterbi -> packed kernel layout     rows, cols
+  group    one or two linears with a shared Hessian factor through LDLQ         rows, rows2, cols
+  hessian  damping and rotation of a Hessian, then its block LDL factor         n
+"""
+import math
+
+import torch
+
+import __graft_entry__
+
+pkg = __graft_entry__.load_package()
+codec, linear, synth = pkg.codec, pkg.linear, pkg.synth
+
+EPS = 1e-5
+
+
+def listed():
+    return [
+        # smallest decode call: a narrow linear for one token; launches and host work decide
+        {"name": "linear-3584x1536-t1", "kind": "linear", "n_in": 3584, "n_out": 1536, "tokens": 1},
+        # the widest single product of a decode step (stacked gate|up rows) for one token
+        {"name": "linear-12288x57344-t1", "kind": "linear", "n_in": 12288, "n_out": 57344, "tokens": 1},
+        # MLP half of a single-request decode step
+        {"name": "mlp-t1", "kind": "mlp", "hidden": 12288, "inter": 28672, "tokens": 1},
+        # projections in front of attention for a few speculated tokens
+        {"name": "qkv-t5", "kind": "qkv", "hidden": 12288, "kv": 1024, "tokens": 5},
+        # a ragged small batch
+        {"name": "mlp-t13", "kind": "mlp", "hidden": 12288, "inter": 28672, "tokens": 13},
+        # continuous batching
+        {"name": "mlp-t64", "kind": "mlp", "hidden": 12288, "inter": 28672, "tokens": 64},
+        # a short prompt through the down projection, not a multiple of any tile
+        {"name": "linear-28672x12288-t200", "kind": "linear", "n_in": 28672, "n_out": 12288, "tokens": 200},
+        # prefill chunk
+        {"name": "mlp-t2048", "kind": "mlp", "hidden": 12288, "inter": 28672, "tokens": 2048},
+        # smallest encode: one 256 x 256 matrix
+        {"name": "encode-256x256", "kind": "encode", "rows": 256, "cols": 256},
+        # a row slab of a q projection without a Hessian
+        {"name": "encode-2048x12288", "kind": "encode", "rows": 2048, "cols": 12288},
+        # a group of two linears with error feedback
+        {"name": "group-4096+1024x4096", "kind": "group", "rows": 4096, "rows2": 1024, "cols": 4096},
+        # the Hessian of a hidden-width group
+        {"name": "hessian-12288", "kind": "hessian", "n": 12288},
+    ]
+
+
+# Widths K * 2^p with a carried Hadamard order K; the fused epilogues carry K = 1, 12, 28.
+_WIDTHS = [384, 512, 640, 768, 896, 1024, 1536, 2048, 2560, 3072, 3584, 4096, 5120, 6144, 7168, 8192, 10240, 12288, 14336,
+           16384, 20480, 24576, 28672]
+_EPILOGUE_WIDTHS = [w for w in _WIDTHS if w not in (640, 2560, 5120, 10240, 20480)]
+
+
+def _log(rng, lo, hi):
+    return int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))
+
+
+def draw(rng):
+    kind = rng.choice(["linear", "linear", "linear", "qkv", "mlp", "mlp", "encode", "group", "hessian"])
+    if kind == "linear":
+        tokens = _log(rng, 1, 2048)
+        n_in, n_out = rng.choice(_WIDTHS), rng.choice(_WIDTHS + [40960, 57344])
+        return {"kind": kind, "n_in": n_in, "n_out": n_out, "tokens": tokens}
+    if kind == "qkv":
+        hidden = rng.choice([w for w in _EPILOGUE_WIDTHS if 2048 <= w <= 16384])
+        return {"kind": kind, "hidden": hidden, "kv": rng.choice([256, 512, 1024, 2048]), "tokens": _log(rng, 1, 600)}
+    if kind == "mlp":
+        hidden = rng.choice([w for w in _EPILOGUE_WIDTHS if 2048 <= w <= 12288])
+        inter = rng.choice([w for w in _EPILOGUE_WIDTHS if 4096 <= w <= 28672])
+        return {"kind": kind, "hidden": hidden, "inter": inter, "tokens": _log(rng, 1, 2048)}
+    if kind == "encode":
+        return {"kind": kind, "rows": 32 * _log(rng, 2, 64), "cols": 32 * _log(rng, 4, 384)}
+    if kind == "group":
+        widths = [w for w in _WIDTHS if w <= 3072]
+        return {"kind": kind, "rows": rng.choice(widths), "rows2": rng.choice([0] + widths),
+                "cols": rng.choice([w for w in widths if w % 128 == 0])}
+    return {"kind": kind, "n": rng.choice([w for w in _WIDTHS if 1024 <= w <= 10240])}
+
+
+# ---------------------------------------------------------------------------------------------------------- state
+
+class _State:
+    pass
+
+
+def _bf(gen, *shape, scale=1.0):
+    return (scale * torch.randn(*shape, generator=gen, device="cuda")).to(torch.bfloat16)
+
+
+def _signs(gen, n, scale=1.0):
+    return (torch.randint(0, 2, (n,), generator=gen, device="cuda") * 2 - 1).float() * scale
+
+
+def _linear(gen, lut, n_in, n_out, su=None):
+    """A linear with uniform random codes; its scale keeps outputs at the size of the inputs."""
+    trellis = torch.randint(-32768, 32768, ((n_out // 16) * (n_in // 16) * 32,), generator=gen, device="cuda",
+                            dtype=torch.int16)
+    return linear.Matrix(trellis, _signs(gen, n_in) if su is None else su, _signs(gen, n_out, n_in ** -0.5), lut, n_in, n_out)
+
+
+def _splits(w, tokens):
+    """K-splits a runtime gives a product: the tensor-core kernel's rule where the batch takes it, whole rows for prefill,
+    else enough work items for every SM."""
+    if tokens > 512:
+        return 1
+    if tokens > 1 and linear.batch_uses_tc(w.n_in, w.n_out, tokens):
+        return linear.tc_splits(w.n_out)
+    want = 1 if w.n_out > 16384 else (2 if w.n_out > 8192 else 4)
+    return min(want, w.n_in // 32)
+
+
+def _products(s, names, tokens):
+    """K-splits, z and (prefill) the dense scratch for the products of the named linears."""
+    mats = [getattr(s, n) for n in names]
+    s.splits = {n: _splits(getattr(s, n), tokens) for n in names}
+    s.z = torch.empty(max(s.splits[n] * tokens * m.n_out for n, m in zip(names, mats)), dtype=torch.float32, device="cuda")
+    s.dense = torch.empty(max(m.n_in * m.n_out for m in mats), dtype=torch.bfloat16, device="cuda") if tokens > 512 else None
+    s.scratch = torch.empty(max(max(m.n_in, m.n_out) for m in mats), dtype=torch.float32, device="cuda")
+
+
+def _multiply(s, name, x, tokens):
+    w = getattr(s, name)
+    if tokens > 512:
+        linear.qtip_multiply_prefill(w, x, s.z, w.n_out, tokens, s.dense)
+    elif tokens == 1:
+        linear.qtip_multiply(w, x, s.z, w.n_out, s.splits[name], 1)
+    else:
+        linear.qtip_multiply_batch(w, x, s.z, w.n_out, s.splits[name], tokens)
+
+
+def _hessian(gen, n):
+    """Second moments of activations with a rank-64 correlated part."""
+    tokens = max(2048, n // 2)
+    x = torch.randn(tokens, n, generator=gen, device="cuda")
+    x += torch.randn(tokens, 64, generator=gen, device="cuda") @ (torch.randn(64, n, generator=gen, device="cuda") / 8.0)
+    x = x.to(torch.bfloat16)
+    return torch.mm(x.T, x, out_dtype=torch.float32) / tokens
+
+
+def prepare(case, seed):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(1000003 * int(seed) + 17)
+    tlut = synth.seeded_tlut(1)
+    s = _State()
+    s.case, kind = case, case["kind"]
+    bf16 = dict(dtype=torch.bfloat16, device="cuda")
+    if kind == "linear":
+        n_in, n_out, t = case["n_in"], case["n_out"], case["tokens"]
+        s.w = _linear(gen, linear.runtime_lut(tlut), n_in, n_out)
+        s.x = _bf(gen, t, n_in)
+        s.rotated, s.y = torch.empty(t, n_in, **bf16), torch.empty(t, n_out, **bf16)
+        _products(s, ["w"], t)
+    elif kind == "qkv":
+        hidden, kv, t = case["hidden"], case["kv"], case["tokens"]
+        s.q = _linear(gen, linear.runtime_lut(tlut), hidden, hidden)
+        s.k8, s.v8 = (torch.randint(0, 256, (kv, hidden), generator=gen, device="cuda", dtype=torch.uint8) for _ in range(2))
+        for w in (s.k8, s.v8):
+            w[(w & 127) == 127] = 0  # no NaN codes
+        s.scale8 = (1 + torch.arange(kv, device="cuda") % 7).float() / 4096.0
+        s.state, s.norm = _bf(gen, t, hidden), (1.0 + 0.05 * torch.randn(hidden, generator=gen, device="cuda")).to(torch.bfloat16)
+        s.u, s.xn, s.yq = (torch.empty(t, hidden, **bf16) for _ in range(3))
+        s.yk, s.yv = (torch.empty(t, kv, **bf16) for _ in range(2))
+        _products(s, ["q"], t)
+        if t >= 8:
+            s.dense8 = torch.empty(kv * hidden, **bf16)
+            s.z8 = torch.empty(linear.fp8_splits(hidden, kv, t) * t * kv, dtype=torch.float32, device="cuda")
+    elif kind == "mlp":
+        hidden, inter, t = case["hidden"], case["inter"], case["tokens"]
+        lut = linear.runtime_lut(tlut)
+        s.gate_up = _linear(gen, lut, hidden, 2 * inter)
+        s.down = _linear(gen, lut, inter, hidden)
+        s.sv_gate, s.sv_up = s.gate_up.sv[:inter].contiguous(), s.gate_up.sv[inter:].contiguous()
+        s.state, s.norm = _bf(gen, t, hidden), (1.0 + 0.05 * torch.randn(hidden, generator=gen, device="cuda")).to(torch.bfloat16)
+        s.u = torch.empty(t, hidden, **bf16)
+        s.h, s.ud = torch.empty(t, inter, **bf16), torch.empty(t, inter, **bf16)
+        s.next_norm, s.next_su = torch.ones(hidden, **bf16), _signs(gen, hidden)
+        s.next_u = torch.empty(t, hidden, **bf16)
+        _products(s, ["gate_up", "down"], t)
+    elif kind == "encode":
+        m, n = case["rows"], case["cols"]
+        s.lut, _ = codec.device_lut(tlut)
+        s.W = torch.randn(m, n, generator=gen, device="cuda")
+        s.tiles = (m // 16) * (n // 16)
+        s.X = torch.empty(s.tiles, 256, dtype=torch.float32, device="cuda")
+        s.states = torch.empty(s.tiles, 128, dtype=torch.int16, device="cuda")
+        s.packed, s.trellis = (torch.empty(s.tiles, 32, dtype=torch.int16, device="cuda") for _ in range(2))
+        s.ws = codec.quantize_workspace(min(max(s.tiles, 8), 2 * 4608))
+    elif kind == "group":
+        m, m2, n = case["rows"], case["rows2"], case["cols"]
+        s.lut, s.lut_rms = codec.device_lut(tlut)
+        s.su = _signs(gen, n)
+        s.svs = [_signs(gen, r) for r in (m, m2) if r]
+        s.weights = [0.02 * torch.randn(r, n, generator=gen, device="cuda") for r in (m, m2) if r]
+        s.HR, s.creg = codec.rotate_hessian_fused(_hessian(gen, n), s.su)
+        s.L = codec.block_ldl(s.HR)
+        s.ws = codec.Workspace(pkg.lib().raw("qtip_quantize_group_workspace_bytes")(n, m + m2, max(m, m2)))
+    else:
+        n = case["n"]
+        s.H, s.su = _hessian(gen, n), _signs(gen, n)
+        s.ws = codec.Workspace(pkg.lib().raw("qtip_block_ldl_workspace_bytes")(n))
+    return s
+
+
+# ------------------------------------------------------------------------------------------------------------ run
+
+def run(s):
+    case, kind = s.case, s.case["kind"]
+    if kind == "linear":
+        t = case["tokens"]
+        if t == 1:
+            linear.qtip_forward(s.w, s.x, s.y, s.scratch, s.rotated, s.z, False, s.splits["w"])
+        else:
+            linear.qtip_prepare(s.w, s.x, s.scratch, s.rotated, t)
+            _multiply(s, "w", s.rotated, t)
+            linear.qtip_finish(s.w, s.z, s.y, s.scratch, False, s.splits["w"], t)
+        return s.y
+    if kind == "qkv":
+        hidden, kv, t = case["hidden"], case["kv"], case["tokens"]
+        linear.input_transform(s.state, s.norm, EPS, s.q.su, hidden, t, s.u, s.xn)
+        _multiply(s, "q", s.u, t)
+        linear.qtip_finish(s.q, s.z, s.yq, s.scratch, False, s.splits["q"], t)
+        for w, y in ((s.k8, s.yk), (s.v8, s.yv)):
+            if t >= 8:
+                linear.fp8_forward_prefill(w, s.scale8, s.xn, y, hidden, kv, t, s.dense8, s.z8)
+            else:
+                linear.fp8_forward(w, s.scale8, s.xn, y, hidden, kv, t)
+        return {"q": s.yq, "k": s.yk, "v": s.yv}
+    if kind == "mlp":
+        hidden, inter, t = case["hidden"], case["inter"], case["tokens"]
+        linear.input_transform(s.state, s.norm, EPS, s.gate_up.su, hidden, t, s.u)
+        _multiply(s, "gate_up", s.u, t)
+        linear.output_gateup(s.z, s.splits["gate_up"], t, s.sv_gate, s.sv_up, inter, s.h)
+        linear.qtip_prepare(s.down, s.h, s.scratch, s.ud, t)
+        _multiply(s, "down", s.ud, t)
+        linear.output_residual_input(s.z, s.splits["down"], t, s.down.sv, hidden, s.state, s.next_norm, EPS, s.next_su, s.next_u)
+        return {"h": s.h, "state": s.state, "next_u": s.next_u}
+    if kind == "encode":
+        codec.tiles_from_matrix(s.W, s.X)
+        codec.quantize_tiles(s.X, s.lut, states=s.states, workspace=s.ws, want_hat=False)
+        codec.pack_trellis(s.states, s.packed)
+        return codec.swizzle_for_kernel(s.packed, case["rows"], case["cols"], s.trellis)
+    if kind == "group":
+        # the call rotates the weights in place: it is given a copy, as the caller's checkpoint loader would hand one over
+        outs, shared = codec.quantize_group([w.clone() for w in s.weights], s.HR, s.L, s.su, s.svs, s.creg, s.lut, s.lut_rms,
+                                            workspace=s.ws)
+        return {"linears": [[o["trellis"], o["SV"], o["proxy"], o["proxy_rot_reg"]] for o in outs], "hatWT": shared["hatWT"]}
+    HR, creg = codec.rotate_hessian_fused(s.H.clone(), s.su)  # rotates in place
+    return {"HR": HR, "creg": creg, "L": codec.block_ldl(HR, workspace=s.ws)}
+
+
+# ------------------------------------------------------------------------------------------- work and tolerance
+
+_STATES, _PASSES = 65536, 2
+
+
+def work(case):
+    kind = case["kind"]
+    if kind == "linear":
+        a, b, t = case["n_in"], case["n_out"], case["tokens"]
+        return {"bytes": a * b // 4 + 4 * (a + b) + 4096 + 2 * t * (a + b), "flops": 2 * t * a * b}
+    if kind == "qkv":
+        h, kv, t = case["hidden"], case["kv"], case["tokens"]
+        return {"bytes": h * h // 4 + 2 * kv * h + 10 * h + 4 * kv + 4096 + 2 * t * (2 * h + 2 * kv), "flops": 2 * t * h * (h + 2 * kv)}
+    if kind == "mlp":
+        h, f, t = case["hidden"], case["inter"], case["tokens"]
+        # codes, signs and norms; the state in and out, the next rotated input and the activated row (its own result)
+        return {"bytes": 3 * h * f // 4 + 4 * (4 * h + 3 * f) + 4096 + 2 * t * (3 * h + f), "flops": 6 * t * h * f}
+    if kind in ("encode", "group"):
+        m, n = case["rows"] + case.get("rows2", 0), case["cols"]
+        # per weight and pass: 128 steps x 65,536 states over 256 weights; an add, two multiply-adds and a comparison each
+        flops = m * n * _STATES // 2 * _PASSES * 6
+        if kind == "encode":
+            return {"bytes": 4 * m * n + m * n // 4, "flops": flops}
+        return {"bytes": 8 * m * n + m * n // 4 + 4 * n * n + 2 * n * n, "flops": flops + m * n * n}
+    n = case["n"]
+    return {"bytes": 4 * n * n * 3, "flops": n ** 3 // 3}
+
+
+def tolerance(case):
+    """About four times what the same path shows when its sums are taken in another order (K-splits of the products; one
+    rounding of the Hessian's entries, which its factor amplifies)."""
+    kind = case["kind"]
+    if kind == "encode":
+        return "exact"
+    if kind == "group":
+        return {"rel": 1e-5, "max": 1e-3, "differ": 0.0}
+    if kind == "hessian":
+        return {"rel": 1e-4, "max": 2e-3}
+    if kind == "mlp":  # three bf16 roundings in a chain, the products of gate and up among them: 3e-3 seen
+        return {"rel": 1.2e-2, "max": 0.08}
+    return {"rel": 1.5e-3, "max": 0.04}
