@@ -257,6 +257,107 @@ def run(s):
     return {"HR": HR, "creg": creg, "L": codec.block_ldl(HR, workspace=s.ws)}
 
 
+# ------------------------------------------------------------------------------------------------ the same in 64 bits
+
+def _codebook64():
+    """The 1,024 decoded pairs (entry = sign << 9 | index, the sign turns the first value) in the runtime's bf16."""
+    t = torch.from_numpy(synth.seeded_tlut(1)).to("cuda").double()
+    t = torch.cat([t, t * torch.tensor([-1.0, 1.0], dtype=torch.float64, device="cuda")])
+    return t.float().to(torch.bfloat16).double()
+
+
+def _product64(w, x):
+    """x . What^T with the weights decoded from the 32 x 32 blocks of codes: word c of tile (i1, j1) of a block stands at
+    4 c + 2 j1 + i1; state k of a word is 16 bits of it and of its successor from bit 4 k on, weights (8 (k & 1) + c / 4,
+    8 (k >> 1) + 2 (c & 3) and + 1) of the tile."""
+    book, n2 = _codebook64(), w.n_in // 32
+    codes = w.trellis.view(w.n_out // 32, n2, 32, 2, 2)  # block-row, block, c, j1, i1
+    z = torch.empty(x.shape[0], w.n_out, dtype=torch.float64, device="cuda")
+    step = max(1, (1 << 27) // (w.n_in * 32))
+    for r0 in range(0, w.n_out // 32, step):
+        own = codes[r0:r0 + step].int() & 0xffff
+        both = own.long() << 16 | own.roll(-1, dims=2).long()
+        k = torch.arange(4, device="cuda")
+        s = (both.unsqueeze(-1) >> (16 - 4 * k)) & 0xffff
+        v = book[((s * (s + 1)) >> 6) & 1023].view(-1, n2, 8, 4, 2, 2, 2, 2, 2)  # row block, block, c/4, c&3, j1, i1, k>>1, k&1, pair
+        rows = v.permute(0, 5, 7, 2, 1, 4, 6, 3, 8).reshape(-1, w.n_in)
+        z[:, 32 * r0:32 * r0 + rows.shape[0]] = x @ rows.T
+    return z
+
+
+def _factor64(n):
+    """The Hadamard factor of order 1, 12, 20 (Paley I) or 28 (Paley II) that a width carries."""
+    K = next((k for k in (28, 20, 12) if n % k == 0 and (n // k) & (n // k - 1) == 0), 1)
+    H = torch.ones(K, K, dtype=torch.float64)
+    if K in (12, 20):
+        q = K - 1
+        squares = {x * x % q for x in range(1, q)}
+        for i in range(K):
+            for j in range(K):
+                d = (j - i) % q
+                H[i, j] = (1 if j == 0 else -1) if i == 0 else (1 if j == 0 or d == 0 or d not in squares else -1)
+    elif K == 28:
+        squares = {x * x % 13 for x in range(1, 13)}
+        c = torch.ones(14, 14, dtype=torch.float64)  # symmetric conference matrix of order 14, its diagonal apart
+        for i in range(1, 14):
+            for j in range(1, 14):
+                c[i, j] = 1 if (j - i) % 13 in squares else -1
+        c.fill_diagonal_(0)
+        e = torch.eye(14, dtype=torch.float64)
+        H = torch.cat([torch.cat([c + e, c - e], 1), torch.cat([c - e, -c - e], 1)])
+    return H.to("cuda")
+
+
+def _rotate64(x, transpose):
+    """Rows of x by (factor (x) Walsh-Hadamard) / sqrt(n), the factor transposed on the input side."""
+    n = x.shape[-1]
+    H = _factor64(n)
+    y = torch.einsum("kr,tkp->trp" if transpose else "rk,tkp->trp", H, x.reshape(-1, H.shape[0], n // H.shape[0]))
+    h = 1
+    while h < y.shape[-1]:
+        a, b = y.reshape(-1, 2, h).unbind(1)
+        y = torch.stack([a + b, a - b], 1).reshape(y.shape)
+        h *= 2
+    return y.reshape(x.shape) / math.sqrt(n)
+
+
+def _rms64(x, w):
+    return x * torch.rsqrt((x * x).mean(-1, keepdim=True) + EPS) * w.double()
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind in ("encode", "group"):  # whole numbers, and values that follow from a search over states
+        return None
+    s = prepare(case, seed)
+    if kind == "linear":
+        return _rotate64(_product64(s.w, _rotate64(s.x.double() * s.w.su.double(), True)), False) * s.w.sv.double()
+    if kind == "qkv":
+        xn = _rms64(s.state.double(), s.norm)
+        q = _rotate64(_product64(s.q, _rotate64(xn * s.q.su.double(), True)), False) * s.q.sv.double()
+        k, v = (xn @ w.view(torch.float8_e4m3fn).double().T * s.scale8.double() for w in (s.k8, s.v8))
+        return {"q": q, "k": k, "v": v}
+    if kind == "mlp":
+        f = case["inter"]
+        z = _product64(s.gate_up, _rotate64(_rms64(s.state.double(), s.norm) * s.gate_up.su.double(), True))
+        g, u = (_rotate64(z[:, i * f:(i + 1) * f], False) * sv.double() for i, sv in ((0, s.sv_gate), (1, s.sv_up)))
+        h = g * torch.sigmoid(g) * u
+        z = _product64(s.down, _rotate64(h * s.down.su.double(), True))
+        state = s.state.double() + _rotate64(z, False) * s.down.sv.double()
+        return {"h": h, "state": state, "next_u": _rotate64(_rms64(state, s.next_norm) * s.next_su.double(), True)}
+    n = case["n"]
+    H, su = s.H.double(), s.su.double()
+    creg = 0.01 * float(H.diagonal().mean())
+    HR = (H + creg * torch.eye(n, dtype=torch.float64, device="cuda")) * su * su[:, None]
+    for _ in range(2):
+        HR = torch.cat([_rotate64(HR[:, i:i + 1024].T, True) for i in range(0, n, 1024)])
+    C = torch.linalg.cholesky((HR + HR.T) / 2)
+    blocks = torch.stack([C[i:i + 16, i:i + 16] for i in range(0, n, 16)])
+    L = torch.matmul(C.view(n, n // 16, 16).transpose(0, 1), torch.linalg.inv(blocks)).transpose(0, 1).reshape(n, n)
+    at = torch.arange(n, device="cuda") // 16
+    return {"HR": HR, "creg": creg, "L": L * (at[:, None] > at)}
+
+
 # ------------------------------------------------------------------------------------------- work and tolerance
 
 _STATES, _PASSES = 65536, 2
