@@ -5,13 +5,16 @@
 //
 // Method (same algebra as the reference): symmetrise in fp64, A = (H + H^T) / 2; Cholesky A = C C^T (lower); for every
 // 16-column block bj, Lb[:, bj] = C[:, bj] * inv(C[bj, bj]) below the diagonal block, zero on and above it.
-// The Cholesky is right-looking with 128-column panels:
-//   1. chol_diag_kernel   one CTA factors the 128 x 128 diagonal block in shared memory;
-//   2. chol_panel_kernel  rows below: x L11^T = a by forward substitution, 64 rows per CTA, L11 and the rows in shared
-//                         memory, four partial sums per row;
-//   3. chol_update_kernel trailing update C -= P P^T on the lower triangle: 128 x 128 tiles, 8 x 8 fp64 accumulators per
+// The Cholesky is right-looking with 128-column panels, two launches a panel:
+//   1. chol_panel_kernel  rows below the diagonal block: x L11^T = a, 64 rows per CTA held in registers, sixteen columns
+//                         at a time through the inverse of their diagonal block;
+//   2. chol_update_kernel trailing update C -= P P^T on the lower triangle: 128 x 128 tiles, 8 x 8 fp64 accumulators per
 //                         thread, the 128-deep panels streamed through shared memory in 16-column slices. This is where
-//                         the n^3 / 6 fused multiply-adds are: DFMA-issue bound (64 lanes per SM and clock).
+//                         the n^3 / 6 fused multiply-adds are: DFMA-issue bound (64 lanes per SM and clock). The CTA of
+//                         tile (0, 0) keeps its tile, which is the next diagonal block, in shared memory and factors it
+//                         there (chol_factor) while the other tiles are updated: the one serial stage of a panel is off
+//                         the critical path as long as the update takes longer than one factorisation.
+// The first diagonal block has a launch of its own (chol_first_kernel).
 // A non-positive pivot or a non-finite result sets a status word in the workspace (qtip_block_ldl_status); the
 // reference returns false in those cases.
 #include "common.cuh"
@@ -44,84 +47,165 @@ __global__ void ldl_symmetrise_kernel(const float* __restrict__ H, double* __res
   }
 }
 
-// Unblocked Cholesky of the kb x kb diagonal block at (k, k), one CTA, block held in shared memory (row stride kNb + 1).
-__global__ __launch_bounds__(256) void chol_diag_kernel(double* __restrict__ A, long n, long k, int kb, int* status) {
-  extern __shared__ double sm[];
-  const int ld = kNb + 1;
-  for (int idx = threadIdx.x; idx < kb * kb; idx += blockDim.x) {
-    const int i = idx / kb, j = idx - i * kb;
-    sm[i * ld + j] = j <= i ? A[(k + i) * n + k + j] : 0.0;
-  }
-  __syncthreads();
-  for (int j = 0; j < kb; ++j) {
-    // column j: every earlier column has already been subtracted from it (right-looking)
-    const double d = sm[j * ld + j];
-    __syncthreads();
-    const bool ok = d > 0.0;
-    if (!ok && threadIdx.x == 0) atomicOr(status, 1);
-    const double dj = ok ? sqrt(d) : 1.0;  // a failed pivot is reported; the factor is then meaningless but finite
-    for (int i = j + threadIdx.x; i < kb; i += blockDim.x) sm[i * ld + j] = (i == j) ? dj : sm[i * ld + j] / dj;
-    __syncthreads();
-    // trailing update of the block: a[i][c] -= a[i][j] a[c][j] for j < c <= i
-    const int rem = kb - j - 1;
-    for (int idx = threadIdx.x; idx < rem * rem; idx += blockDim.x) {
-      const int i = j + 1 + idx / rem, c = j + 1 + idx % rem;
-      if (c <= i) sm[i * ld + c] = fma(-sm[i * ld + j], sm[c * ld + j], sm[i * ld + c]);
+// Cholesky of a kb x kb block (kb a multiple of 16, at most 128) in shared memory, lower triangle, by 256 threads. Sixteen
+// columns at a time: one warp factors the 16 x 16 diagonal block with a row per lane in registers and inverts it (a column
+// per lane), then all warps take the rows below it through the inverse and update what is right of it. The inverses, which
+// the panel kernel and the final block scaling need as well, go to `inv` (256 values a block, row-major, zeros above the
+// diagonal).
+constexpr int kLd = kNb + 1;
+constexpr int kInvLd = 17;
+__device__ __forceinline__ void chol_factor(double* __restrict__ S, double* __restrict__ inv_s, int kb,
+                                            double* __restrict__ inv, int* status) {
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  for (int base = 0; base < kb; base += 16) {
+    if (tid < 32) {
+      const int i = tid & 15;
+      double a[16];
+#pragma unroll
+      for (int c = 0; c < 16; ++c) a[c] = c <= i ? S[(base + i) * kLd + base + c] : 0.0;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const double d = __shfl_sync(0xffffffffu, a[j], j);
+        const bool ok = d > 0.0;
+        if (!ok && tid == 0) atomicOr(status, 1);
+        const double dj = ok ? sqrt(d) : 1.0;  // a failed pivot is reported; the factor is then meaningless but finite
+        a[j] = i == j ? dj : a[j] / dj;
+#pragma unroll
+        for (int c = j + 1; c < 16; ++c) a[c] = fma(-a[j], __shfl_sync(0xffffffffu, a[j], c), a[c]);
+      }
+      double col[16];  // column i of the inverse
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        double t = r == i ? 1.0 : 0.0;
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+          if (q < r) t = fma(-__shfl_sync(0xffffffffu, a[q], r), col[q], t);
+        col[r] = t / __shfl_sync(0xffffffffu, a[r], r);
+      }
+      if (tid < 16) {
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          if (c <= i) S[(base + i) * kLd + base + c] = a[c];
+          inv_s[c * kInvLd + i] = col[c];
+          inv[(base / 16) * 256 + c * 16 + i] = col[c];
+        }
+      }
     }
     __syncthreads();
-  }
-  for (int idx = threadIdx.x; idx < kb * kb; idx += blockDim.x) {
-    const int i = idx / kb, j = idx - i * kb;
-    if (j <= i) A[(k + i) * n + k + j] = sm[i * ld + j];
+    // rows below: x = a inv^T
+    const int below = kb - base - 16;
+    double x[7];
+#pragma unroll
+    for (int a = 0; a < 7; ++a) {
+      const int r = ty + 16 * a;
+      double t = 0.0;
+      if (r < below) {
+#pragma unroll
+        for (int p = 0; p < 16; ++p) t = fma(S[(base + 16 + r) * kLd + base + p], inv_s[tx * kInvLd + p], t);
+      }
+      x[a] = t;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 7; ++a)
+      if (ty + 16 * a < below) S[(base + 16 + ty + 16 * a) * kLd + base + tx] = x[a];
+    __syncthreads();
+    // right of it: a[i][c] -= sum_p x[i][p] x[c][p], 16 x 16 blocks on and below the diagonal
+    for (int a = 0; 16 * a < below; ++a) {
+      double* row = S + (base + 16 + ty + 16 * a) * kLd + base;
+      double xi[16];
+#pragma unroll
+      for (int p = 0; p < 16; ++p) xi[p] = row[p];
+      for (int b = 0; b <= a; ++b) {
+        const double* xc = S + (base + 16 + tx + 16 * b) * kLd + base;
+        double t0 = 0.0, t1 = 0.0;
+#pragma unroll
+        for (int p = 0; p < 16; p += 2) t0 = fma(xi[p], xc[p], t0), t1 = fma(xi[p + 1], xc[p + 1], t1);
+        row[16 + tx + 16 * b] -= t0 + t1;  // above the diagonal of a diagonal block: never read
+      }
+    }
+    __syncthreads();
   }
 }
-
-// Rows r0 + [64 b, 64 b + 64): x L11^T = a, i.e. x[j] = (a[j] - sum_{p < j} x[p] L11[j][p]) / L11[j][j], one thread per
-// row. L11 (kb x kb) and the rows sit in shared memory; each thread keeps four running sums so that the fp64 adds of one
-// row do not form a single chain.
-constexpr int kPanelRows = 64;
-__global__ __launch_bounds__(kPanelRows) void chol_panel_kernel(double* __restrict__ A, long n, long k, int kb) {
-  extern __shared__ double sm[];
-  double* L11 = sm;                   // [kb][kNb + 1]
-  double* X = sm + kNb * (kNb + 1);   // [kPanelRows][kNb + 1]
-  const int ld = kNb + 1;
-  const long r0 = k + kb + long(blockIdx.x) * kPanelRows;
-  const int rows = int(min(long(kPanelRows), n - r0));
+__device__ __forceinline__ void chol_store(const double* __restrict__ S, double* __restrict__ A, long n, long k, int kb) {
   for (int idx = threadIdx.x; idx < kb * kb; idx += blockDim.x) {
     const int i = idx / kb, j = idx - i * kb;
-    L11[i * ld + j] = j <= i ? A[(k + i) * n + k + j] : 0.0;
+    if (j <= i) A[(k + i) * n + k + j] = S[i * kLd + j];
   }
-  for (int idx = threadIdx.x; idx < rows * kb; idx += blockDim.x) {
+}
+__global__ __launch_bounds__(256) void chol_first_kernel(double* __restrict__ A, long n, int kb, double* __restrict__ inv,
+                                                         int* status) {
+  extern __shared__ double sm[];
+  for (int idx = threadIdx.x; idx < kb * kb; idx += blockDim.x) {
     const int i = idx / kb, j = idx - i * kb;
-    X[i * ld + j] = A[(r0 + i) * n + k + j];
+    sm[i * kLd + j] = j <= i ? A[i * n + j] : 0.0;
   }
   __syncthreads();
-  if (int(threadIdx.x) < rows) {
-    double* x = X + threadIdx.x * ld;
-    for (int j = 0; j < kb; ++j) {
-      const double* l = L11 + j * ld;
-      double s0 = x[j], s1 = 0, s2 = 0, s3 = 0;
-      int p = 0;
-      for (; p + 4 <= j; p += 4) {
-        s0 = fma(-l[p], x[p], s0);
-        s1 = fma(-l[p + 1], x[p + 1], s1);
-        s2 = fma(-l[p + 2], x[p + 2], s2);
-        s3 = fma(-l[p + 3], x[p + 3], s3);
+  chol_factor(sm, sm + kNb * kLd, kb, inv, status);
+  chol_store(sm, A, n, 0, kb);
+}
+
+// Rows r0 + [64 b, 64 b + 64): x L11^T = a. Thread (ty, tx) holds rows ty + 16 a and columns tx + 16 j in registers. Sixteen
+// columns at a time: x_b = s_b inv_b^T from shared memory, then every later column block takes x_b L11[j][b]^T off.
+constexpr int kPanelRows = 64;
+__global__ __launch_bounds__(256) void chol_panel_kernel(double* __restrict__ A, long n, long k,
+                                                         const double* __restrict__ inv) {
+  extern __shared__ double sm[];
+  double* L11 = sm;                              // [kNb][kLd]
+  double* inv_s = L11 + kNb * kLd;               // [kNb / 16][16][kInvLd]
+  double* Y = inv_s + (kNb / 16) * 16 * kInvLd;  // [kPanelRows][kInvLd] right-hand side of the current block
+  double* X = Y + kPanelRows * kInvLd;           // [kPanelRows][kInvLd] its solution
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const long r0 = k + kNb + long(blockIdx.x) * kPanelRows;
+  const int rows = int(min(long(kPanelRows), n - r0));
+  double acc[4][8];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[a][j] = ty + 16 * a < rows ? A[(r0 + ty + 16 * a) * n + k + tx + 16 * j] : 0.0;
+  for (int i = ty; i < kNb; i += 16)
+    for (int j = tx; j <= i; j += 16) L11[i * kLd + j] = A[(k + i) * n + k + j];
+  for (int i = tid; i < kNb * 16; i += 256) inv_s[(i >> 4) * kInvLd + (i & 15)] = inv[i];
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a) Y[(ty + 16 * a) * kInvLd + tx] = acc[a][b];
+    __syncthreads();
+    double x[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int p = 0; p < 16; ++p) {
+      const double v = inv_s[(b * 16 + tx) * kInvLd + p];  // zero for p > tx
+#pragma unroll
+      for (int a = 0; a < 4; ++a) x[a] = fma(Y[(ty + 16 * a) * kInvLd + p], v, x[a]);
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) acc[a][b] = x[a], X[(ty + 16 * a) * kInvLd + tx] = x[a];
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < 16; ++p) {
+      double xr[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) xr[a] = X[(ty + 16 * a) * kInvLd + p];
+#pragma unroll
+      for (int j = b + 1; j < 8; ++j) {
+        const double l = L11[(tx + 16 * j) * kLd + 16 * b + p];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) acc[a][j] = fma(-xr[a], l, acc[a][j]);
       }
-      for (; p < j; ++p) s0 = fma(-l[p], x[p], s0);
-      x[j] = ((s0 + s1) + (s2 + s3)) / l[j];
     }
   }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < rows * kb; idx += blockDim.x) {
-    const int i = idx / kb, j = idx - i * kb;
-    A[(r0 + i) * n + k + j] = X[i * ld + j];
-  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (ty + 16 * a < rows) A[(r0 + ty + 16 * a) * n + k + tx + 16 * j] = acc[a][j];
 }
 
 // C[i][j] -= sum_p P[i][p] P[j][p] for the tile (ti, tj), tj <= ti, of the trailing matrix that starts at row / column
 // r0; P = A[r0.., k .. k + kb). 256 threads as 16 x 16, each 8 x 8 outputs at rows ty + 16 a and columns tx + 16 b.
-__global__ __launch_bounds__(256, 1) void chol_update_kernel(double* __restrict__ A, long n, long k, int kb, long r0) {
+// Tile (0, 0) is the next diagonal block: its CTA, the first of the launch, factors it at once.
+__global__ __launch_bounds__(256, 1) void chol_update_kernel(double* __restrict__ A, long n, long k, int kb, long r0,
+                                                             double* __restrict__ inv, int* status) {
   __shared__ double Pi[kKc][kTile + 2];
   __shared__ double Pj[kKc][kTile + 2];
   // linear block index -> (ti, tj) of the lower triangle
@@ -177,6 +261,21 @@ __global__ __launch_bounds__(256, 1) void chol_update_kernel(double* __restrict_
       __syncthreads();
     }
   }
+  if (t == 0) {
+    extern __shared__ double sm[];
+    const int kb2 = int(min(long(kNb), n - r0));
+#pragma unroll
+    for (int x = 0; x < 8; ++x)
+#pragma unroll
+      for (int y = 0; y < 8; ++y) {
+        const int i = ty + 16 * x, j = tx + 16 * y;
+        if (i < kb2 && j <= i) sm[i * kLd + j] = A[(r0 + i) * n + r0 + j] - acc[x][y];
+      }
+    __syncthreads();
+    chol_factor(sm, sm + kNb * kLd, kb2, inv, status);
+    chol_store(sm, A, n, r0, kb2);
+    return;
+  }
 #pragma unroll
   for (int x = 0; x < 8; ++x) {
     const long i = i0 + ty + 16 * x;
@@ -189,54 +288,39 @@ __global__ __launch_bounds__(256, 1) void chol_update_kernel(double* __restrict_
   }
 }
 
-// inv[b] = inverse of the lower-triangular 16 x 16 diagonal block b of C; thread c of a 16-thread group solves column c.
-__global__ void ldl_block_inverse_kernel(const double* __restrict__ A, long n, double* __restrict__ inv) {
-  const long b = long(blockIdx.x) * (blockDim.x / 16) + threadIdx.x / 16;
-  const int c = threadIdx.x & 15;
-  if (b * 16 >= n) return;
-  const double* D = A + (b * 16) * n + b * 16;
-  double col[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    double s = (i == c) ? 1.0 : 0.0;
-#pragma unroll
-    for (int p = 0; p < 16; ++p)
-      if (p < i) s = fma(-D[i * n + p], col[p], s);
-    col[i] = s / D[i * n + i];
-  }
-#pragma unroll
-  for (int i = 0; i < 16; ++i) inv[b * 256 + i * 16 + c] = col[i];
-}
-
 // L[r][16 bj + j] = sum_{p = j}^{15} C[r][16 bj + p] inv[bj][p][j] for bj < r / 16, zero on and above the diagonal
-// block. One thread per (row, column block); fp32 result, optionally the fp64 value beside it.
+// block. One thread per row of a column block, the block's inverse in shared memory (broadcast reads); fp32 result,
+// optionally the fp64 value beside it.
 __global__ __launch_bounds__(128) void ldl_finish_kernel(const double* __restrict__ A, const double* __restrict__ inv,
                                                          long n, float* __restrict__ L, double* __restrict__ L64,
                                                          int* status) {
-  const long nb = n / 16;
-  const long r = blockIdx.y;
-  const long bj = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (bj >= nb) return;
+  __shared__ double iv[256];
+  const long bj = blockIdx.y, r = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) iv[i] = inv[bj * 256 + i];
+  __syncthreads();
+  if (r >= n) return;
   float4* out = reinterpret_cast<float4*>(L + r * n + bj * 16);
   double o[16];
   if (bj >= r / 16) {
 #pragma unroll
     for (int j = 0; j < 16; ++j) o[j] = 0.0;
   } else {
-    const double* a = A + r * n + bj * 16;
-    const double* iv = inv + bj * 256;
+    const double2* a = reinterpret_cast<const double2*>(A + r * n + bj * 16);
     double av[16];
 #pragma unroll
-    for (int p = 0; p < 16; ++p) av[p] = a[p];
+    for (int p = 0; p < 8; ++p) {
+      const double2 v = a[p];
+      av[2 * p] = v.x, av[2 * p + 1] = v.y;
+    }
     bool finite = true;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      double s = 0.0;
+      double t = 0.0;
 #pragma unroll
       for (int p = 0; p < 16; ++p)
-        if (p >= j) s = fma(av[p], iv[p * 16 + j], s);
-      o[j] = s;
-      finite = finite && isfinite(s);
+        if (p >= j) t = fma(av[p], iv[p * 16 + j], t);
+      o[j] = t;
+      finite = finite && isfinite(t);
     }
     if (!finite) atomicOr(status, 2);
   }
@@ -250,11 +334,12 @@ __global__ __launch_bounds__(128) void ldl_finish_kernel(const double* __restric
 }
 
 static size_t align256(size_t x) { return (x + 255) / 256 * 256; }
-constexpr size_t kDiagSmem = size_t(kNb) * (kNb + 1) * 8;
-constexpr size_t kPanelSmem = size_t(kNb + kPanelRows) * (kNb + 1) * 8;
+constexpr size_t kFactorSmem = size_t(kNb * kLd + 16 * kInvLd) * 8;
+constexpr size_t kPanelSmem = size_t(kNb * kLd + (kNb / 16) * 16 * kInvLd + 2 * kPanelRows * kInvLd) * 8;
 
 int block_ldl_device_setup() {
-  QB_CUDA(cudaFuncSetAttribute(chol_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kDiagSmem)));
+  QB_CUDA(cudaFuncSetAttribute(chol_first_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFactorSmem)));
+  QB_CUDA(cudaFuncSetAttribute(chol_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFactorSmem)));
   QB_CUDA(cudaFuncSetAttribute(chol_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPanelSmem)));
   return QTIP_OK;
 }
@@ -280,29 +365,27 @@ extern "C" int qtip_block_ldl(const float* HR_d, long n, float* L_d, double* L64
   cudaStream_t s = as_stream(stream);
   unsigned char* p = static_cast<unsigned char*>(workspace_d);
   int* status = reinterpret_cast<int*>(p);
-  double* A = reinterpret_cast<double*>(p + sizeof(LdlHeader));
-  double* inv = reinterpret_cast<double*>(p + sizeof(LdlHeader) + align256(size_t(n) * n * 8));
+  // 16-byte loads: a workspace that is only 8-byte aligned gives up the last 8 of the header's padding
+  double* A = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(p) + sizeof(LdlHeader)) & ~uintptr_t(15));
+  double* inv = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(A) + align256(size_t(n) * n * 8));
   QB_CUDA(cudaMemsetAsync(status, 0, sizeof(LdlHeader), s));
   {
     const unsigned g = blocks_for(n, 32);
     ldl_symmetrise_kernel<<<dim3(g, g), dim3(32, 8), 0, s>>>(HR_d, A, n);
     QB_LAUNCHED();
   }
-  for (long k = 0; k < n; k += kNb) {
-    const int kb = int(min(long(kNb), n - k));
-    chol_diag_kernel<<<1, 256, kDiagSmem, s>>>(A, n, k, kb, status);
-    QB_LAUNCHED();
-    const long r0 = k + kb, nr = n - r0;
-    if (nr <= 0) break;
-    chol_panel_kernel<<<blocks_for(nr, kPanelRows), kPanelRows, kPanelSmem, s>>>(A, n, k, kb);
+  chol_first_kernel<<<1, 256, kFactorSmem, s>>>(A, n, int(min(long(kNb), n)), inv, status);
+  QB_LAUNCHED();
+  for (long k = 0; k + kNb < n; k += kNb) {
+    const long r0 = k + kNb, nr = n - r0;
+    chol_panel_kernel<<<blocks_for(nr, kPanelRows), 256, kPanelSmem, s>>>(A, n, k, inv + k / 16 * 256);
     QB_LAUNCHED();
     const long tiles = (nr + kTile - 1) / kTile;
-    chol_update_kernel<<<unsigned(tiles * (tiles + 1) / 2), 256, 0, s>>>(A, n, k, kb, r0);
+    chol_update_kernel<<<unsigned(tiles * (tiles + 1) / 2), 256, kFactorSmem, s>>>(A, n, k, kNb, r0, inv + r0 / 16 * 256,
+                                                                                   status);
     QB_LAUNCHED();
   }
-  ldl_block_inverse_kernel<<<blocks_for(n / 16, 8), 128, 0, s>>>(A, n, inv);
-  QB_LAUNCHED();
-  ldl_finish_kernel<<<dim3(blocks_for(n / 16, 128), unsigned(n)), 128, 0, s>>>(A, inv, n, L_d, L64_d, status);
+  ldl_finish_kernel<<<dim3(blocks_for(n, 128), unsigned(n / 16)), 128, 0, s>>>(A, inv, n, L_d, L64_d, status);
   QB_LAUNCHED();
   return QTIP_OK;
 }

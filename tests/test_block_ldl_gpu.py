@@ -80,3 +80,16 @@ def test_block_ldl_reports_a_matrix_that_is_not_positive_definite(gpu):
         gpu.codec.block_ldl(dev(H))
     assert e.value.code == -6
     gpu.codec.block_ldl(dev(gpu.synth.spd_hessian(256, 2).astype(np.float32)))  # the next call starts clean
+
+
+@pytest.mark.parametrize("n", [112, 128, 240, 256, 384])
+def test_block_ldl_panel_edges(gpu, oracle, n):
+    """Sizes around the 128-column panel: a last diagonal block of 112 or 128 columns, alone and behind other panels; and a
+    pivot that fails in the first, in a middle and in the last 16-column block is reported."""
+    H = gpu.synth.spd_hessian(n, 20 + n).astype(np.float32)
+    check(gpu, H, oracle)
+    for at in (0, n // 2, n - 1):
+        bad = H.copy()
+        bad[at, at] = -1.0
+        with pytest.raises(gpu.QtipError, match="positive definite"):
+            gpu.codec.block_ldl(dev(bad))
