@@ -17,6 +17,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "trellis_decode.cuh"
 
 namespace qb {
 
@@ -32,7 +33,6 @@ int trellis_tc_multiply(qtip_matrix w, const uint16_t* x, float* z, int stride, 
 #endif
 constexpr int kGemmThreads = QB_GEMV_THREADS;  // 1024 (64 registers per thread) or 512 (128)
 constexpr int kMaxItemsPerCta = kGemmThreads / 32 / 8;  // 4 concurrent work items of 8 warps each, or 2 x 16, or 1 x 32
-constexpr int kLutBytes = 1024 * 32 * 4;                         // 128 KiB, 32 copies
 #ifndef QB_GEMV_CHUNK
 #define QB_GEMV_CHUNK 2
 #endif
@@ -46,53 +46,6 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a
 }
 __device__ __forceinline__ void warps_sync(int id, int warps) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(warps * 32) : "memory");
-}
-
-// Dynamic shared memory of the GEMM kernel, named at namespace scope so that every access is known to be a
-// shared-memory access at a constant base (a pointer carried through a struct is not): words [0, 32768) hold the
-// replicated LUT.
-extern __shared__ __align__(16) uint32_t gemm_smem_words[];
-
-// Decodes the two windows that one 32-bit word pair holds: o = word c of tiles (i1 = 1 : i1 = 0) of one tile column,
-// p = word c + 1 of the same tiles. State t of a window is its 16 bits starting at bit 4 t; bits above 15 of a state
-// register never reach the table index, so a state is cut with ONE funnel shift from the two source registers (the first
-// state of the low tile is `o` itself), doubled, hashed with one multiply-add (2 v (v + 1), entry in bits 7..16) and
-// turned into the byte address of the lane's own copy (entry e, copy l at byte 128 e + 4 l) with one three-input logic
-// operation: shift, add, multiply-add, and-or, load per state.
-#ifndef QB_GEMV_DECODE
-#define QB_GEMV_DECODE 1
-#endif
-__device__ __forceinline__ uint32_t lut_word(uint32_t v, uint32_t lane4) {
-#if QB_GEMV_DECODE == 1
-  const uint32_t v2 = v + v;
-  uint32_t y2;
-  asm("mad.lo.u32 %0, %1, %2, %2;" : "=r"(y2) : "r"(v), "r"(v2));
-  const uint32_t at = (y2 & 0x1ff80u) | lane4;
-#elif QB_GEMV_DECODE == 2
-  const uint32_t y = v * v + v;
-  const uint32_t at = ((y << 1) & 0x1ff80u) | lane4;
-#else
-  const uint32_t y = v * v + v;
-  const uint32_t at = (((y >> 6) & 1023u) << 7) + lane4;
-#endif
-  return *reinterpret_cast<const uint32_t*>(reinterpret_cast<const unsigned char*>(gemm_smem_words) + at);
-}
-__device__ __forceinline__ void decode_pair(uint32_t o, uint32_t p, uint32_t lane4, uint32_t (&lo)[4],
-                                            uint32_t (&hi)[4]) {
-#if QB_GEMV_DECODE == 0
-  const uint32_t u0 = __byte_perm(o, p, 0x1054), u1 = __byte_perm(o, p, 0x3276);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) lo[k] = lut_word(u0 >> (16 - 4 * k), lane4), hi[k] = lut_word(u1 >> (16 - 4 * k), lane4);
-#else
-  const uint32_t pl = p << 16, oh = o >> 16;
-  lo[0] = lut_word(o, lane4);
-  hi[0] = lut_word(oh, lane4);
-#pragma unroll
-  for (int k = 1; k < 4; ++k) {
-    lo[k] = lut_word(__funnelshift_l(pl, o, 4 * k), lane4);
-    hi[k] = lut_word(__funnelshift_l(p, oh, 4 * k), lane4);
-  }
-#endif
 }
 
 // Tensor-parallel push: the products of this rank's rows go straight into every rank's gathered buffer (plain stores

@@ -43,6 +43,19 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile 
     }
   }
 }
+// One lane of a converged warp. Written with elect.sync, and not as "lane == 0", because the compiler then knows that a
+// single thread issues what follows: tcgen05 and TMA instructions take their operands from uniform registers. Measured on
+// the fused decode product, 57344 x 12288: 128 us at 16 tokens, 215 us with "lane == 0" and nothing else changed.
+__device__ __forceinline__ bool tc_elect() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
+}
+__device__ __forceinline__ int tc_warp() { return __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ void tc_tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),

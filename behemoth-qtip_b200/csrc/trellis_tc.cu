@@ -1,72 +1,85 @@
-// Mid-size batches (17 .. a few hundred tokens): z[token][row] = sum_k What[row][k] x[token][k] with What decoded from the
-// 2-bit trellis codes INSIDE the kernel, straight into the shared-memory A operand of tcgen05.mma. No dense copy of the
-// weights is ever written: the codes are read once per 256-token tile, which is what keeps this regime on the HBM
-// roofline of the codes instead of that of bf16 weights.
+// Batches of tokens: z[token][row] = sum_k What[row][k] x[token][k] with What decoded from the 2-bit trellis codes INSIDE
+// the kernel, straight into the tensor-memory A operand of tcgen05.mma. No copy of the weights is ever written, neither to
+// global nor to shared memory: the codes are read once per token tile (up to 256 tokens).
 //
-// Work item = 128 output rows (four 32-row block-rows) x one token tile (N = 64, 128 or 256 tokens) x one K-split.
-// The kernel is persistent: one CTA per SM walks its items (item = CTA, CTA + grid, ...) and every role keeps a running
-// K-step index, so the stage ring, the table in shared memory and the TMEM allocation live across items and the
-// pipeline never drains between them. Per K step (64 input columns = two 32-column blocks per block-row):
-//   warps 0..15 (decoders), in G groups (4, or 2 with 128/256-token tiles); group g owns the steps gk = g (mod G) and
-//       stage g of the ring, so G steps are being decoded at once and a warp meets a barrier only once per whole
-//       32 x 32 block or two. Per block: 8 bytes of codes per lane (requested 4 G steps ahead), the neighbour's words
-//       by shuffle, four windows of four states, sixteen look-ups in the 32-copy table (as the GEMV kernel), and four
-//       stmatrix.x4: the four look-ups of a window are exactly an m16n8k16 A fragment, i.e. four 8 x 8 bf16 matrices,
-//       and stmatrix writes them as 16-byte rows to the addresses the lanes name -- here the K-major, 128-byte-swizzled
-//       positions tcgen05 expects (row r, 16-byte chunk c at r * 128 + ((c ^ (r & 7)) << 4)). Eight consecutive rows
-//       hit eight different chunk positions: no bank conflicts. Then fence.proxy.async (the MMA reads through the
-//       async proxy) and one arrive per warp on the stage's "full" barrier.
-//   warp 16, one lane : TMA load of the step's activation tile (N tokens x 64 columns, K-major, 128-byte swizzle, zero
-//       fill beyond the last token) into the same stage; its transaction bytes complete the same "full" barrier.
-//   warp 17, one lane : ONE wait, four tcgen05.mma (M128 x N x K16) and ONE tcgen05.commit (on the stage's "empty"
-//       barrier) per step -- with few tokens an MMA is short, and the waits and commits of this single thread set the
-//       pace, so there is exactly one of each. Item i accumulates in TMEM buffer i & 1; after an item's last step a
-//       commit on "accumulator full". Warp 17 also allocates and frees the 2 N TMEM columns.
+// Why the operand goes through tensor memory. The decode itself needs the shared-memory pipe: one conflict-free look-up per
+// 32 states. An A tile written to shared memory costs that pipe two more passes per look-up (the store, and the tensor
+// core's read), so a product with the operand in shared memory cannot go below three times the look-up time; with tcgen05.st
+// the four decoded words of a window go from the registers to the tensor memory and the pipe only serves look-ups and the
+// activations. The 16x128b shape of tcgen05.st takes exactly the m16n8k16 fragment that the look-ups yield.
+//
+// Work item = 128 output rows (four 32-row block-rows) x one token tile (N = 16 .. 256 tokens, the batch divided evenly) x
+// one K-split. The kernel is persistent: one CTA per SM walks its items (item = CTA, CTA + grid, ...) and every role keeps
+// running ring positions, so the pipeline never drains between items. Per K step (64 KSUB input columns):
+//   warps 0..15 (decoders): warp w owns TMEM lanes 32 (w & 3) .. + 31, that is block-row w & 3 of the item, and the K
+//       steps gk = w >> 2 (mod 4). Per step it decodes 2 KSUB 32 x 32 blocks: 8 bytes of codes per lane and block (requested
+//       some own steps ahead), the neighbour's words by shuffle, four windows of four states, sixteen look-ups in the
+//       32-copy table per block, two tcgen05.st per block; then one arrive on the step's "full" barrier (four warps).
+//   warp 16, one lane : TMA loads of the step's activation tile (N tokens x 64 KSUB columns, K-major, 128-byte swizzle, zero
+//       fill beyond the last token) into its own ring in shared memory.
+//   warp 17, one lane : ONE wait, 4 KSUB tcgen05.mma (M128 x N x K16, A in TMEM, B in shared memory) and ONE commit per
+//       step: this thread sets the pace, so both operands of a step share a "full" and an "empty" barrier although the
+//       activation ring is the shallower one (its producer waits for the step that used the place before). Up to 128
+//       tokens item i accumulates in TMEM buffer i & 1, above that in a single buffer.
 //   warps 18..21      : epilogue of item i (tcgen05.ld of their 32 TMEM lanes, coalesced fp32 stores of z) under the
-//       main loop of item i + 1, then an arrive on "accumulator empty".
+//       main loop of item i + 1 (up to 128 tokens), then an arrive on "accumulator empty".
 // Every mbarrier wait is bounded (tc_wait): on a time-out the CTA's abort flag and the status word are raised, all
 // roles fall through, TMEM is freed and the kernel returns.
 #include "tc_common.cuh"
+#include "trellis_decode.cuh"
 
 namespace qb {
 
-constexpr int kFtRows = 128, kFtDecoders = 16, kFtEpilogueWarps = 4;
+constexpr int kFtRows = 128, kFtDecoders = 16, kFtSlots = kFtDecoders / 4, kFtEpilogueWarps = 4;
 constexpr int kFtThreads = (kFtDecoders + 2 + kFtEpilogueWarps) * 32;
-constexpr int kFtLutBytes = 1024 * 32 * 4;         // 32 copies of the table
-constexpr int kFtMaxStages = 8;
+constexpr int kFtTmemCols = 512;
+constexpr int kFtMaxStages = 12;  // of the A ring; the activation ring has at most as many
 
 struct FtSmem {
   unsigned long long full[kFtMaxStages], empty[kFtMaxStages], acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   int abort_flag;
 };
-// One ring: a stage holds the decoded A tile and the activation tile of a K step, filled behind ONE barrier (the arrivals
-// of the group's decoder warps plus the TMA's transaction bytes) and released by ONE tcgen05.commit, so the single MMA
-// thread runs one wait and one commit per step. A K step is KB blocks of 32 columns; stages = decoder groups = G.
-// 64-token tiles: 128-column steps, two stages (fewer, larger steps: 229 us against 264 us with 64-column steps and
-// four stages on 57344 x 12288); 128- and 256-token tiles: 64-column steps, two stages (96 KiB of stages in all cases).
+// TMEM: one or two accumulators of d_cols columns, then the A ring. Shared memory: table, activation ring, barriers.
+// 128-column steps halve the barrier round trips per column; above 128 tokens their activation tiles leave no room for a
+// ring. Rows that are an odd number of 64-column slices take 64-column steps.
 struct FtConfig {
-  int groups, kblk;
+  int ksub;  // 64-column slices per K step
+  int n_tile, tok_tiles, d_cols, d_bufs, a_stages, b_stages;
 };
-static FtConfig ft_config(int n_tile, int n_in) {
-  if (n_tile <= 64) return n_in % 128 == 0 ? FtConfig{2, 4} : FtConfig{4, 2};
-  return FtConfig{2, 2};
+constexpr size_t kFtMaxSmem = 227 * 1024;
+static FtConfig ft_config(int tokens, int n_in) {
+  FtConfig c;
+  c.tok_tiles = (tokens + 255) / 256;
+  c.n_tile = ((tokens + c.tok_tiles - 1) / c.tok_tiles + 15) / 16 * 16;  // M128 wants N in steps of 16
+  c.ksub = c.n_tile <= 128 && n_in % 128 == 0 ? 2 : 1;
+  c.d_cols = (c.n_tile + 31) / 32 * 32;
+  c.d_bufs = c.n_tile <= 128 ? 2 : 1;
+  c.a_stages = min(kFtMaxStages, (kFtTmemCols - c.d_bufs * c.d_cols) / (32 * c.ksub));  // at least kFtSlots
+  const size_t room = kFtMaxSmem - 1024 - kLutBytes - sizeof(FtSmem);
+  c.b_stages = int(min(size_t(c.a_stages), room / (size_t(c.n_tile) * 128 * c.ksub)));
+  return c;
 }
-static size_t ft_smem(int n_tile, FtConfig c) {
-  return 1024 + kFtLutBytes + size_t(c.groups) * (size_t(kFtRows) * 32 * c.kblk * 2 + size_t(n_tile) * 32 * c.kblk * 2) +
-         sizeof(FtSmem);
+static size_t ft_smem(const FtConfig& c) {
+  return 1024 + kLutBytes + size_t(c.b_stages) * c.n_tile * 128 * c.ksub + sizeof(FtSmem);
 }
 
 __device__ int g_ft_status;  // used when the caller passes no status word
 
-extern __shared__ __align__(16) unsigned char ft_smem_raw[];
-
-// No "memory" clobber: the stores go to the A ring only, and the compiler must stay free to issue the table look-ups of
-// the following windows before this store (a clobber would serialise look-up latency window by window). The fence and
-// the barrier arrive that follow the last store of a step are volatile with a clobber, which keeps the order that matters.
-__device__ __forceinline__ void stmatrix_x4(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
-  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r0), "r"(r1), "r"(r2),
-               "r"(r3));
+// Eight decoded words per lane: rows (lane / 4) and + 8 of 16 TMEM lanes, columns (lane & 3) + 4 q. a[2 q + h] is row half
+// h of column group q, which is the order of the states in two windows (tile columns 0 and 1 of a block).
+__device__ __forceinline__ void tmem_st_16x16(uint32_t taddr, const uint32_t (&a)[4], const uint32_t (&b)[4]) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(a[0]),
+               "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]));
+}
+__device__ __forceinline__ void tc_mma_tmem_a(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                              bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(uint32_t(accumulate))
+      : "memory");
 }
 
 // One work item = 128 output rows x one token tile x one K-split.
@@ -83,56 +96,62 @@ __device__ __forceinline__ FtItem ft_item(int item, int tok_tiles, int splits, i
   it.steps = int(long(k_total) * (it.split + 1) / splits) - it.ks_lo;  // >= 1: the host keeps splits <= k_total
   return it;
 }
-// Walks the K steps of this CTA's items (item = first + i * stride) as one long sequence with a running index `gk`:
-// stage and barrier parity of a step depend on gk alone, so the ring keeps turning across item boundaries.
+struct FtGeom {
+  int n_items, stride, tok_tiles, splits, k_total, n_tile;
+};
+// Walks K steps k0, k0 + by, ... of this CTA's items (item = CTA, CTA + grid, ...) as one long sequence.
 struct FtWalk {
-  int item, n_items, stride, tok_tiles, splits, k_total, n_tile;
-  int gk, base;  // global step index of the cursor, and of the first step of the current item
+  int item, k;
   FtItem cur;
-  __device__ __forceinline__ void start(int first, int n_items_, int stride_, int tok_tiles_, int splits_, int k_total_,
-                                        int n_tile_, int gk0) {
-    item = first, n_items = n_items_, stride = stride_, tok_tiles = tok_tiles_, splits = splits_, k_total = k_total_;
-    n_tile = n_tile_, gk = gk0, base = 0;
-    if (item < n_items) cur = ft_item(item, tok_tiles, splits, k_total, n_tile);
-    settle();
+  __device__ __forceinline__ void start(const FtGeom& g, int k0) {
+    item = blockIdx.x, k = k0;
+    cur = ft_item(item, g.tok_tiles, g.splits, g.k_total, g.n_tile);  // the grid has at most n_items CTAs
+    settle(g);
   }
-  __device__ __forceinline__ void settle() {
-    while (item < n_items && gk >= base + cur.steps) {
-      base += cur.steps;
-      item += stride;
-      if (item < n_items) cur = ft_item(item, tok_tiles, splits, k_total, n_tile);
+  __device__ __forceinline__ void settle(const FtGeom& g) {
+    while (item < g.n_items && k >= cur.steps) {
+      k -= cur.steps;
+      item += g.stride;
+      if (item < g.n_items) cur = ft_item(item, g.tok_tiles, g.splits, g.k_total, g.n_tile);
     }
   }
-  __device__ __forceinline__ bool done() const { return item >= n_items; }
-  __device__ __forceinline__ int k() const { return gk - base; }  // step inside the current item
-  __device__ __forceinline__ void advance(int by) {
-    gk += by;
-    settle();
+  __device__ __forceinline__ void advance(const FtGeom& g, int by) {
+    k += by;
+    if (k >= cur.steps) settle(g);
+  }
+};
+// Position in a ring of `depth` stages: the parity of a barrier's n-th use is n & 1.
+struct FtRing {
+  int stage, phase;
+  __device__ __forceinline__ void advance(int by, int depth) {
+    stage += by;
+    if (stage >= depth) stage -= depth, phase ^= 1;
   }
 };
 
 // Persistent: grid = min(SMs, items); CTA c takes items c, c + grid, ... z[(split * tokens + token) * stride + row].
-// G = decoder groups = stages of the ring, KB = 32-column blocks per K step.
-template <int G, int KB>
+template <int KSUB>
 __global__ __launch_bounds__(kFtThreads, 1) void trellis_tc_kernel(qtip_matrix w, const __grid_constant__ CUtensorMap map_x,
-                                                                   float* __restrict__ z, int stride, int tokens, int n_tile,
-                                                                   int splits, int n_items, int* __restrict__ status) {
-  constexpr int kFtKblk = KB, kFtK = 32 * KB;
-  constexpr uint32_t kFtABytes = kFtRows * kFtK * 2;  // 16 or 32 KiB per stage
-  const uint32_t raw = smem_u32(ft_smem_raw);
-  const uint32_t base = (raw + 1023u) & ~1023u;  // swizzled tiles need 1,024-byte alignment
-  unsigned char* smem = ft_smem_raw + (base - raw);
-  uint32_t* lut_s = reinterpret_cast<uint32_t*>(smem);
-  const uint32_t a_ring = base + kFtLutBytes, b_ring = a_ring + uint32_t(G) * kFtABytes;
-  const uint32_t b_bytes = uint32_t(n_tile) * kFtK * 2;
-  FtSmem& sm = *reinterpret_cast<FtSmem*>(smem + kFtLutBytes + size_t(G) * (kFtABytes + b_bytes));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int k_total = w.in / kFtK, tok_tiles = (tokens + n_tile - 1) / n_tile;
+                                                                   float* __restrict__ z, int stride, int tokens,
+                                                                   const FtConfig cfg, int splits, int n_items,
+                                                                   int* __restrict__ status) {
+  constexpr int kFtK = 64 * KSUB;     // input columns per K step
+  constexpr int kFtACols = kFtK / 2;  // TMEM columns of one A stage: two bf16 per 32-bit column
+  unsigned char* smem = reinterpret_cast<unsigned char*>(gemm_smem_words);  // the table is at its start
+  const uint32_t raw = smem_u32(smem);
+  const uint32_t b_ring = (raw + uint32_t(kLutBytes) + 1023u) & ~1023u;  // swizzled tiles need 1,024-byte alignment
+  const uint32_t b_bytes = uint32_t(cfg.n_tile) * kFtK * 2;
+  FtSmem& sm = *reinterpret_cast<FtSmem*>(smem + (b_ring - raw) + size_t(cfg.b_stages) * b_bytes);
+  const int warp = tc_warp(), lane = threadIdx.x & 31;
+  FtGeom geo;
+  geo.n_items = n_items, geo.stride = gridDim.x, geo.tok_tiles = cfg.tok_tiles, geo.splits = splits;
+  geo.k_total = w.in / kFtK, geo.n_tile = cfg.n_tile;
   volatile int* abort_flag = &sm.abort_flag;
 
+  chain_release();
   if (threadIdx.x == 0) {
     for (int s = 0; s < kFtMaxStages; ++s) {
-      tc_mbar_init(smem_u32(&sm.full[s]), kFtDecoders / G + 1);  // the group's warps + the TMA lane (with its bytes)
+      tc_mbar_init(smem_u32(&sm.full[s]), 5);  // one warp per block-row, and the TMA lane with its bytes
       tc_mbar_init(smem_u32(&sm.empty[s]), 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -142,220 +161,202 @@ __global__ __launch_bounds__(kFtThreads, 1) void trellis_tc_kernel(qtip_matrix w
     sm.abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == kFtDecoders + 1) {  // TMEM allocation: whole warp, two accumulators of n_tile columns
+  if (warp == kFtDecoders + 1) {  // TMEM allocation: whole warp
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)),
-                 "r"(uint32_t(2 * n_tile))
+                 "r"(uint32_t(kFtTmemCols))
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (warp < kFtDecoders) {
-    // 32 copies of the table: each decoder thread reads two entries, the warp spreads them with shuffles so that every
-    // store instruction writes 32 consecutive words.
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int e0 = (warp * 2 + h) * 32;
+    // 32 copies of the table: each decoder thread reads one entry at a time, the warp spreads them with shuffles so that
+    // every store instruction writes 32 consecutive words.
+#pragma unroll 1
+    for (int h = warp; h < 32; h += kFtDecoders) {
+      const int e0 = h * 32;
       const uint32_t mine = w.lut[e0 + lane];
 #pragma unroll
-      for (int e = 0; e < 32; ++e) lut_s[(e0 + e) * 32 + lane] = __shfl_sync(0xffffffffu, mine, e);
+      for (int e = 0; e < 32; ++e) gemm_smem_words[(e0 + e) * 32 + lane] = __shfl_sync(0xffffffffu, mine, e);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = sm.tmem_base;
+  const uint32_t a_tmem = tmem + uint32_t(cfg.d_bufs * cfg.d_cols);
 
   if (warp < kFtDecoders) {
-    // ---- decoders: G groups of 16 / G warps; group g decodes the steps gk = g (mod G) into stage g, so G steps are in
-    // the making at any time and a warp meets a barrier once per G / 2 whole 32 x 32 blocks.
-    constexpr int kWpg = kFtDecoders / G, kBpw = 4 * kFtKblk / kWpg;  // warps per group, blocks per warp and step
-    const int grp = warp / kWpg, mem = warp % kWpg;
-    const int n2 = w.in / 32;
-    const uint32_t a_tile = a_ring + uint32_t(grp) * kFtABytes;
-    // stmatrix row addresses of this lane inside a 16 x 16 tile: matrix q = lane >> 3 (q & 1: rows + 8, q >> 1:
-    // columns + 8), row lane & 7
-    const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8, lchunk = lane >> 4;
-    int brl[kBpw], kbl[kBpw];
-#pragma unroll
-    for (int i = 0; i < kBpw; ++i) {
-      const int blk = mem * kBpw + i;  // block of the step: block-row blk / kFtKblk, column block blk % kFtKblk
-      brl[i] = blk / kFtKblk, kbl[i] = blk % kFtKblk;
-    }
-    const uint2* codes = reinterpret_cast<const uint2*>(w.trellis) + lane;
-    auto fetch = [&](const FtWalk& wk, uint2(&dst)[kBpw]) {
-      // block (block-row, column block) of K step ks: 8-byte unit ((br * n2 + 2 ks + kbl) * 32 + lane)
-      const FtWalk& x = wk;
-      const bool live = !x.done();
-      const int ks = live ? x.cur.ks_lo + x.k() : 0, r0 = live ? x.cur.row0 / 32 : 0;
-#pragma unroll
-      for (int i = 0; i < kBpw; ++i) dst[i] = codes[(size_t(r0 + brl[i]) * n2 + kFtKblk * ks + kbl[i]) * 32];
-    };
-    constexpr int kAhead = 4;  // group steps of codes in flight per lane (= 4 G K steps)
-    uint2 next[kAhead][kBpw];
-    FtWalk use, pre;  // the step being decoded, and the step whose codes are being requested (kAhead group steps later)
-    use.start(blockIdx.x, n_items, gridDim.x, tok_tiles, splits, k_total, n_tile, grp);
+    const int slot = warp >> 2, quarter = warp & 3;
+    const uint32_t lane4 = uint32_t(lane) * 4u;
+    const size_t row_units = size_t(w.in / 32) * 32;  // 8-byte units of one block-row
+    const uint2* codes = reinterpret_cast<const uint2*>(w.trellis) + lane + size_t(quarter) * row_units;
+    constexpr int kAhead = 4 / KSUB;  // own steps of codes in flight per lane
+    uint2 next[kAhead][2 * KSUB];
+    FtWalk use, pre;  // the step being decoded, and the step whose codes are being requested (kAhead own steps later)
+    use.start(geo, slot);
     pre = use;
+    auto place = [&]() {  // past the last item: a harmless re-read of its first blocks
+      return codes + size_t(pre.cur.row0 / 32) * row_units +
+             size_t(pre.cur.ks_lo + (pre.item < n_items ? pre.k : 0)) * (64 * KSUB);
+    };
+    const uint2* from = place();
+    auto fetch = [&](uint2(&dst)[2 * KSUB]) {
 #pragma unroll
-    for (int q = 0; q < kAhead; ++q) {
-      fetch(pre, next[q]);
-      pre.advance(G);
-    }
+      for (int i = 0; i < 2 * KSUB; ++i) dst[i] = from[32 * i];
+      pre.k += kFtSlots;
+      if (pre.k < pre.cur.steps) {
+        from += kFtSlots * 64 * KSUB;
+      } else {
+        pre.settle(geo);
+        from = place();
+      }
+    };
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) fetch(next[q]);
+    FtRing ring{slot, 0};
+    const uint32_t lanes = a_tmem + (uint32_t(quarter * 32) << 16);
     bool ok = true;
-    while (!use.done() && ok) {
+    while (use.item < n_items && ok) {
 #pragma unroll
       for (int q = 0; q < kAhead; ++q) {
-        if (use.done()) break;
-        uint2 own[kBpw];
+        if (use.item >= n_items) break;
+        uint2 own[2 * KSUB];
 #pragma unroll
-        for (int i = 0; i < kBpw; ++i) own[i] = next[q][i];
-        fetch(pre, next[q]);
-        pre.advance(G);
-        const int uses = use.gk / G;  // earlier uses of stage `grp`
-        if (uses >= 1 && !tc_wait(smem_u32(&sm.empty[grp]), uint32_t((uses - 1) & 1), abort_flag, status)) {
-          ok = false;
-          break;
-        }
+        for (int i = 0; i < 2 * KSUB; ++i) own[i] = next[q][i];
+        fetch(next[q]);
+        const uint32_t at = lanes + uint32_t(ring.stage * kFtACols);
 #pragma unroll
-        for (int i = 0; i < kBpw; ++i) {
-          const uint2 peer = make_uint2(__shfl_sync(0xffffffffu, own[i].x, (lane + 1) & 31),
-                                        __shfl_sync(0xffffffffu, own[i].y, (lane + 1) & 31));
-#pragma unroll
-          for (int j1 = 0; j1 < 2; ++j1) {
-            const uint32_t o = j1 ? own[i].y : own[i].x, pw = j1 ? peer.y : peer.x;
-#pragma unroll
-            for (int i1 = 0; i1 < 2; ++i1) {
-              const uint32_t u = __byte_perm(o, pw, i1 ? 0x3276 : 0x1054);  // word c << 16 | word c + 1
-              uint32_t a[4];
-#pragma unroll
-              for (int t = 0; t < 4; ++t) {
-                const uint32_t v = u >> (16 - 4 * t);
-                const uint32_t y = v * v + v;
-                a[t] = lut_s[((y >> 6) & 1023u) * 32u + lane];
-              }
-              const int r = brl[i] * 32 + i1 * 16 + lrow, ch = kbl[i] * 4 + j1 * 2 + lchunk;
-              stmatrix_x4(a_tile + uint32_t(ch >> 3) * 16384u + uint32_t(r) * 128u + (uint32_t((ch & 7) ^ (r & 7)) << 4),
-                          a[0], a[1], a[2], a[3]);
-            }
+        for (int i = 0; i < 2 * KSUB; ++i) {
+          const uint32_t px = __shfl_sync(0xffffffffu, own[i].x, (lane + 1) & 31);
+          const uint32_t py = __shfl_sync(0xffffffffu, own[i].y, (lane + 1) & 31);
+          uint32_t lo[2][4], hi[2][4];
+          decode_pair(own[i].x, px, lane4, lo[0], hi[0]);
+          decode_pair(own[i].y, py, lane4, lo[1], hi[1]);
+          if (i == 0) {  // the tensor core has read this stage's earlier contents
+            ok = __all_sync(0xffffffffu, tc_wait(smem_u32(&sm.empty[ring.stage]), uint32_t(ring.phase ^ 1), abort_flag, status));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           }
+          tmem_st_16x16(at + uint32_t(16 * i), lo[0], lo[1]);
+          tmem_st_16x16(at + uint32_t(16 * i) + (16u << 16), hi[0], hi[1]);
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (!ok) break;
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) tc_mbar_arrive(smem_u32(&sm.full[grp]));
-        use.advance(G);
+        if (lane == 0) tc_mbar_arrive(smem_u32(&sm.full[ring.stage]));
+        ring.advance(kFtSlots, cfg.a_stages);
+        use.advance(geo, kFtSlots);
       }
     }
   } else if (warp == kFtDecoders) {
     // ---- TMA producer of the activation tiles
-    if (lane == 0) {
+    if (tc_elect()) {
+      chain_wait();  // the activations may come from the kernel before this one
       FtWalk wk;
-      wk.start(blockIdx.x, n_items, gridDim.x, tok_tiles, splits, k_total, n_tile, 0);
-      for (; !wk.done(); wk.advance(1)) {
-        const int s = wk.gk % G, uses = wk.gk / G;
-        if (uses >= 1 && !tc_wait(smem_u32(&sm.empty[s]), uint32_t((uses - 1) & 1), abort_flag, status)) break;
-        const uint32_t bar = smem_u32(&sm.full[s]);
+      wk.start(geo, 0);
+      FtRing ring{0, 0}, rb{0, 0}, before{0, 0};  // the step, its place in the activation ring, the step that held the place
+      int filled = 0;
+      for (; wk.item < n_items; wk.advance(geo, 1), ring.advance(1, cfg.a_stages), rb.advance(1, cfg.b_stages)) {
+        if (filled < cfg.b_stages) {
+          ++filled;
+        } else {
+          if (!tc_wait(smem_u32(&sm.empty[before.stage]), uint32_t(before.phase), abort_flag, status)) break;
+          before.advance(1, cfg.a_stages);
+        }
+        const uint32_t bar = smem_u32(&sm.full[ring.stage]);
         tc_mbar_expect_tx(bar, b_bytes);
-        for (int sub = 0; sub < kFtKblk / 2; ++sub)  // one 64-column box per 128-byte-swizzled sub-tile
-          tc_tma_load_2d(b_ring + uint32_t(s) * b_bytes + uint32_t(sub) * uint32_t(n_tile) * 128u, &map_x,
-                         (wk.cur.ks_lo + wk.k()) * kFtK + 64 * sub, wk.cur.tok0, bar);
+#pragma unroll
+        for (int sub = 0; sub < KSUB; ++sub)  // one 64-column box per 128-byte-swizzled tile
+          tc_tma_load_2d(b_ring + uint32_t(rb.stage) * b_bytes + uint32_t(sub * cfg.n_tile) * 128u, &map_x,
+                         (wk.cur.ks_lo + wk.k) * kFtK + 64 * sub, wk.cur.tok0, bar);
       }
     }
   } else if (warp == kFtDecoders + 1) {
-    // ---- MMA issuer: item i of this CTA accumulates in TMEM buffer i & 1, so the epilogue of one item runs under the
-    // main loop of the next
-    if (lane == 0) {
-      const uint32_t idesc = tc_idesc(kFtRows, n_tile);
+    // ---- MMA issuer
+    if (tc_elect()) {
+      const uint32_t idesc = tc_idesc(kFtRows, cfg.n_tile);
       FtWalk wk;
-      wk.start(blockIdx.x, n_items, gridDim.x, tok_tiles, splits, k_total, n_tile, 0);
+      wk.start(geo, 0);
+      FtRing ra{0, 0}, rb{0, 0}, rd{0, 0};
       bool ok = true;
-      for (int i = 0; !wk.done() && ok; ++i) {
-        const int buf = i & 1, steps = wk.cur.steps;
-        if (i >= 2) ok = tc_wait(smem_u32(&sm.acc_empty[buf]), uint32_t(((i >> 1) - 1) & 1), abort_flag, status);
+      while (wk.item < n_items && ok) {
+        const int steps = wk.cur.steps;
+        ok = tc_wait(smem_u32(&sm.acc_empty[rd.stage]), uint32_t(rd.phase ^ 1), abort_flag, status);
         if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int k = 0; k < steps; ++k) {
-          const int s = wk.gk % G;
-          ok = tc_wait(smem_u32(&sm.full[s]), uint32_t((wk.gk / G) & 1), abort_flag, status);
+          ok = tc_wait(smem_u32(&sm.full[ra.stage]), uint32_t(ra.phase), abort_flag, status);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-          for (int sub = 0; sub < kFtKblk / 2; ++sub) {
-            const uint64_t a_desc = tc_smem_desc(a_ring + uint32_t(s) * kFtABytes + uint32_t(sub) * 16384u);
-            const uint64_t b_desc = tc_smem_desc(b_ring + uint32_t(s) * b_bytes + uint32_t(sub) * uint32_t(n_tile) * 128u);
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-              tc_mma(tmem + uint32_t(buf * n_tile), a_desc + uint64_t(2 * kk), b_desc + uint64_t(2 * kk), idesc,
-                     k > 0 || kk > 0 || sub > 0);
+          for (int kk = 0; kk < kFtK / 16; ++kk) {
+            const uint64_t b_desc = tc_smem_desc(b_ring + uint32_t(rb.stage) * b_bytes + uint32_t((kk >> 2) * cfg.n_tile) * 128u);
+            tc_mma_tmem_a(tmem + uint32_t(rd.stage * cfg.d_cols), a_tmem + uint32_t(ra.stage * kFtACols + 8 * kk),
+                          b_desc + uint64_t(2 * (kk & 3)), idesc, k > 0 || kk > 0);
           }
-          tc_commit(smem_u32(&sm.empty[s]));
-          wk.advance(1);
+          tc_commit(smem_u32(&sm.empty[ra.stage]));
+          ra.advance(1, cfg.a_stages);
+          rb.advance(1, cfg.b_stages);
+          wk.advance(geo, 1);
         }
-        if (ok) tc_commit(smem_u32(&sm.acc_full[buf]));
+        if (ok) tc_commit(smem_u32(&sm.acc_full[rd.stage]));
+        rd.advance(1, cfg.d_bufs);
       }
     }
   } else {
     // ---- epilogue warps: warp e reads TMEM lanes 32 (e % 4) .. + 31 (rows), columns = tokens of the tile
+    chain_wait();  // z may still be read by the kernel before this one
     const int quarter = warp & 3;
-    int i = 0;
-    for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++i) {
-      const FtItem it = ft_item(item, tok_tiles, splits, k_total, n_tile);
-      const int buf = i & 1;
-      if (!tc_wait(smem_u32(&sm.acc_full[buf]), uint32_t((i >> 1) & 1), abort_flag, status)) break;
+    FtRing rd{0, 0};
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x, rd.advance(1, cfg.d_bufs)) {
+      const FtItem it = ft_item(item, cfg.tok_tiles, splits, geo.k_total, cfg.n_tile);
+      if (!__all_sync(0xffffffffu, tc_wait(smem_u32(&sm.acc_full[rd.stage]), uint32_t(rd.phase), abort_flag, status))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      float* zs = z + size_t(it.split) * tokens * stride + it.row0 + quarter * 32 + lane;
+      float* zs = z + (size_t(it.split) * tokens + it.tok0) * stride + it.row0 + quarter * 32 + lane;
+      const int live = min(cfg.n_tile, tokens - it.tok0);
 #pragma unroll 1
-      for (int cc = 0; cc < n_tile; cc += 32) {
-        if (it.tok0 + cc >= tokens) break;
-        uint32_t v[32];
-        const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(buf * n_tile + cc);
+      for (int cc = 0; cc < live; cc += 16) {
+        uint32_t v[16];
+        const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(rd.stage * cfg.d_cols + cc);
         asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-            "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-              "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-              "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-              "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+              "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
             : "r"(taddr)
             : "memory");
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const int tok = it.tok0 + cc + c;
-          if (tok < tokens) zs[size_t(tok) * stride] = __uint_as_float(v[c]);
-        }
+        for (int c = 0; c < 16; ++c)
+          if (cc + c < live) zs[size_t(cc + c) * stride] = __uint_as_float(v[c]);
       }
       // the accumulator has been read: hand the buffer back to the MMA thread
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) tc_mbar_arrive(smem_u32(&sm.acc_empty[buf]));
+      if (lane == 0) tc_mbar_arrive(smem_u32(&sm.acc_empty[rd.stage]));
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == kFtDecoders + 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(uint32_t(2 * n_tile)) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(uint32_t(kFtTmemCols)) : "memory");
   }
 }
 
 int trellis_tc_device_setup() {
-  const int big = int(ft_smem(256, FtConfig{2, 2}));  // every configuration stays within this size
-  QB_CUDA(cudaFuncSetAttribute(trellis_tc_kernel<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  QB_CUDA(cudaFuncSetAttribute(trellis_tc_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  QB_CUDA(cudaFuncSetAttribute(trellis_tc_kernel<2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  QB_CUDA(cudaFuncSetAttribute(trellis_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFtMaxSmem)));
+  QB_CUDA(cudaFuncSetAttribute(trellis_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFtMaxSmem)));
   return QTIP_OK;
 }
-
-// Token tile of the fused kernel for a batch: the smallest of 64 / 128 / 256 that holds it, else 256.
-static int ft_token_tile(int tokens) { return tokens <= 64 ? 64 : (tokens <= 128 ? 128 : 256); }
 
 int trellis_tc_multiply(qtip_matrix w, const uint16_t* x, float* z, int stride, int splits, int tokens, int* status,
                         cudaStream_t s) {
   QB_REQUIRE(w.in % 64 == 0 && w.out % kFtRows == 0, QTIP_E_GEOMETRY,
              "the fused tensor-core product needs in %% 64 == 0 and out %% 128 == 0 (in = %d, out = %d)", w.in, w.out);
   QB_REQUIRE(reinterpret_cast<uintptr_t>(x) % 16 == 0, QTIP_E_ARG, "activations must be 16-byte aligned");
-  const int n_tile = ft_token_tile(tokens);
+  const FtConfig cfg = ft_config(tokens, w.in);
   CUtensorMap map_x;
-  int rc = tc_make_map(&map_x, x, uint64_t(tokens), uint64_t(w.in), uint32_t(n_tile));
+  int rc = tc_make_map(&map_x, x, uint64_t(tokens), uint64_t(w.in), uint32_t(cfg.n_tile));
   if (rc) return rc;
   if (!status) {
     void* p = nullptr;
@@ -365,21 +366,14 @@ int trellis_tc_multiply(qtip_matrix w, const uint16_t* x, float* z, int stride, 
   const DeviceInfo* info = device_info();
   if (!info) return QTIP_E_DEVICE;
   // More K-splits than K steps: the surplus slices of z hold zeros, the kernel runs with one step per split.
-  const FtConfig cfg = ft_config(n_tile, w.in);
-  const int k_total = w.in / (32 * cfg.kblk), eff = splits < k_total ? splits : k_total;
+  const int k_total = w.in / (64 * cfg.ksub), eff = splits < k_total ? splits : k_total;
   if (eff < splits)
     QB_CUDA(cudaMemsetAsync(z + size_t(eff) * tokens * stride, 0, size_t(splits - eff) * tokens * stride * sizeof(float), s));
-  const long items = long(w.out / kFtRows) * ((tokens + n_tile - 1) / n_tile) * eff;
+  const long items = long(w.out / kFtRows) * cfg.tok_tiles * eff;
   QB_REQUIRE(items < (1l << 30), QTIP_E_GEOMETRY, "too many work items (%ld)", items);
   const int grid = int(items < info->sm_count ? items : info->sm_count);
-  const size_t smem = ft_smem(n_tile, cfg);
-  if (cfg.groups == 2 && cfg.kblk == 4)
-    trellis_tc_kernel<2, 4><<<grid, kFtThreads, smem, s>>>(w, map_x, z, stride, tokens, n_tile, eff, int(items), status);
-  else if (cfg.groups == 4)
-    trellis_tc_kernel<4, 2><<<grid, kFtThreads, smem, s>>>(w, map_x, z, stride, tokens, n_tile, eff, int(items), status);
-  else
-    trellis_tc_kernel<2, 2><<<grid, kFtThreads, smem, s>>>(w, map_x, z, stride, tokens, n_tile, eff, int(items), status);
-  QB_LAUNCHED();
+  QB_CUDA(launch_chained(cfg.ksub == 2 ? trellis_tc_kernel<2> : trellis_tc_kernel<1>, dim3(grid), dim3(kFtThreads),
+                         ft_smem(cfg), s, w, map_x, z, stride, tokens, cfg, eff, int(items), status));
   return QTIP_OK;
 }
 

@@ -297,3 +297,22 @@ def test_fused_decode_tensor_core_product(gpu, oracle, n_in, n_out, tokens, spli
     else:
         gpu.linear.qtip_multiply_tc(w, bf16_dev(xb), z2, n_out, splits, tokens, status)
     assert torch.equal(z, z2)
+
+
+@pytest.mark.parametrize("n_in,n_out,tokens,splits", [(64, 128, 2, 1), (192, 256, 16, 2), (128, 128, 17, 1), (384, 128, 128, 3),
+                                                      (320, 256, 129, 1), (896, 384, 257, 2), (1024, 128, 511, 1),
+                                                      (128, 20480, 5, 1), (256, 20480, 130, 2), (64, 19072, 33, 1)])
+def test_fused_decode_tile_edges(gpu, oracle, n_in, n_out, tokens, splits):
+    """The fused product at the edges of its tiles: token tiles of 16 .. 256 in steps of 16 with one live column in the last
+    16, one and two accumulators, rows of an odd number of 64-column slices, items with fewer K steps than decoder groups,
+    and more items than SMs. Against float64 on the decoded weights; only the order of at most 1,024 fp32 sums differs
+    (5e-6: sqrt(1024) x 2^-24 with a factor of two)."""
+    w, tr, su, sv, tl = make_linear(gpu, n_in, n_out, 900 + tokens)
+    xb = gpu.synth.f32_to_bf16_bits(np.random.default_rng(tokens).standard_normal((tokens, n_in)).astype(np.float32))
+    z = torch.full((splits, tokens, n_out), float("nan"), dtype=torch.float32, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    gpu.linear.qtip_multiply_tc(w, bf16_dev(xb), z, n_out, splits, tokens, status)
+    assert int(status) == 0
+    W = oracle.decode_rows(tr, n_in, n_out, tl, 0, n_out, True).astype(np.float64)
+    ref = gpu.synth.bf16_bits_to_f32(xb).astype(np.float64) @ W.T
+    assert rel_l2(z.sum(0).cpu().numpy(), ref) < 5e-6
