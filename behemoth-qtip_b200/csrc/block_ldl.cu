@@ -8,10 +8,9 @@
 // The Cholesky is right-looking with 128-column panels, two launches a panel:
 //   1. chol_panel_kernel  rows below the diagonal block: x L11^T = a, 64 rows per CTA held in registers, sixteen columns
 //                         at a time through the inverse of their diagonal block;
-//   2. chol_update_kernel trailing update C -= P P^T on the lower triangle: 128 x 128 tiles, 8 x 8 fp64 accumulators per
-//                         thread, the 128-deep panels streamed through shared memory in 16-column slices. This is where
-//                         the n^3 / 6 fused multiply-adds are: DFMA-issue bound (64 lanes per SM and clock). The CTA of
-//                         tile (0, 0) keeps its tile, which is the next diagonal block, in shared memory and factors it
+//   2. chol_update_kernel trailing update C -= P P^T on the lower triangle: 128 x 128 tiles on the fp64 tensor cores, the
+//                         128-deep panels streamed through shared memory in 16-column slices. This is where the n^3 / 6
+//                         multiply-adds are: bound by the fp64 pipes (64 lanes per SM and clock). The CTA of tile (0, 0) keeps its tile, which is the next diagonal block, in shared memory and factors it
 //                         there (chol_factor) while the other tiles are updated: the one serial stage of a panel is off
 //                         the critical path as long as the update takes longer than one factorisation.
 // The first diagonal block has a launch of its own (chol_first_kernel).
@@ -54,6 +53,7 @@ __global__ void ldl_symmetrise_kernel(const float* __restrict__ H, double* __res
 // diagonal).
 constexpr int kLd = kNb + 1;
 constexpr int kInvLd = 17;
+__device__ __forceinline__ void factor_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 __device__ __forceinline__ void chol_factor(double* __restrict__ S, double* __restrict__ inv_s, int kb,
                                             double* __restrict__ inv, int* status) {
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -91,7 +91,7 @@ __device__ __forceinline__ void chol_factor(double* __restrict__ S, double* __re
         }
       }
     }
-    __syncthreads();
+    factor_sync();
     // rows below: x = a inv^T
     const int below = kb - base - 16;
     double x[7];
@@ -105,11 +105,11 @@ __device__ __forceinline__ void chol_factor(double* __restrict__ S, double* __re
       }
       x[a] = t;
     }
-    __syncthreads();
+    factor_sync();
 #pragma unroll
     for (int a = 0; a < 7; ++a)
       if (ty + 16 * a < below) S[(base + 16 + ty + 16 * a) * kLd + base + tx] = x[a];
-    __syncthreads();
+    factor_sync();
     // right of it: a[i][c] -= sum_p x[i][p] x[c][p], 16 x 16 blocks on and below the diagonal
     for (int a = 0; 16 * a < below; ++a) {
       double* row = S + (base + 16 + ty + 16 * a) * kLd + base;
@@ -124,7 +124,7 @@ __device__ __forceinline__ void chol_factor(double* __restrict__ S, double* __re
         row[16 + tx + 16 * b] -= t0 + t1;  // above the diagonal of a diagonal block: never read
       }
     }
-    __syncthreads();
+    factor_sync();
   }
 }
 __device__ __forceinline__ void chol_store(const double* __restrict__ S, double* __restrict__ A, long n, long k, int kb) {
@@ -202,12 +202,22 @@ __global__ __launch_bounds__(256) void chol_panel_kernel(double* __restrict__ A,
 }
 
 // C[i][j] -= sum_p P[i][p] P[j][p] for the tile (ti, tj), tj <= ti, of the trailing matrix that starts at row / column
-// r0; P = A[r0.., k .. k + kb). 256 threads as 16 x 16, each 8 x 8 outputs at rows ty + 16 a and columns tx + 16 b.
+// r0; P = A[r0.., k .. k + 128). Sixteen warps as 4 x 4, each 32 x 32 outputs as 4 x 4 fp64 tensor-core fragments
+// (m8n8k4). The two operand panels pass through a ring of 16-column slices (cp.async; row stride 20 doubles: the 4 x 4
+// words that a half-warp reads for a fragment lie in 16 different bank pairs).
+// n = 12,288: all updates 66 ms with 8 x 8 outputs a thread and scalar multiply-adds, about 30 ms with the fragments.
 // Tile (0, 0) is the next diagonal block: its CTA, the first of the launch, factors it at once.
-__global__ __launch_bounds__(256, 1) void chol_update_kernel(double* __restrict__ A, long n, long k, int kb, long r0,
-                                                             double* __restrict__ inv, int* status) {
-  __shared__ double Pi[kKc][kTile + 2];
-  __shared__ double Pj[kKc][kTile + 2];
+constexpr int kSliceLd = kKc + 4, kSlices = kNb / kKc, kUpdThreads = 512, kUpdStages = 4;
+constexpr size_t kStageDoubles = size_t(2) * kTile * kSliceLd;
+__device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+__global__ __launch_bounds__(kUpdThreads, 1) void chol_update_kernel(double* __restrict__ A, long n, long k, long r0,
+                                                                     double* __restrict__ inv, int* status) {
+  extern __shared__ __align__(16) double upd_sm[];
+  double* sm = upd_sm;
   // linear block index -> (ti, tj) of the lower triangle
   const long t = blockIdx.x;
   long ti = long((sqrt(8.0 * double(t) + 1.0) - 1.0) * 0.5);
@@ -215,75 +225,79 @@ __global__ __launch_bounds__(256, 1) void chol_update_kernel(double* __restrict_
   while (ti * (ti + 1) / 2 > t) --ti;
   const long tj = t - ti * (ti + 1) / 2;
   const long i0 = r0 + ti * kTile, j0 = r0 + tj * kTile;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  double acc[8][8];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+  const int wi = (warp >> 2) * 32, wj = (warp & 3) * 32;
+  // a slice is 2 x 128 rows of 16 doubles = 2 x 1,024 copies of 16 bytes; rows past n repeat the last one and are not stored
+  auto stage = [&](int slice) {
+    double* dst = sm + size_t(slice % kUpdStages) * kStageDoubles;
 #pragma unroll
-  for (int a = 0; a < 8; ++a)
-#pragma unroll
-    for (int b = 0; b < 8; ++b) acc[a][b] = 0.0;
-  // staging: thread -> (row = tid / 2, eight consecutive panel columns (tid & 1) * 8 ..)
-  const int srow = threadIdx.x >> 1, scol = (threadIdx.x & 1) * 8;
-  const bool vi = i0 + srow < n, vj = j0 + srow < n;
-  const double* gi = A + (i0 + srow) * n + k + scol;
-  const double* gj = A + (j0 + srow) * n + k + scol;
-  double ri[8], rj[8];
-  auto fetch = [&](int c0) {
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const bool in = c0 + scol + q < kb;
-      ri[q] = (vi && in) ? gi[c0 + q] : 0.0;
-      rj[q] = (vj && in) ? gj[c0 + q] : 0.0;
+    for (int c = 0; c < 2 * kTile * kKc / 2 / kUpdThreads; ++c) {
+      const int idx = c * kUpdThreads + tid, side = idx >> 10, row = (idx >> 3) & 127, col = (idx & 7) * 2;
+      const long src = min((side ? j0 : i0) + row, n - 1);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + (side * kTile + row) * kSliceLd + col)),
+                   "l"(A + src * n + k + slice * kKc + col));
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  auto stash = [&]() {
+  double acc[4][4][2];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) Pi[scol + q][srow] = ri[q], Pj[scol + q][srow] = rj[q];
-  };
-  fetch(0);
-  stash();
-  __syncthreads();
-  const int slices = (kb + kKc - 1) / kKc;
-  for (int s = 0; s < slices; ++s) {
-    if (s + 1 < slices) fetch((s + 1) * kKc);  // the next slice travels to registers under this slice's arithmetic
+  for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int p = 0; p < kKc; ++p) {
-      double a[8], b[8];
+    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) a[q] = Pi[p][ty + 16 * q], b[q] = Pj[p][tx + 16 * q];
+  for (int s = 0; s < kUpdStages - 1; ++s) stage(s);
+#pragma unroll 1
+  for (int s = 0; s < kSlices; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kUpdStages - 2) : "memory");
+    __syncthreads();  // slice s is there for all, and everyone has left the stage that is filled next
+    if (s + kUpdStages - 1 < kSlices) stage(s + kUpdStages - 1);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    const double* Pi = sm + size_t(s % kUpdStages) * kStageDoubles + (wi + g) * kSliceLd + q;
+    const double* Pj = sm + size_t(s % kUpdStages) * kStageDoubles + (kTile + wj + g) * kSliceLd + q;
 #pragma unroll
-      for (int x = 0; x < 8; ++x)
+    for (int p = 0; p < kKc; p += 4) {
+      double a[4], b[4];
 #pragma unroll
-        for (int y = 0; y < 8; ++y) acc[x][y] = fma(a[x], b[y], acc[x][y]);
-    }
-    __syncthreads();
-    if (s + 1 < slices) {
-      stash();
-      __syncthreads();
+      for (int x = 0; x < 4; ++x) a[x] = Pi[8 * x * kSliceLd + p], b[x] = Pj[8 * x * kSliceLd + p];
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y) dmma_8x8x4(acc[x][y], a[x], b[y]);
     }
   }
   if (t == 0) {
-    extern __shared__ double sm[];
     const int kb2 = int(min(long(kNb), n - r0));
+    __syncthreads();  // the ring becomes the block
 #pragma unroll
-    for (int x = 0; x < 8; ++x)
+    for (int x = 0; x < 4; ++x)
 #pragma unroll
-      for (int y = 0; y < 8; ++y) {
-        const int i = ty + 16 * x, j = tx + 16 * y;
-        if (i < kb2 && j <= i) sm[i * kLd + j] = A[(r0 + i) * n + r0 + j] - acc[x][y];
-      }
+      for (int y = 0; y < 4; ++y)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int i = wi + 8 * x + g, j = wj + 8 * y + 2 * q + e;
+          if (i < kb2 && j <= i) sm[i * kLd + j] = A[(r0 + i) * n + r0 + j] - acc[x][y][e];
+        }
     __syncthreads();
-    chol_factor(sm, sm + kNb * kLd, kb2, inv, status);
+    if (tid < 256) chol_factor(sm, sm + kNb * kLd, kb2, inv, status);
+    __syncthreads();
     chol_store(sm, A, n, r0, kb2);
     return;
   }
 #pragma unroll
-  for (int x = 0; x < 8; ++x) {
-    const long i = i0 + ty + 16 * x;
+  for (int x = 0; x < 4; ++x) {
+    const long i = i0 + wi + 8 * x + g;
     if (i >= n) continue;
+    double2 c[4];
 #pragma unroll
-    for (int y = 0; y < 8; ++y) {
-      const long j = j0 + tx + 16 * y;
-      if (j <= i) A[i * n + j] -= acc[x][y];
+    for (int y = 0; y < 4; ++y) {
+      const long j = j0 + wj + 8 * y + 2 * q;  // even: 16-byte aligned
+      c[y] = j < n ? *reinterpret_cast<const double2*>(A + i * n + j) : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+      const long j = j0 + wj + 8 * y + 2 * q;
+      c[y].x -= acc[x][y][0], c[y].y -= acc[x][y][1];
+      if (j < n) *reinterpret_cast<double2*>(A + i * n + j) = c[y];  // above the diagonal: never read
     }
   }
 }
@@ -335,11 +349,12 @@ __global__ __launch_bounds__(128) void ldl_finish_kernel(const double* __restric
 
 static size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 constexpr size_t kFactorSmem = size_t(kNb * kLd + 16 * kInvLd) * 8;
+constexpr size_t kUpdSmem = kUpdStages * kStageDoubles * 8 > kFactorSmem ? kUpdStages * kStageDoubles * 8 : kFactorSmem;
 constexpr size_t kPanelSmem = size_t(kNb * kLd + (kNb / 16) * 16 * kInvLd + 2 * kPanelRows * kInvLd) * 8;
 
 int block_ldl_device_setup() {
   QB_CUDA(cudaFuncSetAttribute(chol_first_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFactorSmem)));
-  QB_CUDA(cudaFuncSetAttribute(chol_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFactorSmem)));
+  QB_CUDA(cudaFuncSetAttribute(chol_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kUpdSmem)));
   QB_CUDA(cudaFuncSetAttribute(chol_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPanelSmem)));
   return QTIP_OK;
 }
@@ -381,8 +396,8 @@ extern "C" int qtip_block_ldl(const float* HR_d, long n, float* L_d, double* L64
     chol_panel_kernel<<<blocks_for(nr, kPanelRows), 256, kPanelSmem, s>>>(A, n, k, inv + k / 16 * 256);
     QB_LAUNCHED();
     const long tiles = (nr + kTile - 1) / kTile;
-    chol_update_kernel<<<unsigned(tiles * (tiles + 1) / 2), 256, kFactorSmem, s>>>(A, n, k, kNb, r0, inv + r0 / 16 * 256,
-                                                                                   status);
+    chol_update_kernel<<<unsigned(tiles * (tiles + 1) / 2), kUpdThreads, kUpdSmem, s>>>(A, n, k, r0,
+                                                                                         inv + r0 / 16 * 256, status);
     QB_LAUNCHED();
   }
   ldl_finish_kernel<<<dim3(blocks_for(n, 128), unsigned(n / 16)), 128, 0, s>>>(A, inv, n, L_d, L64_d, status);
