@@ -8,11 +8,12 @@
 // The Cholesky is right-looking with 128-column panels, two launches a panel:
 //   1. chol_panel_kernel  rows below the diagonal block: x L11^T = a, 64 rows per CTA held in registers, sixteen columns
 //                         at a time through the inverse of their diagonal block;
-//   2. chol_update_kernel trailing update C -= P P^T on the lower triangle: 128 x 128 tiles on the fp64 tensor cores, the
+//   2. chol_update_kernel trailing update C -= P P^T on the lower triangle: 128 x 64 tiles on the fp64 tensor cores, the
 //                         128-deep panels streamed through shared memory in 16-column slices. This is where the n^3 / 6
-//                         multiply-adds are: bound by the fp64 pipes (64 lanes per SM and clock). The CTA of tile (0, 0) keeps its tile, which is the next diagonal block, in shared memory and factors it
-//                         there (chol_factor) while the other tiles are updated: the one serial stage of a panel is off
-//                         the critical path as long as the update takes longer than one factorisation.
+//                         multiply-adds are: bound by the fp64 pipes (64 lanes per SM and clock). The CTA of the first
+//                         tile takes the next diagonal block whole and factors it in shared memory (chol_factor) while
+//                         the other tiles are updated: the one serial stage of a panel is off the critical path as long
+//                         as the update takes longer than one factorisation.
 // The first diagonal block has a launch of its own (chol_first_kernel).
 // A non-positive pivot or a non-finite result sets a status word in the workspace (qtip_block_ldl_status); the
 // reference returns false in those cases.
@@ -46,14 +47,14 @@ __global__ void ldl_symmetrise_kernel(const float* __restrict__ H, double* __res
   }
 }
 
-// Cholesky of a kb x kb block (kb a multiple of 16, at most 128) in shared memory, lower triangle, by 256 threads. Sixteen
+// Cholesky of a kb x kb block (kb a multiple of 16, at most 128) in shared memory, packed lower triangle, by 256 threads. Sixteen
 // columns at a time: one warp factors the 16 x 16 diagonal block with a row per lane in registers and inverts it (a column
 // per lane), then all warps take the rows below it through the inverse and update what is right of it. The inverses, which
 // the panel kernel and the final block scaling need as well, go to `inv` (256 values a block, row-major, zeros above the
 // diagonal).
-constexpr int kLd = kNb + 1;
+constexpr int kLd = kNb + 1;  // L11 in the panel kernel
 constexpr int kInvLd = 17;
-__device__ __forceinline__ void factor_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ int tri(int i) { return i * (i + 1) / 2; }  // first word of row i of a packed lower triangle
 __device__ __forceinline__ void chol_factor(double* __restrict__ S, double* __restrict__ inv_s, int kb,
                                             double* __restrict__ inv, int* status) {
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -62,7 +63,7 @@ __device__ __forceinline__ void chol_factor(double* __restrict__ S, double* __re
       const int i = tid & 15;
       double a[16];
 #pragma unroll
-      for (int c = 0; c < 16; ++c) a[c] = c <= i ? S[(base + i) * kLd + base + c] : 0.0;
+      for (int c = 0; c < 16; ++c) a[c] = c <= i ? S[tri(base + i) + base + c] : 0.0;
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const double d = __shfl_sync(0xffffffffu, a[j], j);
@@ -85,13 +86,13 @@ __device__ __forceinline__ void chol_factor(double* __restrict__ S, double* __re
       if (tid < 16) {
 #pragma unroll
         for (int c = 0; c < 16; ++c) {
-          if (c <= i) S[(base + i) * kLd + base + c] = a[c];
+          if (c <= i) S[tri(base + i) + base + c] = a[c];
           inv_s[c * kInvLd + i] = col[c];
           inv[(base / 16) * 256 + c * 16 + i] = col[c];
         }
       }
     }
-    factor_sync();
+    __syncthreads();
     // rows below: x = a inv^T
     const int below = kb - base - 16;
     double x[7];
@@ -101,48 +102,51 @@ __device__ __forceinline__ void chol_factor(double* __restrict__ S, double* __re
       double t = 0.0;
       if (r < below) {
 #pragma unroll
-        for (int p = 0; p < 16; ++p) t = fma(S[(base + 16 + r) * kLd + base + p], inv_s[tx * kInvLd + p], t);
+        for (int p = 0; p < 16; ++p) t = fma(S[tri(base + 16 + r) + base + p], inv_s[tx * kInvLd + p], t);
       }
       x[a] = t;
     }
-    factor_sync();
+    __syncthreads();
 #pragma unroll
     for (int a = 0; a < 7; ++a)
-      if (ty + 16 * a < below) S[(base + 16 + ty + 16 * a) * kLd + base + tx] = x[a];
-    factor_sync();
+      if (ty + 16 * a < below) S[tri(base + 16 + ty + 16 * a) + base + tx] = x[a];
+    __syncthreads();
     // right of it: a[i][c] -= sum_p x[i][p] x[c][p], 16 x 16 blocks on and below the diagonal
     for (int a = 0; 16 * a < below; ++a) {
-      double* row = S + (base + 16 + ty + 16 * a) * kLd + base;
+      double* row = S + tri(base + 16 + ty + 16 * a) + base;
       double xi[16];
 #pragma unroll
       for (int p = 0; p < 16; ++p) xi[p] = row[p];
       for (int b = 0; b <= a; ++b) {
-        const double* xc = S + (base + 16 + tx + 16 * b) * kLd + base;
+        const double* xc = S + tri(base + 16 + tx + 16 * b) + base;
         double t0 = 0.0, t1 = 0.0;
 #pragma unroll
         for (int p = 0; p < 16; p += 2) t0 = fma(xi[p], xc[p], t0), t1 = fma(xi[p + 1], xc[p + 1], t1);
-        row[16 + tx + 16 * b] -= t0 + t1;  // above the diagonal of a diagonal block: never read
+        if (b < a || tx <= ty) row[16 + tx + 16 * b] -= t0 + t1;
       }
     }
-    factor_sync();
+    __syncthreads();
   }
 }
-__device__ __forceinline__ void chol_store(const double* __restrict__ S, double* __restrict__ A, long n, long k, int kb) {
+// The diagonal block at (k, k): loaded, factored, stored by a CTA of 256 threads.
+__device__ __forceinline__ void chol_diagonal(double* __restrict__ A, long n, long k, double* __restrict__ sm,
+                                              double* __restrict__ inv, int* status) {
+  const int kb = int(min(long(kNb), n - k));
   for (int idx = threadIdx.x; idx < kb * kb; idx += blockDim.x) {
     const int i = idx / kb, j = idx - i * kb;
-    if (j <= i) A[(k + i) * n + k + j] = S[i * kLd + j];
-  }
-}
-__global__ __launch_bounds__(256) void chol_first_kernel(double* __restrict__ A, long n, int kb, double* __restrict__ inv,
-                                                         int* status) {
-  extern __shared__ double sm[];
-  for (int idx = threadIdx.x; idx < kb * kb; idx += blockDim.x) {
-    const int i = idx / kb, j = idx - i * kb;
-    sm[i * kLd + j] = j <= i ? A[i * n + j] : 0.0;
+    if (j <= i) sm[tri(i) + j] = A[(k + i) * n + k + j];
   }
   __syncthreads();
-  chol_factor(sm, sm + kNb * kLd, kb, inv, status);
-  chol_store(sm, A, n, 0, kb);
+  chol_factor(sm, sm + tri(kNb), kb, inv, status);
+  for (int idx = threadIdx.x; idx < kb * kb; idx += blockDim.x) {
+    const int i = idx / kb, j = idx - i * kb;
+    if (j <= i) A[(k + i) * n + k + j] = sm[tri(i) + j];
+  }
+}
+__global__ __launch_bounds__(256) void chol_first_kernel(double* __restrict__ A, long n, double* __restrict__ inv,
+                                                         int* status) {
+  extern __shared__ double sm[];
+  chol_diagonal(A, n, 0, sm, inv, status);
 }
 
 // Rows r0 + [64 b, 64 b + 64): x L11^T = a. Thread (ty, tx) holds rows ty + 16 a and columns tx + 16 j in registers. Sixteen
@@ -201,40 +205,31 @@ __global__ __launch_bounds__(256) void chol_panel_kernel(double* __restrict__ A,
       if (ty + 16 * a < rows) A[(r0 + ty + 16 * a) * n + k + tx + 16 * j] = acc[a][j];
 }
 
-// C[i][j] -= sum_p P[i][p] P[j][p] for the tile (ti, tj), tj <= ti, of the trailing matrix that starts at row / column
-// r0; P = A[r0.., k .. k + 128). Sixteen warps as 4 x 4, each 32 x 32 outputs as 4 x 4 fp64 tensor-core fragments
+// C[i][j] -= sum_p P[i][p] P[j][p] for a 128 x 64 tile of the lower triangle of the trailing matrix that starts at row /
+// column r0; P = A[r0.., k .. k + 128). Eight warps as 4 x 2, each 32 x 32 outputs as 4 x 4 fp64 tensor-core fragments
 // (m8n8k4). The two operand panels pass through a ring of 16-column slices (cp.async; row stride 20 doubles: the 4 x 4
-// words that a half-warp reads for a fragment lie in 16 different bank pairs).
-// n = 12,288: all updates 66 ms with 8 x 8 outputs a thread and scalar multiply-adds, about 30 ms with the fragments.
-// Tile (0, 0) is the next diagonal block: its CTA, the first of the launch, factors it at once.
-constexpr int kSliceLd = kKc + 4, kSlices = kNb / kKc, kUpdThreads = 512, kUpdStages = 4;
-constexpr size_t kStageDoubles = size_t(2) * kTile * kSliceLd;
+// words that a half-warp reads for a fragment lie in 16 different bank pairs). Two CTAs share an SM, so that one reads and
+// writes its part of C while the other multiplies. n = 12,288, all updates: 66 ms with scalar multiply-adds and 8 x 8
+// outputs a thread, 29.9 ms with fragments and one 128 x 128 tile per SM, 27.2 ms so (the fp64 rate gives 16.6).
+// Tile row ti has 2 ti + 2 tiles. The first CTA takes both tiles of the next diagonal block and factors it at once.
+constexpr int kTileCols = 64, kSliceLd = kKc + 4, kSlices = kNb / kKc, kUpdThreads = 256, kUpdStages = 3;
+constexpr int kStageDoubles = (kTile + kTileCols) * kSliceLd;
 __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                : "+d"(c[0]), "+d"(c[1])
                : "d"(a), "d"(b));
 }
-__global__ __launch_bounds__(kUpdThreads, 1) void chol_update_kernel(double* __restrict__ A, long n, long k, long r0,
-                                                                     double* __restrict__ inv, int* status) {
-  extern __shared__ __align__(16) double upd_sm[];
-  double* sm = upd_sm;
-  // linear block index -> (ti, tj) of the lower triangle
-  const long t = blockIdx.x;
-  long ti = long((sqrt(8.0 * double(t) + 1.0) - 1.0) * 0.5);
-  while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-  while (ti * (ti + 1) / 2 > t) --ti;
-  const long tj = t - ti * (ti + 1) / 2;
-  const long i0 = r0 + ti * kTile, j0 = r0 + tj * kTile;
+__device__ __forceinline__ void chol_update_tile(double* __restrict__ A, long n, long k, long i0, long j0, double* sm) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
-  const int wi = (warp >> 2) * 32, wj = (warp & 3) * 32;
-  // a slice is 2 x 128 rows of 16 doubles = 2 x 1,024 copies of 16 bytes; rows past n repeat the last one and are not stored
+  const int wi = (warp >> 1) * 32, wj = (warp & 1) * 32;
+  // a slice is 128 + 64 rows of 16 doubles, 8 copies of 16 bytes a row; rows past n repeat the last one and are not stored
   auto stage = [&](int slice) {
-    double* dst = sm + size_t(slice % kUpdStages) * kStageDoubles;
+    double* dst = sm + (slice % kUpdStages) * kStageDoubles;
 #pragma unroll
-    for (int c = 0; c < 2 * kTile * kKc / 2 / kUpdThreads; ++c) {
-      const int idx = c * kUpdThreads + tid, side = idx >> 10, row = (idx >> 3) & 127, col = (idx & 7) * 2;
-      const long src = min((side ? j0 : i0) + row, n - 1);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + (side * kTile + row) * kSliceLd + col)),
+    for (int c = 0; c < (kTile + kTileCols) * kKc / 2 / kUpdThreads; ++c) {
+      const int idx = c * kUpdThreads + tid, row = idx >> 3, col = (idx & 7) * 2;
+      const long src = min(row < kTile ? i0 + row : j0 + row - kTile, n - 1);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + row * kSliceLd + col)),
                    "l"(A + src * n + k + slice * kKc + col));
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -252,8 +247,8 @@ __global__ __launch_bounds__(kUpdThreads, 1) void chol_update_kernel(double* __r
     __syncthreads();  // slice s is there for all, and everyone has left the stage that is filled next
     if (s + kUpdStages - 1 < kSlices) stage(s + kUpdStages - 1);
     else asm volatile("cp.async.commit_group;" ::: "memory");
-    const double* Pi = sm + size_t(s % kUpdStages) * kStageDoubles + (wi + g) * kSliceLd + q;
-    const double* Pj = sm + size_t(s % kUpdStages) * kStageDoubles + (kTile + wj + g) * kSliceLd + q;
+    const double* Pi = sm + (s % kUpdStages) * kStageDoubles + (wi + g) * kSliceLd + q;
+    const double* Pj = sm + (s % kUpdStages) * kStageDoubles + (kTile + wj + g) * kSliceLd + q;
 #pragma unroll
     for (int p = 0; p < kKc; p += 4) {
       double a[4], b[4];
@@ -264,24 +259,6 @@ __global__ __launch_bounds__(kUpdThreads, 1) void chol_update_kernel(double* __r
 #pragma unroll
         for (int y = 0; y < 4; ++y) dmma_8x8x4(acc[x][y], a[x], b[y]);
     }
-  }
-  if (t == 0) {
-    const int kb2 = int(min(long(kNb), n - r0));
-    __syncthreads();  // the ring becomes the block
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-      for (int y = 0; y < 4; ++y)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i = wi + 8 * x + g, j = wj + 8 * y + 2 * q + e;
-          if (i < kb2 && j <= i) sm[i * kLd + j] = A[(r0 + i) * n + r0 + j] - acc[x][y][e];
-        }
-    __syncthreads();
-    if (tid < 256) chol_factor(sm, sm + kNb * kLd, kb2, inv, status);
-    __syncthreads();
-    chol_store(sm, A, n, r0, kb2);
-    return;
   }
 #pragma unroll
   for (int x = 0; x < 4; ++x) {
@@ -299,6 +276,24 @@ __global__ __launch_bounds__(kUpdThreads, 1) void chol_update_kernel(double* __r
       c[y].x -= acc[x][y][0], c[y].y -= acc[x][y][1];
       if (j < n) *reinterpret_cast<double2*>(A + i * n + j) = c[y];  // above the diagonal: never read
     }
+  }
+}
+__global__ __launch_bounds__(kUpdThreads, 2) void chol_update_kernel(double* __restrict__ A, long n, long k, long r0,
+                                                                     double* __restrict__ inv, int* status) {
+  extern __shared__ __align__(16) double upd_sm[];
+  // linear block index -> tile row ti, tile column cj of the ti (ti + 1) + cj tiles in row order
+  const long t = blockIdx.x;
+  long ti = long((sqrt(4.0 * double(t) + 1.0) - 1.0) * 0.5);
+  while ((ti + 1) * (ti + 2) <= t) ++ti;
+  while (ti * (ti + 1) > t) --ti;
+  const long cj = t - ti * (ti + 1), j0 = r0 + cj * kTileCols;
+  if (t == 1 || j0 >= n) return;  // the first CTA's second tile; columns past the edge
+  chol_update_tile(A, n, k, r0 + ti * kTile, j0, upd_sm);
+  if (t == 0) {
+    __syncthreads();
+    if (r0 + kTileCols < n) chol_update_tile(A, n, k, r0, r0 + kTileCols, upd_sm);
+    __syncthreads();  // the block is in global memory, and the ring becomes its copy
+    chol_diagonal(A, n, r0, upd_sm, inv, status);
   }
 }
 
@@ -348,8 +343,9 @@ __global__ __launch_bounds__(128) void ldl_finish_kernel(const double* __restric
 }
 
 static size_t align256(size_t x) { return (x + 255) / 256 * 256; }
-constexpr size_t kFactorSmem = size_t(kNb * kLd + 16 * kInvLd) * 8;
-constexpr size_t kUpdSmem = kUpdStages * kStageDoubles * 8 > kFactorSmem ? kUpdStages * kStageDoubles * 8 : kFactorSmem;
+constexpr size_t kFactorSmem = size_t(kNb * (kNb + 1) / 2 + 16 * kInvLd) * 8;
+constexpr size_t kUpdSmem = size_t(kUpdStages) * kStageDoubles * 8;
+static_assert(kUpdSmem >= kFactorSmem, "the ring of the update is reused for the diagonal block");
 constexpr size_t kPanelSmem = size_t(kNb * kLd + (kNb / 16) * 16 * kInvLd + 2 * kPanelRows * kInvLd) * 8;
 
 int block_ldl_device_setup() {
@@ -389,14 +385,14 @@ extern "C" int qtip_block_ldl(const float* HR_d, long n, float* L_d, double* L64
     ldl_symmetrise_kernel<<<dim3(g, g), dim3(32, 8), 0, s>>>(HR_d, A, n);
     QB_LAUNCHED();
   }
-  chol_first_kernel<<<1, 256, kFactorSmem, s>>>(A, n, int(min(long(kNb), n)), inv, status);
+  chol_first_kernel<<<1, 256, kFactorSmem, s>>>(A, n, inv, status);
   QB_LAUNCHED();
   for (long k = 0; k + kNb < n; k += kNb) {
     const long r0 = k + kNb, nr = n - r0;
     chol_panel_kernel<<<blocks_for(nr, kPanelRows), 256, kPanelSmem, s>>>(A, n, k, inv + k / 16 * 256);
     QB_LAUNCHED();
     const long tiles = (nr + kTile - 1) / kTile;
-    chol_update_kernel<<<unsigned(tiles * (tiles + 1) / 2), kUpdThreads, kUpdSmem, s>>>(A, n, k, r0,
+    chol_update_kernel<<<unsigned(tiles * (tiles + 1)), kUpdThreads, kUpdSmem, s>>>(A, n, k, r0,
                                                                                          inv + r0 / 16 * 256, status);
     QB_LAUNCHED();
   }
