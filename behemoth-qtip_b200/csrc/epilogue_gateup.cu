@@ -10,6 +10,8 @@ template <int K>
 static int configure_out() {
   QB_CUDA(cudaFuncSetAttribute(had_row_gateup_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxRowFloats * 4));
   QB_CUDA(cudaFuncSetAttribute(had_chunk_gateup_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 8192 * 4));
+  if constexpr (kHasCluster<K>)
+    QB_CUDA(cudaFuncSetAttribute(had_cluster_gateup_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * kMaxRowFloats));
   return QTIP_OK;
 }
 int epilogue_gateup_device_setup() {
@@ -36,20 +38,26 @@ int hadamard_output_gateup(const float* z, int splits, long split_stride, int ro
   if (K <= 0) return K;
   QB_REQUIRE(K != 20, QTIP_E_GEOMETRY, "the fused epilogues carry the Hadamard orders 1, 12 and 28 (F = %d needs 20)", F);
   if (rows == 0) return QTIP_OK;
-  const bool chunks = K > 1 && rows < kChunkRowsBelow && a.P <= 8192;
-  QB_REQUIRE(chunks || 2L * F <= kMaxRowFloats, QTIP_E_GEOMETRY, "gate/up rows of 2 x %d floats do not fit a CTA", F);
+  const Path path = had_path(K, F, a.P, rows, kMaxRowFloats);
+  QB_REQUIRE((K > 1 && rows < kChunkRowsBelow && a.P <= 8192) || 2L * F <= kMaxRowFloats, QTIP_E_GEOMETRY, "gate/up rows of 2 x %d floats do not fit a CTA", F);
   QB_REQUIRE(rows <= 65535, QTIP_E_GEOMETRY, "too many rows");
   const int threads = a.P >= 1024 ? 1024 : (a.P < 64 ? 64 : a.P);
   const size_t chunk_smem = (size_t(a.P > 1024 ? a.P : 1024) + a.P) * 4, row_smem = size_t(F) * 8;
   // few rows: a link of a decode step's kernel chain (programmatic dependent launch, like the other chunk kernels)
 #define QB_GATEUP(K_)                                                                                                  \
-  if (chunks)                                                                                                          \
+  if (path == Path::Chunk)                                                                                                          \
     QB_CUDA(launch_chained(had_chunk_gateup_kernel<K_>, dim3(K_, unsigned(rows)), dim3(threads), chunk_smem, s, a, sv_up)); \
   else had_row_gateup_kernel<K_><<<unsigned(rows), 1024, row_smem, s>>>(a, sv_up)
   switch (K) {
     case 1: had_row_gateup_kernel<1><<<unsigned(rows), 1024, row_smem, s>>>(a, sv_up); break;
     case 12: QB_GATEUP(12); break;
-    default: QB_GATEUP(28); break;
+    default:
+      if (path == Path::Cluster) {
+        QB_CUDA(launch_cluster(had_cluster_gateup_kernel<28>, rows, size_t(F) * 3, s, a, sv_up));
+        break;
+      }
+      QB_GATEUP(28);
+      break;
   }
 #undef QB_GATEUP
   QB_LAUNCHED();

@@ -302,10 +302,11 @@ __device__ __forceinline__ void fwht_warp_1024(float (&v)[32]) {
       }
 }
 
-// FWHT of the K chunks (P = 1024 H floats each, H = 1 or 2) of a mixed row in shared memory, one 1,024-float unit per
-// warp at a time, results straight to the destination (H = 1) or after one more stage across the two halves (H = 2).
+// FWHT of K chunks (P = 1024 H floats each, H = 1 or 2; the row's chunks chunk0, chunk0 + 1, ...) of a mixed row in shared
+// memory, one 1,024-float unit per warp at a time, results straight to the destination (H = 1) or after one more stage
+// across the two halves (H = 2).
 template <int H, Mode M>
-__device__ __forceinline__ void row_chunks_warp(const HadArgs& a, long row, float* row_s, int K) {
+__device__ __forceinline__ void row_chunks_warp(const HadArgs& a, long row, float* row_s, int K, int chunk0 = 0) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   for (int u = warp; u < K * H; u += nwarps) {
     float* unit = row_s + u * 1024;
@@ -315,7 +316,7 @@ __device__ __forceinline__ void row_chunks_warp(const HadArgs& a, long row, floa
     fwht_warp_1024(v);
 #pragma unroll
     for (int r = 0; r < 32; ++r) {
-      if constexpr (H == 1) store_dst<M>(a, row, u * 1024 + 32 * r + lane, v[r]);
+      if constexpr (H == 1) store_dst<M>(a, row, (chunk0 * H + u) * 1024 + 32 * r + lane, v[r]);
       else unit[32 * r + lane] = v[r];
     }
   }
@@ -324,8 +325,8 @@ __device__ __forceinline__ void row_chunks_warp(const HadArgs& a, long row, floa
     for (int j = threadIdx.x; j < K * 1024; j += blockDim.x) {
       const int c = j >> 10, i = j & 1023;
       const float x = row_s[c * 2048 + i], y = row_s[c * 2048 + 1024 + i];
-      store_dst<M>(a, row, c * 2048 + i, x + y);
-      store_dst<M>(a, row, c * 2048 + 1024 + i, x - y);
+      store_dst<M>(a, row, (chunk0 + c) * 2048 + i, x + y);
+      store_dst<M>(a, row, (chunk0 + c) * 2048 + 1024 + i, x - y);
     }
   }
 }
@@ -473,30 +474,137 @@ __global__ __launch_bounds__(1024, 1) void had_chunk_gateup_kernel(HadArgs a, co
   }
 }
 
+// ---- a cluster of four CTAs per row: CTA q mixes columns [q P / 4, (q + 1) P / 4) of all K chunks, so the row is read
+// once, and pushes each mixed value through distributed shared memory to the CTA that owns its chunk (K / 4 whole chunks
+// per CTA); after one cluster barrier every CTA transforms and stores its own chunks. Bits as the other two kernels. For
+// rows of order 28 between the few whose latency the chunk kernel hides best and the many that give every SM a row of its
+// own: the chunk kernel reads a row 28 times, the whole-row kernel leaves most SMs idle (figures at had_path).
+constexpr int kHadCluster = 4, kClusterThreads = 256;
+
+__device__ __forceinline__ void had_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void had_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void had_cluster_sync() {
+  had_cluster_arrive();
+  had_cluster_wait();
+}
+__device__ __forceinline__ uint32_t had_peer(const void* p, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(uint32_t(rank)));
+  return r;
+}
+__device__ __forceinline__ void had_peer_store(uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+
+// work: K / 4 chunks of P floats in every CTA of the cluster, free in all of them when this is called.
+template <int K, bool T, Mode M>
+__device__ __forceinline__ void cluster_transform(const HadArgs& a, long row, float* work, int q) {
+  constexpr SignMasks<K, T> masks{};
+  constexpr int KC = K / kHadCluster;
+  const int P = a.P, cols = P / kHadCluster;
+  uint32_t peer[kHadCluster];
+#pragma unroll
+  for (int o = 0; o < kHadCluster; ++o) peer[o] = had_peer(work, o);
+  for (int i = q * cols + threadIdx.x; i < (q + 1) * cols; i += blockDim.x) {
+    float v[K];
+    load_column<K, M>(a, row, i, P, v);
+#pragma unroll
+    for (int r = 0; r < K; ++r)
+      had_peer_store(peer[r / KC] + uint32_t((r % KC) * P + i) * 4u, mix_row<K>(v, masks.m[r]));
+  }
+  had_cluster_sync();
+  if (P == 1024) return row_chunks_warp<1, M>(a, row, work, KC, q * KC);
+  if (P == 2048) return row_chunks_warp<2, M>(a, row, work, KC, q * KC);
+  fwht_shared(work, P, KC);
+  for (int j = threadIdx.x; j < KC * P; j += blockDim.x) store_dst<M>(a, row, q * KC * P + j, work[j]);
+}
+
+template <int K, bool T, Mode M>
+__global__ __cluster_dims__(kHadCluster, 1, 1) __launch_bounds__(kClusterThreads, 2) void had_cluster_kernel(HadArgs a) {
+  extern __shared__ float row_s[];
+  const int q = blockIdx.x;
+  const long row = blockIdx.y;
+  had_cluster_arrive();  // every CTA of the cluster runs before one stores into another
+  chain_release();
+  chain_wait();
+  if constexpr (M == Mode::PrepareNorm) {
+    __shared__ float slots[1024];
+    a.write_xn = true;  // a column is mixed by one CTA only
+    if (a.norm) a.factor = row_norm_factor<M>(a, row, slots);
+  }
+  had_cluster_wait();
+  cluster_transform<K, T, M>(a, row, row_s, q);
+}
+
+// Gate/up epilogue: the gate chunks stay in the CTA that owns them, the up chunks use a work area of their own (a peer may
+// still be reading the first one).
+template <int K>
+__global__ __cluster_dims__(kHadCluster, 1, 1) __launch_bounds__(kClusterThreads, 2) void had_cluster_gateup_kernel(
+    HadArgs a, const float* sign_up) {
+  extern __shared__ float row_s[];
+  const int q = blockIdx.x, own = a.n / kHadCluster;
+  const long row = blockIdx.y;
+  a.aux = row_s + 2 * own, a.aux_base = q * own;
+  had_cluster_arrive();
+  chain_release();
+  chain_wait();
+  had_cluster_wait();
+#pragma unroll 1
+  for (int phase = 0; phase < 2; ++phase) {
+    a.phase = phase;
+    cluster_transform<K, false, Mode::FinishGateUp>(a, row, row_s + phase * own, q);
+    __syncthreads();
+    a.src = static_cast<const float*>(a.src) + a.n;
+    a.sign = sign_up;
+  }
+}
+
 constexpr int kMaxRowFloats = 57344;  // 224 KiB of the 227 KiB a CTA may hold
-#ifndef QB_HAD_CHUNK_ROWS
-#define QB_HAD_CHUNK_ROWS 32
-#endif
-constexpr int kChunkRowsBelow = QB_HAD_CHUNK_ROWS;  // fewer rows than this: K CTAs per row
+constexpr int kChunkRowsBelow = 32;  // fewer rows than this: K CTAs per row
+// Kernel of a transform by its row count and shape; `room`: longest row of the whole-row kernel. A cluster per row from 16 to
+// 127 rows of order 28, measured on 28,672-wide rows in four splits (chunk or whole-row kernel against cluster, us): output
+// transform 28.9 / 13.7 at 31 rows, 21.0 / 14.6 at 64; gate/up epilogue 63.4 / 29.5 and 45.0 / 31.0; input transform
+// 20.9 / 10.6 at 31. At 13 rows in two splits they are level (25.1 / 24.1) and the chunk kernel is the better link of a
+// chain of launches; at 200 the whole-row kernel has a row for every SM (53.5 / 52.8, and 112 / 137 at 512). Order 12 has
+// less to gain from reading a row once (gate/up at 64 rows 27.1 / 21.8, at 200 47.9 / 64.7) and keeps the two kernels.
+enum class Path { Chunk, Cluster, Row };
+template <int K>
+constexpr bool kHasCluster = K == 28;
+static Path had_path(int K, int n, int P, long rows, int room) {
+  if (K == 28 && rows >= 16 && rows < 128 && P % (4 * kHadCluster) == 0 && n <= room) return Path::Cluster;
+  return K > 1 && rows < kChunkRowsBelow && P <= 8192 ? Path::Chunk : Path::Row;
+}
+// The kernels of a cluster are a link of the decode step's chain like the chunk kernels.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_cluster(void (*kernel)(Params...), long rows, size_t smem, cudaStream_t s, Args&&... args) {
+  return launch_chained(kernel, dim3(kHadCluster, unsigned(rows)), dim3(kClusterThreads), smem, s, args...);
+}
 
 template <int K, bool T, Mode M>
 static int configure() {
   QB_CUDA(cudaFuncSetAttribute(had_row_kernel<K, T, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (M == Mode::PrepareNorm ? kMaxRowFloats - 1024 : kMaxRowFloats) * 4));
   QB_CUDA(cudaFuncSetAttribute(had_chunk_kernel<K, T, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * 4));
+  if constexpr (kHasCluster<K> && M != Mode::F32Inplace)
+    QB_CUDA(cudaFuncSetAttribute(had_cluster_kernel<K, T, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxRowFloats));
   return QTIP_OK;
 }
 template <int K, bool T, Mode M>
 static int launch(const HadArgs& a, long rows, bool force_row, cudaStream_t s) {
   const int threads = a.P >= 1024 ? 1024 : (a.P < 64 ? 64 : a.P);
-  if (!force_row && K > 1 && rows < kChunkRowsBelow && a.P <= 8192) {
-    QB_REQUIRE(rows <= 65535, QTIP_E_GEOMETRY, "too many rows for the chunk kernel");
+  constexpr int kRoom = M == Mode::PrepareNorm ? kMaxRowFloats - 1024 : kMaxRowFloats;  // 4 KiB of static slots
+  const Path path = force_row ? Path::Row : had_path(K, a.n, a.P, rows, kRoom);
+  if constexpr (kHasCluster<K> && M != Mode::F32Inplace)
+    if (path == Path::Cluster) {
+      QB_CUDA(launch_cluster(had_cluster_kernel<K, T, M>, rows, size_t(a.n), s, a));
+      return QTIP_OK;
+    }
+  if (path == Path::Chunk) {
     // Few rows: a latency-bound link of a decode step's kernel chain, launched so that it can become resident while
     // the kernel before it drains (measured on the layer workload: 295 -> 279 us per layer at one token; the whole-row
     // kernels of larger batches lose 1 % when launched this way and keep the plain launch).
     QB_CUDA(launch_chained(had_chunk_kernel<K, T, M>, dim3(K, unsigned(rows)), dim3(threads), size_t(a.P) * 4, s, a));
   } else {
-    constexpr int kRoom = M == Mode::PrepareNorm ? kMaxRowFloats - 1024 : kMaxRowFloats;  // 4 KiB of static slots
     QB_REQUIRE(a.n <= kRoom, QTIP_E_GEOMETRY, "Hadamard rows longer than %d are not supported (n = %d)", kRoom, a.n);
     // Rows that leave room for several CTAs per SM run with fewer threads per row once there are rows for every SM:
     // the load, transform and store phases of different rows then overlap on each SM. Measured on 12288-wide fp32 rows:

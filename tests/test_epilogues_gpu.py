@@ -181,3 +181,56 @@ def test_large_batch_row_kernels_match_the_chunk_kernels(gpu, n):
         y_one = torch.empty(1, n, dtype=torch.bfloat16, device="cuda")
         lin.qtip_finish_b16(w, zb[r:r + 1].contiguous(), y_one, scratch, 1)
         assert torch.equal(y_big[r].view(torch.int16), y_one[0].view(torch.int16)), "bf16 output transform, row %d" % r
+
+
+@pytest.mark.parametrize("n,rows", [(448, 16), (896, 127), (3584, 33), (28672, 31), (28672, 64), (57344, 17)])
+def test_rows_of_order_28_match_single_rows(gpu, n, rows):
+    """16 to 127 rows of order 28 run on a cluster per row: every stage gives the bits of the same rows taken one at a time
+    (chunk kernel), K-splits, gathered sources and the normalised copy included."""
+    lin = gpu.linear
+    gen = torch.Generator(device="cuda").manual_seed(n + rows)
+    def randn(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda")
+    su, sv, sv2 = (torch.randint(0, 2, (n,), generator=gen, device="cuda").float() * 2 - 1 for _ in range(3))
+    w = lin.Matrix(None, su, sv, None, n, n)
+    x, norm = randn(rows, n).to(torch.bfloat16), (1 + 0.1 * randn(n)).to(torch.bfloat16)
+    one = lambda f: torch.cat([f(r) for r in range(rows)])  # noqa: E731
+    empty = lambda r: torch.empty(r, n, dtype=torch.bfloat16, device="cuda")  # noqa: E731
+
+    def prepare(t):
+        u = empty(t.shape[0])
+        lin.qtip_prepare(w, t.contiguous(), None, u, t.shape[0])
+        return u
+    assert torch.equal(prepare(x), one(lambda r: prepare(x[r:r + 1])))
+
+    def input_transform(t):
+        u, xn = empty(t.shape[0]), empty(t.shape[0])
+        lin.input_transform(t.contiguous(), norm, 1e-5, su, n, t.shape[0], u, xn)
+        return torch.cat([u, xn], 1)
+    if n < 57344:  # the norm's slots do not fit beside a row of 57,344
+        assert torch.equal(input_transform(x), one(lambda r: input_transform(x[r:r + 1])))
+
+    z = randn(2, rows, n)
+    def finish(t):
+        y = empty(t.shape[1])
+        lin.qtip_finish(w, t.contiguous(), y, None, True, t.shape[0], t.shape[1])
+        return y
+    assert torch.equal(finish(z), one(lambda r: finish(z[:, r:r + 1])))
+    gathered = z.view(2, rows, 2, n // 2).permute(0, 2, 1, 3).contiguous()  # [split][rank][row][n / 2]
+    y = empty(rows)
+    lin.qtip_finish(w, gathered, y, None, True, 2, rows, rank_major=2)
+    assert torch.equal(y, finish(z))
+
+    def residual(t, state):
+        state = state.contiguous().clone()
+        lin.output_residual(t.contiguous(), t.shape[0], t.shape[1], sv, n, state)
+        return state
+    assert torch.equal(residual(z, x), one(lambda r: residual(z[:, r:r + 1], x[r:r + 1])))
+
+    z2 = randn(2, rows, 2 * n)
+    def gateup(t):
+        h = empty(t.shape[1])
+        lin.output_gateup(t.contiguous(), t.shape[0], t.shape[1], sv, sv2, n, h)
+        return h
+    if 2 * n <= 57344 or rows < 32:
+        assert torch.equal(gateup(z2), one(lambda r: gateup(z2[:, r:r + 1])))
