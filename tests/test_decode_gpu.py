@@ -316,3 +316,13 @@ def test_fused_decode_tile_edges(gpu, oracle, n_in, n_out, tokens, splits):
     W = oracle.decode_rows(tr, n_in, n_out, tl, 0, n_out, True).astype(np.float64)
     ref = gpu.synth.bf16_bits_to_f32(xb).astype(np.float64) @ W.T
     assert rel_l2(z.sum(0).cpu().numpy(), ref) < 5e-6
+
+
+@pytest.mark.parametrize("n_in,n_out", [(32, 32), (288, 64), (480, 160), (224, 32 * 601), (8224, 96)])
+def test_decode_matrix_strip_edges(gpu, oracle, n_in, n_out):
+    """Strips of 256 columns: rows that end inside a strip, fewer strips than the groups of one CTA, and more than one round
+    of strips over all SMs (601 block-rows)."""
+    w, tr, su, sv, tl = make_linear(gpu, n_in, n_out, 300 + n_in)
+    out = torch.full((n_out, n_in), float("nan"), dtype=torch.bfloat16, device="cuda")
+    gpu.linear.qtip_decode_matrix(w, out)
+    assert np.array_equal(out.float().cpu().numpy(), oracle.decode_rows(tr, n_in, n_out, tl, 0, n_out, True))
