@@ -102,9 +102,11 @@ __device__ __forceinline__ void prefetch_run(const ItemCtx& c, int item, int n_i
 
 // One work item = one 32-row block-row x one K-split, shared by `nw` warps (this is warp `wi` of them): each warp takes
 // a contiguous run of 32x32 blocks, then the partial sums are added in warp order through `red` and written to z.
-template <int NT, bool XS, bool PUSH>
+// HALF (one token): only the 16 rows `half` of the block-row, at half the decode work for all of its code bytes.
+template <int NT, bool XS, bool PUSH, bool HALF = false>
 __device__ __forceinline__ void run_item(const ItemCtx& c, const TpPush& push, int item, int nw, int wi, int bar_id,
-                                         float* red) {
+                                         float* red, int half = 0) {
+  static_assert(!HALF || XS, "half block-rows are for one token");
   constexpr int RT = XS ? 1 : NT * 8;  // tokens kept per warp in the reduction buffer
   const int lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
   const uint32_t lane4 = uint32_t(lane) * 4u;
@@ -149,6 +151,11 @@ __device__ __forceinline__ void run_item(const ItemCtx& c, const TpPush& push, i
 #pragma unroll
     for (int j1 = 0; j1 < 2; ++j1) {
       uint32_t a[2][4];
+      if constexpr (HALF) {
+        decode_half(j1 ? own.y : own.x, j1 ? peer.y : peer.x, half != 0, lane4, a[0]);
+        mma_bf16_16816(acc[0][0], a[0], bw[0][2 * j1], bw[0][2 * j1 + 1]);
+        continue;
+      }
       decode_pair(j1 ? own.y : own.x, j1 ? peer.y : peer.x, lane4, a[0], a[1]);
 #pragma unroll
       for (int i1 = 0; i1 < 2; ++i1)
@@ -196,7 +203,7 @@ __device__ __forceinline__ void run_item(const ItemCtx& c, const TpPush& push, i
   if constexpr (XS) {
     if (tg == 0) {
 #pragma unroll
-      for (int i1 = 0; i1 < 2; ++i1) {
+      for (int i1 = 0; i1 < (HALF ? 1 : 2); ++i1) {
         wr[i1 * 16 + g] = acc[0][i1][0];
         wr[i1 * 16 + g + 8] = acc[0][i1][2];
       }
@@ -214,8 +221,8 @@ __device__ __forceinline__ void run_item(const ItemCtx& c, const TpPush& push, i
       }
   }
   warps_sync(bar_id, nw);
-  for (int o = wi * 32 + lane; o < RT * 32; o += nw * 32) {
-    const int tok = o >> 5, row = o & 31;
+  for (int o = wi * 32 + lane; o < (HALF ? 16 : RT * 32); o += nw * 32) {
+    const int tok = o >> 5, row = (o & 31) + (HALF ? half * 16 : 0);
     if (tok < c.tokens) {
       float s = red[o];
       for (int q = 1; q < nw; ++q) s += red[size_t(q) * RT * 32 + o];
@@ -303,7 +310,7 @@ __global__ __launch_bounds__(kGemmThreads, 1) void trellis_gemm_kernel(qtip_matr
   c.z = z;
   c.n2 = w.in / 32, c.in_words = w.in / 2, c.stride = stride, c.splits = splits;
   c.tokens_total = tokens_total, c.t0 = t0, c.tokens = tokens;
-  const int n_items = (w.out / 32) * splits;
+  int n_items = (w.out / 32) * splits;
   constexpr int ipc = IPC, wpi = (kGemmThreads / 32) / IPC;  // items per CTA at a time, warps per work item
   const int slots = gridDim.x * ipc;
   const int n_grouped = n_items / slots * slots;
@@ -315,7 +322,18 @@ __global__ __launch_bounds__(kGemmThreads, 1) void trellis_gemm_kernel(qtip_matr
   }
   prefetch_run(c, n_grouped + blockIdx.x, n_items, kGemmThreads / 32, warp);
   __syncthreads();
-  for (int item = n_grouped + blockIdx.x; item < n_items; item += gridDim.x)
+  const int rest = n_items - n_grouped, grid = gridDim.x;
+  // A last round that has work for at most half of the CTAs goes out in half block-rows, one per CTA: they read all of the
+  // code bytes for half of the decode work, so the round costs well under a unit (57344 x 12288, 12 units and 16 items: 94.7
+  // -> 90.8 us). More than one round of them is no gain (12288 x 28672 in two splits, 352 halves for 176 items: 55.8 -> 56.9).
+  if constexpr (XS) {
+    if (2 * rest <= grid) {
+      for (int u = blockIdx.x; u < 2 * rest; u += grid)  // at most one
+        run_item<NT, XS, PUSH, true>(c, push, n_grouped + (u >> 1), kGemmThreads / 32, warp, 0, red, u & 1);
+      n_items = n_grouped;
+    }
+  }
+  for (int item = n_grouped + blockIdx.x; item < n_items; item += grid)
     run_item<NT, XS, PUSH>(c, push, item, kGemmThreads / 32, warp, 0, red);
   if constexpr (PUSH) {
     // The barrier orders every thread's peer stores before thread 0's fence (fences are cumulative), the fence orders

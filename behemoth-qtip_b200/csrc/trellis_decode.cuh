@@ -53,5 +53,12 @@ __device__ __forceinline__ void decode_pair(uint32_t o, uint32_t p, uint32_t lan
   }
 #endif
 }
+// One of the two windows only: `upper` (the same for the whole warp) takes the tile i1 = 1.
+__device__ __forceinline__ void decode_half(uint32_t o, uint32_t p, bool upper, uint32_t lane4, uint32_t (&v)[4]) {
+  const uint32_t first = upper ? o >> 16 : o, next = upper ? p : p << 16;
+  v[0] = lut_word(first, lane4);
+#pragma unroll
+  for (int k = 1; k < 4; ++k) v[k] = lut_word(__funnelshift_l(next, first, 4 * k), lane4);
+}
 
 }  // namespace qb
