@@ -112,7 +112,7 @@ def qtip_multiply_batch(w, x, z, stride, splits, tokens, implementation=-1):
 
 
 def qtip_multiply_tc(w, x, z, stride, splits, tokens, status=None):
-    """Decode fused into the tcgen05 product (17 .. a few hundred tokens); z [splits, tokens, stride] fp32."""
+    """Decode fused into the tcgen05 product (9 .. a few hundred tokens); z [splits, tokens, stride] fp32."""
     init()
     lib().call("qtip_multiply_tc", w.pod, _p(x, torch.bfloat16), _p(z, torch.float32), stride, splits, tokens,
                _p(status, torch.int32), _stream())
