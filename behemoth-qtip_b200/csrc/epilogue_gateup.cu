@@ -39,13 +39,14 @@ int hadamard_output_gateup(const float* z, int splits, long split_stride, int ro
   QB_REQUIRE(K != 20, QTIP_E_GEOMETRY, "the fused epilogues carry the Hadamard orders 1, 12 and 28 (F = %d needs 20)", F);
   if (rows == 0) return QTIP_OK;
   const Path path = had_path(K, F, a.P, rows, kMaxRowFloats);
-  QB_REQUIRE((K > 1 && rows < kChunkRowsBelow && a.P <= 8192) || 2L * F <= kMaxRowFloats, QTIP_E_GEOMETRY, "gate/up rows of 2 x %d floats do not fit a CTA", F);
+  QB_REQUIRE((K > 1 && rows < kChunkRowsBelow && a.P <= 8192) || 2L * F <= kMaxRowFloats, QTIP_E_GEOMETRY,
+             "gate/up rows of 2 x %d floats do not fit a CTA", F);
   QB_REQUIRE(rows <= 65535, QTIP_E_GEOMETRY, "too many rows");
   const int threads = a.P >= 1024 ? 1024 : (a.P < 64 ? 64 : a.P);
   const size_t chunk_smem = (size_t(a.P > 1024 ? a.P : 1024) + a.P) * 4, row_smem = size_t(F) * 8;
   // few rows: a link of a decode step's kernel chain (programmatic dependent launch, like the other chunk kernels)
 #define QB_GATEUP(K_)                                                                                                  \
-  if (path == Path::Chunk)                                                                                                          \
+  if (path == Path::Chunk)                                                                                             \
     QB_CUDA(launch_chained(had_chunk_gateup_kernel<K_>, dim3(K_, unsigned(rows)), dim3(threads), chunk_smem, s, a, sv_up)); \
   else had_row_gateup_kernel<K_><<<unsigned(rows), 1024, row_smem, s>>>(a, sv_up)
   switch (K) {

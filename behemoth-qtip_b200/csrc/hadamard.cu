@@ -2,12 +2,13 @@
 //
 // (hadK (x) H_P) = (I (x) H_P)(hadK (x) I): the order-K mix across the K chunks is done first, then a natural-order
 // fast Walsh-Hadamard transform on each chunk of P. Every variant below uses that order and the same summation order,
-// so the whole-row kernel and the chunk-per-CTA kernel give identical bits.
+// so the kernels give identical bits.
 //
 //  * had_row_kernel: one CTA per row, the whole row (up to 57,344 floats = 224 KiB) in shared memory, read and written
 //    once. Used for the quantizer's fp32 matrices and for prefill-sized token batches.
 //  * had_chunk_kernel: K CTAs per row, each mixing its own chunk from the full row (served by L2) and transforming it.
 //    No inter-CTA step; used for a few tokens where latency, not traffic, decides.
+//  * had_cluster_kernel: a cluster of four CTAs per row for 16 to 127 rows of order 28 (see had_path).
 //
 // Sources/destinations (Mode): fp32 in place (quantizer); bf16 x times SU -> bf16 (operator input); fp32 partial
 // products summed over K-splits, optionally rounded to bf16 -> times SV -> bf16 (operator output); bf16 z -> same.
