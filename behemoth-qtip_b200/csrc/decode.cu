@@ -582,12 +582,11 @@ extern "C" int qtip_multiply_batch(qtip_matrix w, const uint16_t* x_d, float* z_
   // implementation: 0 = MMA-fragment kernel (16 tokens per pass), 2 = decode fused into the tcgen05 product, other
   // values = by batch size and shape (below).
   const bool fused_ok = w.in % 64 == 0 && w.out % 128 == 0 && reinterpret_cast<uintptr_t>(x_d) % 16 == 0;
-  // By batch size: from 9 tokens. The fragment kernel's work grows with the token columns it keeps in registers, the fused
-  // one's does not (13 tokens: 57344 x 12288 190 us against 123, 12288 x 28672 108 against 58, 12288 x 12288 51 against 28).
-  // Below, with half the columns and 32-row work items that fill the SMs at any number of K-splits, the fragment kernel is
-  // as fast or faster at the K-splits that callers use there (8 tokens, 57344 x 12288 in one split: 126 us; 12288 x 12288
-  // in two: 36 us both).
-  const bool fused_pays = tokens > 8;
+  // By batch size: above 16 tokens always; from 9 tokens for matrices of up to 16,384 rows, which callers split along K
+  // (12288 x 12288 at 16 tokens in three splits: 28 us against 52 us). Wider ones come in one split, and there the fused
+  // kernel adds the whole K range in one chain where the fragment kernel adds eight or more partial sums: 57344 x 12288 at
+  // 13 tokens 138 us against 190 us, but z is 1.4e-5 away from its value in 64 bits against 1.6e-6.
+  const bool fused_pays = tokens > 16 || (tokens > 8 && w.out <= 16384);
   if (implementation == 2 || (implementation != 0 && fused_pays && fused_ok)) {
     if (!device_info()) return QTIP_E_DEVICE;
     return trellis_tc_multiply(w, x_d, z_d, stride, splits, tokens, nullptr, as_stream(stream));

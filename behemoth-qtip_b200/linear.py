@@ -126,8 +126,7 @@ def tc_splits(n_out, sm_count=148, max_splits=4):
 
 
 def batch_uses_tc(n_in, n_out, tokens):
-    """Batches whose K-splits are best chosen by tc_splits. (qtip_multiply_batch takes the fused kernel from 9 tokens for every
-    width that it can run; up to 16 tokens of more than 16,384 rows, one split already fills most SMs.)"""
+    """The rule by which qtip_multiply_batch (implementation = -1) takes the fused tensor-core kernel."""
     return n_in % 64 == 0 and n_out % 128 == 0 and (tokens > 16 or (tokens > 8 and n_out <= 16384))
 
 

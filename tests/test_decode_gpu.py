@@ -345,3 +345,21 @@ def test_one_token_short_last_round(gpu, oracle, n_in, n_out, splits):
     again = torch.zeros_like(z)
     gpu.linear.qtip_multiply(w, bf16_dev(xb), again, n_out, splits)
     assert torch.equal(z, again)
+
+
+@pytest.mark.parametrize("n_in,n_out,tokens", [(1024, 16512, 16), (3584, 16512, 13), (12288, 20480, 9)])
+def test_wide_batches_keep_their_partial_sums(gpu, n_in, n_out, tokens):
+    """9 to 16 tokens of more than 16,384 rows in one split: eight warps add an eighth of the K range each, in steps of 16
+    columns. A step drops less than 2^-23 of its running sum, so the products stay within n_in / 8 / 16 x 2^-24 (steps times
+    half of that) of float64 on the decoded weights; one chain over all of K is about eight times further off. And the bits
+    are those of the 16-token kernel."""
+    w, *_ = make_linear(gpu, n_in, n_out, 700 + tokens)
+    x = torch.randn(tokens, n_in, generator=torch.Generator(device="cuda").manual_seed(tokens), device="cuda").to(torch.bfloat16)
+    z, z0 = (torch.full((1, tokens, n_out), float("nan"), dtype=torch.float32, device="cuda") for _ in range(2))
+    gpu.linear.qtip_multiply_batch(w, x, z, n_out, 1, tokens)
+    gpu.linear.qtip_multiply_batch(w, x, z0, n_out, 1, tokens, 0)
+    dense = torch.empty(n_out, n_in, dtype=torch.bfloat16, device="cuda")
+    gpu.linear.qtip_decode_matrix(w, dense)
+    ref = x.double() @ dense.double().T
+    assert float((z[0].double() - ref).norm() / ref.norm()) < max(8, n_in // 128) * 2.0 ** -24
+    assert torch.equal(z, z0)
