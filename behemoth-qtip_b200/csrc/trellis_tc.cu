@@ -43,16 +43,28 @@ struct FtSmem {
 // TMEM: one or two accumulators of d_cols columns, then the A ring. Shared memory: table, activation ring, barriers.
 // 128-column steps halve the barrier round trips per column; above 128 tokens their activation tiles leave no room for a
 // ring. Rows that are an odd number of 64-column slices take 64-column steps.
+// Where the K-splits are cut is part of the result: it decides which sums are chains of their own. Up to 64 tokens the cuts
+// lie between 128 columns (where those divide the row), above between 64. With 128-column steps a cut may then fall into a
+// step (`halves`): both splits run it, and the MMA thread leaves out the half that is not theirs. A kernel of its own, because
+// the test in the MMA thread costs every other shape 4 %; 12288 x 28672 in three splits at 65 / 128 tokens: 65 / 80 us, 91 / 96 with
+// 64-column steps.
 struct FtConfig {
-  int ksub;  // 64-column slices per K step
+  int ksub;     // 64-column slices per K step
+  bool halves;  // some cut is in the middle of a step
+  int cuts;     // possible cuts of a row
   int n_tile, tok_tiles, d_cols, d_bufs, a_stages, b_stages;
 };
 constexpr size_t kFtMaxSmem = 227 * 1024;
-static FtConfig ft_config(int tokens, int n_in) {
+static FtConfig ft_config(int tokens, int n_in, int splits) {
   FtConfig c;
   c.tok_tiles = (tokens + 255) / 256;
   c.n_tile = ((tokens + c.tok_tiles - 1) / c.tok_tiles + 15) / 16 * 16;  // M128 wants N in steps of 16
   c.ksub = c.n_tile <= 128 && n_in % 128 == 0 ? 2 : 1;
+  const int slices = n_in / 64;
+  c.halves = false;
+  for (int sp = 1; c.ksub == 2 && tokens > 64 && sp < splits && sp < slices; ++sp)
+    c.halves = c.halves || (long(slices) * sp / min(splits, slices)) % 2 != 0;
+  c.cuts = c.ksub == 2 && !c.halves ? slices / 2 : slices;
   c.d_cols = (c.n_tile + 31) / 32 * 32;
   c.d_bufs = c.n_tile <= 128 ? 2 : 1;
   c.a_stages = min(kFtMaxStages, (kFtTmemCols - c.d_bufs * c.d_cols) / (32 * c.ksub));  // at least kFtSlots
@@ -85,7 +97,10 @@ __device__ __forceinline__ void tc_mma_tmem_a(uint32_t d_tmem, uint32_t a_tmem, 
 // One work item = 128 output rows x one token tile x one K-split.
 struct FtItem {
   int row0, tok0, split, ks_lo, steps;
+  bool lo_odd, hi_odd;  // only the second half of the first step, only the first half of the last one
 };
+// k_total: possible cuts of a row
+template <bool HALVES>
 __device__ __forceinline__ FtItem ft_item(int item, int tok_tiles, int splits, int k_total, int n_tile) {
   FtItem it;
   it.split = item % splits;
@@ -94,25 +109,32 @@ __device__ __forceinline__ FtItem ft_item(int item, int tok_tiles, int splits, i
   it.row0 = (t / tok_tiles) * kFtRows;
   it.ks_lo = int(long(k_total) * it.split / splits);
   it.steps = int(long(k_total) * (it.split + 1) / splits) - it.ks_lo;  // >= 1: the host keeps splits <= k_total
+  it.lo_odd = it.hi_odd = false;
+  if constexpr (HALVES) {  // cut between the 64-column slices of 128-column steps
+    const int lo = it.ks_lo, hi = lo + it.steps;
+    it.ks_lo = lo >> 1, it.steps = ((hi + 1) >> 1) - it.ks_lo;
+    it.lo_odd = lo & 1, it.hi_odd = hi & 1;
+  }
   return it;
 }
 struct FtGeom {
   int n_items, stride, tok_tiles, splits, k_total, n_tile;
 };
 // Walks K steps k0, k0 + by, ... of this CTA's items (item = CTA, CTA + grid, ...) as one long sequence.
+template <bool HALVES>
 struct FtWalk {
   int item, k;
   FtItem cur;
   __device__ __forceinline__ void start(const FtGeom& g, int k0) {
     item = blockIdx.x, k = k0;
-    cur = ft_item(item, g.tok_tiles, g.splits, g.k_total, g.n_tile);  // the grid has at most n_items CTAs
+    cur = ft_item<HALVES>(item, g.tok_tiles, g.splits, g.k_total, g.n_tile);  // the grid has at most n_items CTAs
     settle(g);
   }
   __device__ __forceinline__ void settle(const FtGeom& g) {
     while (item < g.n_items && k >= cur.steps) {
       k -= cur.steps;
       item += g.stride;
-      if (item < g.n_items) cur = ft_item(item, g.tok_tiles, g.splits, g.k_total, g.n_tile);
+      if (item < g.n_items) cur = ft_item<HALVES>(item, g.tok_tiles, g.splits, g.k_total, g.n_tile);
     }
   }
   __device__ __forceinline__ void advance(const FtGeom& g, int by) {
@@ -130,7 +152,7 @@ struct FtRing {
 };
 
 // Persistent: grid = min(SMs, items); CTA c takes items c, c + grid, ... z[(split * tokens + token) * stride + row].
-template <int KSUB>
+template <int KSUB, bool HALVES>
 __global__ __launch_bounds__(kFtThreads, 1) void trellis_tc_kernel(qtip_matrix w, const __grid_constant__ CUtensorMap map_x,
                                                                    float* __restrict__ z, int stride, int tokens,
                                                                    const FtConfig cfg, int splits, int n_items,
@@ -145,7 +167,7 @@ __global__ __launch_bounds__(kFtThreads, 1) void trellis_tc_kernel(qtip_matrix w
   const int warp = tc_warp(), lane = threadIdx.x & 31;
   FtGeom geo;
   geo.n_items = n_items, geo.stride = gridDim.x, geo.tok_tiles = cfg.tok_tiles, geo.splits = splits;
-  geo.k_total = w.in / kFtK, geo.n_tile = cfg.n_tile;
+  geo.k_total = HALVES ? w.in / 64 : w.in / kFtK, geo.n_tile = cfg.n_tile;
   volatile int* abort_flag = &sm.abort_flag;
 
   chain_release();
@@ -191,7 +213,7 @@ __global__ __launch_bounds__(kFtThreads, 1) void trellis_tc_kernel(qtip_matrix w
     const uint2* codes = reinterpret_cast<const uint2*>(w.trellis) + lane + size_t(quarter) * row_units;
     constexpr int kAhead = 4 / KSUB;  // own steps of codes in flight per lane
     uint2 next[kAhead][2 * KSUB];
-    FtWalk use, pre;  // the step being decoded, and the step whose codes are being requested (kAhead own steps later)
+    FtWalk<HALVES> use, pre;  // the step being decoded, and the step whose codes are being requested (kAhead own steps later)
     use.start(geo, slot);
     pre = use;
     auto place = [&]() {  // past the last item: a harmless re-read of its first blocks
@@ -252,7 +274,7 @@ __global__ __launch_bounds__(kFtThreads, 1) void trellis_tc_kernel(qtip_matrix w
     // ---- TMA producer of the activation tiles
     if (tc_elect()) {
       chain_wait();  // the activations may come from the kernel before this one
-      FtWalk wk;
+      FtWalk<HALVES> wk;
       wk.start(geo, 0);
       FtRing ring{0, 0}, rb{0, 0}, before{0, 0};  // the step, its place in the activation ring, the step that held the place
       int filled = 0;
@@ -275,12 +297,13 @@ __global__ __launch_bounds__(kFtThreads, 1) void trellis_tc_kernel(qtip_matrix w
     // ---- MMA issuer
     if (tc_elect()) {
       const uint32_t idesc = tc_idesc(kFtRows, cfg.n_tile);
-      FtWalk wk;
+      FtWalk<HALVES> wk;
       wk.start(geo, 0);
       FtRing ra{0, 0}, rb{0, 0}, rd{0, 0};
       bool ok = true;
       while (wk.item < n_items && ok) {
         const int steps = wk.cur.steps;
+        const bool lo_odd = HALVES && wk.cur.lo_odd, hi_odd = HALVES && wk.cur.hi_odd;
         ok = tc_wait(smem_u32(&sm.acc_empty[rd.stage]), uint32_t(rd.phase ^ 1), abort_flag, status);
         if (!ok) break;
         for (int k = 0; k < steps; ++k) {
@@ -289,9 +312,10 @@ __global__ __launch_bounds__(kFtThreads, 1) void trellis_tc_kernel(qtip_matrix w
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
           for (int kk = 0; kk < kFtK / 16; ++kk) {
+            if (HALVES && (kk < 4 ? lo_odd && k == 0 : hi_odd && k == steps - 1)) continue;
             const uint64_t b_desc = tc_smem_desc(b_ring + uint32_t(rb.stage) * b_bytes + uint32_t((kk >> 2) * cfg.n_tile) * 128u);
             tc_mma_tmem_a(tmem + uint32_t(rd.stage * cfg.d_cols), a_tmem + uint32_t(ra.stage * kFtACols + 8 * kk),
-                          b_desc + uint64_t(2 * (kk & 3)), idesc, k > 0 || kk > 0);
+                          b_desc + uint64_t(2 * (kk & 3)), idesc, k > 0 || kk > (HALVES && lo_odd ? 4 : 0));
           }
           tc_commit(smem_u32(&sm.empty[ra.stage]));
           ra.advance(1, cfg.a_stages);
@@ -308,7 +332,7 @@ __global__ __launch_bounds__(kFtThreads, 1) void trellis_tc_kernel(qtip_matrix w
     const int quarter = warp & 3;
     FtRing rd{0, 0};
     for (int item = blockIdx.x; item < n_items; item += gridDim.x, rd.advance(1, cfg.d_bufs)) {
-      const FtItem it = ft_item(item, cfg.tok_tiles, splits, geo.k_total, cfg.n_tile);
+      const FtItem it = ft_item<HALVES>(item, cfg.tok_tiles, splits, geo.k_total, cfg.n_tile);
       if (!__all_sync(0xffffffffu, tc_wait(smem_u32(&sm.acc_full[rd.stage]), uint32_t(rd.phase), abort_flag, status))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       float* zs = z + (size_t(it.split) * tokens + it.tok0) * stride + it.row0 + quarter * 32 + lane;
@@ -344,8 +368,9 @@ __global__ __launch_bounds__(kFtThreads, 1) void trellis_tc_kernel(qtip_matrix w
 }
 
 int trellis_tc_device_setup() {
-  QB_CUDA(cudaFuncSetAttribute(trellis_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFtMaxSmem)));
-  QB_CUDA(cudaFuncSetAttribute(trellis_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFtMaxSmem)));
+  QB_CUDA(cudaFuncSetAttribute(trellis_tc_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFtMaxSmem)));
+  QB_CUDA(cudaFuncSetAttribute(trellis_tc_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFtMaxSmem)));
+  QB_CUDA(cudaFuncSetAttribute(trellis_tc_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFtMaxSmem)));
   return QTIP_OK;
 }
 
@@ -354,7 +379,7 @@ int trellis_tc_multiply(qtip_matrix w, const uint16_t* x, float* z, int stride, 
   QB_REQUIRE(w.in % 64 == 0 && w.out % kFtRows == 0, QTIP_E_GEOMETRY,
              "the fused tensor-core product needs in %% 64 == 0 and out %% 128 == 0 (in = %d, out = %d)", w.in, w.out);
   QB_REQUIRE(reinterpret_cast<uintptr_t>(x) % 16 == 0, QTIP_E_ARG, "activations must be 16-byte aligned");
-  const FtConfig cfg = ft_config(tokens, w.in);
+  const FtConfig cfg = ft_config(tokens, w.in, splits);
   CUtensorMap map_x;
   int rc = tc_make_map(&map_x, x, uint64_t(tokens), uint64_t(w.in), uint32_t(cfg.n_tile));
   if (rc) return rc;
@@ -365,15 +390,17 @@ int trellis_tc_multiply(qtip_matrix w, const uint16_t* x, float* z, int stride, 
   }
   const DeviceInfo* info = device_info();
   if (!info) return QTIP_E_DEVICE;
-  // More K-splits than K steps: the surplus slices of z hold zeros, the kernel runs with one step per split.
-  const int k_total = w.in / (64 * cfg.ksub), eff = splits < k_total ? splits : k_total;
+  // More K-splits than cuts: the surplus slices of z hold zeros, the kernel runs with one cut per split.
+  const int eff = splits < cfg.cuts ? splits : cfg.cuts;
   if (eff < splits)
     QB_CUDA(cudaMemsetAsync(z + size_t(eff) * tokens * stride, 0, size_t(splits - eff) * tokens * stride * sizeof(float), s));
   const long items = long(w.out / kFtRows) * cfg.tok_tiles * eff;
   QB_REQUIRE(items < (1l << 30), QTIP_E_GEOMETRY, "too many work items (%ld)", items);
   const int grid = int(items < info->sm_count ? items : info->sm_count);
-  QB_CUDA(launch_chained(cfg.ksub == 2 ? trellis_tc_kernel<2> : trellis_tc_kernel<1>, dim3(grid), dim3(kFtThreads),
-                         ft_smem(cfg), s, w, map_x, z, stride, tokens, cfg, eff, int(items), status));
+  const auto kernel = cfg.halves ? trellis_tc_kernel<2, true>
+                      : cfg.ksub == 2 ? trellis_tc_kernel<2, false> : trellis_tc_kernel<1, false>;
+  QB_CUDA(launch_chained(kernel, dim3(grid), dim3(kFtThreads), ft_smem(cfg), s, w, map_x, z, stride, tokens, cfg, eff,
+                         int(items), status));
   return QTIP_OK;
 }
 

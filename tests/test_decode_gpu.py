@@ -363,3 +363,21 @@ def test_wide_batches_keep_their_partial_sums(gpu, n_in, n_out, tokens):
     ref = x.double() @ dense.double().T
     assert float((z[0].double() - ref).norm() / ref.norm()) < max(8, n_in // 128) * 2.0 ** -24
     assert torch.equal(z, z0)
+
+
+@pytest.mark.parametrize("n_in,n_out,splits", [(128, 128, 2), (384, 256, 4), (384, 256, 6), (640, 384, 3), (896, 128, 7),
+                                               (3584, 1536, 3), (128, 20480, 2)])
+def test_cuts_inside_a_step_of_the_fused_product(gpu, n_in, n_out, splits):
+    """65 to 128 tokens take 128-column steps, yet their K-splits are cut between 64 columns: cuts inside a step, splits of
+    half a step, as many splits as slices, more items than SMs. Every partial sum has the bits of the same tokens in a batch
+    of 144, which takes 64-column steps, and none is empty."""
+    w, *_ = make_linear(gpu, n_in, n_out, 40 + splits)
+    x = torch.randn(144, n_in, generator=torch.Generator(device="cuda").manual_seed(n_in), device="cuda").to(torch.bfloat16)
+    full = torch.full((splits, 144, n_out), float("nan"), device="cuda")
+    gpu.linear.qtip_multiply_tc(w, x, full, n_out, splits, 144)
+    assert bool(full.any(-1).all())
+    for tokens in (65, 96, 128):
+        z = torch.full((splits, tokens, n_out), float("nan"), device="cuda")
+        gpu.linear.qtip_multiply_tc(w, x[:tokens], z, n_out, splits, tokens)
+        assert torch.equal(z, full[:, :tokens])
+    gpu.linear.kernel_status()
