@@ -247,7 +247,8 @@ typedef struct qtip_matrix {
   const uint16_t* trellis; /* _d kernel-layout words, (out/16)(in/16)*32 */
   const float* su;         /* _d [in]  +-1 */
   const float* sv;         /* _d [out] sign * Wscale */
-  const uint32_t* lut;     /* _d [1024] bf16x2 (qtip_runtime_lut) */
+  const uint32_t* lut;     /* _d [1024] bf16x2 (qtip_runtime_lut); the products read it ahead of the kernel before them
+                              in the stream, so a table that a KERNEL writes needs a synchronisation before its first use */
   int in, out;
 } qtip_matrix; /* field for field runtime/cuda/kernels.hpp:5-10 (QtipMatrix) */
 
