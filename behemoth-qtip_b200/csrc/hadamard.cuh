@@ -524,13 +524,16 @@ __global__ __cluster_dims__(kHadCluster, 1, 1) __launch_bounds__(kClusterThreads
   extern __shared__ float row_s[];
   const int q = blockIdx.x;
   const long row = blockIdx.y;
-  had_cluster_arrive();  // every CTA of the cluster runs before one stores into another
+  // The first cluster barrier: every CTA of the cluster runs before one stores into another. With a norm it also stands
+  // between the reads of the whole row for the norm and the first store of xn, which may be the row itself.
+  if constexpr (M != Mode::PrepareNorm) had_cluster_arrive();
   chain_release();
   chain_wait();
   if constexpr (M == Mode::PrepareNorm) {
     __shared__ float slots[1024];
     a.write_xn = true;  // a column is mixed by one CTA only
     if (a.norm) a.factor = row_norm_factor<M>(a, row, slots);
+    had_cluster_arrive();
   }
   had_cluster_wait();
   cluster_transform<K, T, M>(a, row, row_s, q);

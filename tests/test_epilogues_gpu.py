@@ -234,3 +234,18 @@ def test_rows_of_order_28_match_single_rows(gpu, n, rows):
         return h
     if 2 * n <= 57344 or rows < 32:
         assert torch.equal(gateup(z2), one(lambda r: gateup(z2[:, r:r + 1])))
+
+
+@pytest.mark.parametrize("n,rows", [(3584, 16), (3584, 127), (7168, 33), (28672, 40), (28672, 64)])
+def test_rows_of_order_28_normalised_in_place(gpu, n, rows):
+    """xn may be the row that it is made from: every CTA of a row's cluster has read the whole row for the norm before one
+    of them stores. Again and again on fresh rows, against a buffer of its own."""
+    lin, gen = gpu.linear, torch.Generator(device="cuda").manual_seed(n + rows)
+    norm = (1 + 0.1 * torch.randn(n, generator=gen, device="cuda")).to(torch.bfloat16)
+    su = torch.randint(0, 2, (n,), generator=gen, device="cuda").float() * 2 - 1
+    for _ in range(8):
+        x = torch.randn(rows, n, generator=gen, device="cuda").to(torch.bfloat16)
+        u, xn, u2 = (torch.empty_like(x) for _ in range(3))
+        lin.input_transform(x, norm, 1e-5, su, n, rows, u, xn)
+        lin.input_transform(x, norm, 1e-5, su, n, rows, u2, x)
+        assert torch.equal(x, xn) and torch.equal(u, u2)
