@@ -481,8 +481,16 @@ __global__ __launch_bounds__(1024, 1) void had_chunk_gateup_kernel(HadArgs a, co
 // own: the chunk kernel reads a row 28 times, the whole-row kernel leaves most SMs idle (figures at had_path).
 constexpr int kHadCluster = 4, kClusterThreads = 256;
 
-__device__ __forceinline__ void had_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void had_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// The aligned forms want all lanes of a warp at the same instruction, and the lanes of a warp may come out of a loop over fewer
+// than 32 columns one after another.
+__device__ __forceinline__ void had_cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void had_cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void had_cluster_sync() {
   had_cluster_arrive();
   had_cluster_wait();

@@ -183,7 +183,8 @@ def test_large_batch_row_kernels_match_the_chunk_kernels(gpu, n):
         assert torch.equal(y_big[r].view(torch.int16), y_one[0].view(torch.int16)), "bf16 output transform, row %d" % r
 
 
-@pytest.mark.parametrize("n,rows", [(448, 16), (896, 127), (3584, 33), (28672, 31), (28672, 64), (57344, 17)])
+@pytest.mark.parametrize("n,rows", [(448, 16), (448, 64), (896, 127), (1792, 33), (1792, 64), (3584, 33), (28672, 31),
+                                    (28672, 64), (57344, 17)])
 def test_rows_of_order_28_match_single_rows(gpu, n, rows):
     """16 to 127 rows of order 28 run on a cluster per row: every stage gives the bits of the same rows taken one at a time
     (chunk kernel), K-splits, gathered sources and the normalised copy included."""
