@@ -573,16 +573,32 @@ __global__ __cluster_dims__(kHadCluster, 1, 1) __launch_bounds__(kClusterThreads
 constexpr int kMaxRowFloats = 57344;  // 224 KiB of the 227 KiB a CTA may hold
 constexpr int kChunkRowsBelow = 32;  // fewer rows than this: K CTAs per row
 // Kernel of a transform by its row count and shape; `room`: longest row of the whole-row kernel. A cluster per row from 16 to
-// 127 rows of order 28, measured on 28,672-wide rows in four splits (chunk or whole-row kernel against cluster, us): output
-// transform 28.9 / 13.7 at 31 rows, 21.0 / 14.6 at 64; gate/up epilogue 63.4 / 29.5 and 45.0 / 31.0; input transform
-// 20.9 / 10.6 at 31. At 13 rows in two splits they are level (25.1 / 24.1) and the chunk kernel is the better link of a
-// chain of launches; at 200 the whole-row kernel has a row for every SM (53.5 / 52.8, and 112 / 137 at 512). Order 12 has
-// less to gain from reading a row once (gate/up at 64 rows 27.1 / 21.8, at 200 47.9 / 64.7) and keeps the two kernels.
+// 64 rows of order 28. Below 16 rows the chunk kernel is the better link of a chain of launches (13 rows of 28,672 in two
+// splits: gate/up 25.1 us against 24.1, the MLP around it 265 against 299). From 72 rows the clusters, two CTAs an SM, no
+// longer run all at once. Chunk or whole-row kernel against cluster, us, 28,672 columns in four splits (one for the norm):
+//   rows              16            31            64            72            96
+//   output          18.9 / 13.4   28.8 / 14.1   20.6 / 15.0   20.6 / 25.1   21.0 / 27.5
+//   gate/up         41.1 / 28.3   63.7 / 29.9   45.5 / 33.0   47.4 / 59.1   61.9 / 71.8
+//   input + norm    31.4 / 15.7   46.2 / 17.0   22.7 / 17.4   22.7 / 29.7   22.7 / 32.1
+// The same lines hold at 3,584, 7,168 and 14,336 columns. Order 12 has less to gain from reading a row once (gate/up at 64
+// rows 27.1 / 21.8, at 200 47.9 / 64.7) and keeps the two kernels.
 enum class Path { Chunk, Cluster, Row };
 template <int K>
 constexpr bool kHasCluster = K == 28;
-static Path had_path(int K, int n, int P, long rows, int room) {
-  if (K == 28 && rows >= 16 && rows < 128 && P % (4 * kHadCluster) == 0 && n <= room) return Path::Cluster;
+// Few splits are little to read 28 times, and the residual's read and write of the state is the cluster kernel's to wait for:
+// where the chunk kernel transforms in registers (P of 1,024 and 2,048) it stays faster for the residual (16 rows of 28,672 in
+// one split 11.2 / 15.2, two splits 14.0 / 16.0, three 16.7 / 16.8; of 57,344 in one split 23.3 / 26.4, in two 33.2 / 28.0), and
+// at P = 256, where up to 21 rows of its CTAs run at once, for residual and gate/up of one split (20 rows of 7,168: 7.6 / 7.9,
+// 10.8 / 11.6). The whole-row kernel has caught up in one split from 48 rows of 28,672 (50 rows: 16.7 / 17.2).
+static bool cluster_is_slower(Mode m, int P, int splits, long rows) {
+  if (m == Mode::FinishResidual && P == 1024 && splits == 1) return rows <= 28 || rows >= 48;
+  if (m == Mode::FinishResidual && P == 1024) return splits == 2 && rows <= 21;
+  if (m == Mode::FinishResidual && P == 2048) return splits == 1 && rows <= 21;
+  return (m == Mode::FinishResidual || m == Mode::FinishGateUp) && P == 256 && splits == 1 && rows <= 21;
+}
+static Path had_path(Mode m, int K, int n, int P, int splits, long rows, int room) {
+  if (K == 28 && rows >= 16 && rows <= 64 && P % (4 * kHadCluster) == 0 && n <= room && !cluster_is_slower(m, P, splits, rows))
+    return Path::Cluster;
   return K > 1 && rows < kChunkRowsBelow && P <= 8192 ? Path::Chunk : Path::Row;
 }
 // The kernels of a cluster are a link of the decode step's chain like the chunk kernels.
@@ -604,7 +620,7 @@ template <int K, bool T, Mode M>
 static int launch(const HadArgs& a, long rows, bool force_row, cudaStream_t s) {
   const int threads = a.P >= 1024 ? 1024 : (a.P < 64 ? 64 : a.P);
   constexpr int kRoom = M == Mode::PrepareNorm ? kMaxRowFloats - 1024 : kMaxRowFloats;  // 4 KiB of static slots
-  const Path path = force_row ? Path::Row : had_path(K, a.n, a.P, rows, kRoom);
+  const Path path = force_row ? Path::Row : had_path(M, K, a.n, a.P, a.splits, rows, kRoom);
   if constexpr (kHasCluster<K> && M != Mode::F32Inplace)
     if (path == Path::Cluster) {
       QB_CUDA(launch_cluster(had_cluster_kernel<K, T, M>, rows, size_t(a.n), s, a));

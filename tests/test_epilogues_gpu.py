@@ -184,9 +184,9 @@ def test_large_batch_row_kernels_match_the_chunk_kernels(gpu, n):
 
 
 @pytest.mark.parametrize("n,rows", [(448, 16), (448, 64), (896, 127), (1792, 33), (1792, 64), (3584, 33), (28672, 31),
-                                    (28672, 64), (57344, 17)])
+                                    (28672, 64), (57344, 17), (3584, 65), (7168, 20), (7168, 22), (28672, 21), (57344, 22)])
 def test_rows_of_order_28_match_single_rows(gpu, n, rows):
-    """16 to 127 rows of order 28 run on a cluster per row: every stage gives the bits of the same rows taken one at a time
+    """16 to 64 rows of order 28 run on a cluster per row, more on a CTA per row: every stage gives the bits of the same rows taken one at a time
     (chunk kernel), K-splits, gathered sources and the normalised copy included."""
     lin = gpu.linear
     gen = torch.Generator(device="cuda").manual_seed(n + rows)
