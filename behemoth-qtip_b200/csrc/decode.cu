@@ -368,12 +368,45 @@ __global__ void tp_wait_kernel(unsigned* ctl_words, int slot, int ranks) {
   tp_wait_warp(reinterpret_cast<TpControl*>(ctl_words), slot, ranks);
 }
 
-// Dense decode to bf16, row-major [out][in]. One persistent CTA per SM holds the 32-copy table (a single copy costs three to
+// Dense decode to bf16, row-major [out][in], of a few strips: a CTA decodes one 32-row x 256-column strip through shared
+// memory so that global stores are 16-byte and coalesced. A single copy of the table: 4 KiB to fill instead of 128, for
+// look-ups that cost three to four passes of the shared-memory pipe each.
+constexpr int kDecCols = 256, kDecLd = kDecCols / 2 + 4;  // bf16 pairs; + 4 words of padding per row
+__global__ __launch_bounds__(256) void decode_strip_kernel(qtip_matrix w, uint16_t* __restrict__ out) {
+  __shared__ uint32_t lut_s[1024];
+  __shared__ __align__(16) uint32_t tile[32 * kDecLd];
+  for (int i = threadIdx.x; i < 1024; i += 256) lut_s[i] = w.lut[i];
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, A = lane >> 2, B = lane & 3;
+  const int br = blockIdx.y, n2 = w.in / 32, blk0 = blockIdx.x * (kDecCols / 32), blk = blk0 + warp;
+  if (blk < n2) {
+    const uint2* codes = reinterpret_cast<const uint2*>(w.trellis) + (size_t(br) * n2 + blk) * 32;
+    const uint2 own = codes[lane], peer = codes[(lane + 1) & 31];
+#pragma unroll
+    for (int j1 = 0; j1 < 2; ++j1)
+#pragma unroll
+      for (int i1 = 0; i1 < 2; ++i1) {
+        const uint32_t u = __byte_perm(j1 ? own.y : own.x, j1 ? peer.y : peer.x, i1 ? 0x3276 : 0x1054);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          tile[(i1 * 16 + (k & 1) * 8 + A) * kDecLd + warp * 16 + j1 * 8 + (k >> 1) * 4 + B] = lut_s[lut_entry(u >> (16 - 4 * k))];
+      }
+  }
+  __syncthreads();
+  const int cols8 = min(kDecCols, w.in - blk0 * 32) / 8;  // w.in is a multiple of 32
+  for (int i = threadIdx.x; i < 32 * cols8; i += 256) {
+    const int r = i / cols8, c8 = i % cols8;
+    *reinterpret_cast<uint4*>(out + (size_t(br) * 32 + r) * w.in + blk0 * 32 + c8 * 8) =
+        *reinterpret_cast<const uint4*>(tile + r * kDecLd + c8 * 4);
+  }
+}
+
+// The same for many strips. One persistent CTA per SM holds the 32-copy table (a single copy costs three to
 // four passes of the shared-memory pipe per look-up); its four groups of eight warps walk the 32-row x 256-column strips, a
 // 32 x 32 block per warp, through a tile in shared memory so that global stores are 16-byte and coalesced. The groups are
 // out of phase, so one decodes while another stores. Bound by the 2 bytes written per weight: 57344 x 12288 and 12288 x 28672
 // together 566 -> 434 us (one copy of the table and a strip per CTA before), 2.37 GB: 5.5 TB/s.
-constexpr int kDecCols = 256, kDecGroups = 4, kDecLd = kDecCols / 2 + 4;  // bf16 pairs; + 4 words of padding per row
+constexpr int kDecGroups = 4;
 constexpr size_t kDecSmem = kLutBytes + size_t(kDecGroups) * 32 * kDecLd * 4;
 __global__ __launch_bounds__(kDecGroups * 256, 1) void decode_matrix_kernel(qtip_matrix w, uint16_t* __restrict__ out) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -597,12 +630,21 @@ extern "C" int qtip_decode_matrix(qtip_matrix w, uint16_t* out_d, void* stream) 
   int rc = check_matrix(w, "qtip_decode_matrix");
   if (rc) return rc;
   QB_REQUIRE(out_d, QTIP_E_ARG, "qtip_decode_matrix: null output");
-  QB_REQUIRE(w.out / 32 <= 65535, QTIP_E_GEOMETRY, "qtip_decode_matrix: out = %d too large", w.out);
+  QB_REQUIRE(w.out / 32 <= 65535, QTIP_E_GEOMETRY, "qtip_decode_matrix: out = %d too large", w.out);  // grid.y of the strips
   const DeviceInfo* info = device_info();
   if (!info) return QTIP_E_DEVICE;
   const long strips = long(w.out / 32) * blocks_for(w.in, kDecCols);
-  const int grid = int(min(long(info->sm_count), (strips + kDecGroups - 1) / kDecGroups));
-  decode_matrix_kernel<<<grid, kDecGroups * 256, kDecSmem, as_stream(stream)>>>(w, out_d);
+  // Which of the two, by strips per SM (strip kernel against persistent, us): up to three the table costs more than it saves
+  // (24 strips 3.0 / 4.2, 128 3.1 / 4.6, 288 3.8 / 4.7, 384 4.3 / 4.7); with four every group of a CTA has its strip (448 4.7 /
+  // 4.3, 560 4.9 / 4.9); five to seven are a second round for some (640 5.3 / 6.2, 896 6.1 / 6.3); above that the persistent
+  // kernel gains (1,120 6.8 / 6.4; 86,016 of 57344 x 12288 371 / 298).
+  const long per_sm = (strips + info->sm_count - 1) / info->sm_count;
+  if (per_sm <= 7 && per_sm != 4) {
+    decode_strip_kernel<<<dim3(blocks_for(w.in, kDecCols), w.out / 32), 256, 0, as_stream(stream)>>>(w, out_d);
+  } else {
+    const int grid = int(min(long(info->sm_count), (strips + kDecGroups - 1) / kDecGroups));
+    decode_matrix_kernel<<<grid, kDecGroups * 256, kDecSmem, as_stream(stream)>>>(w, out_d);
+  }
   QB_LAUNCHED();
   return QTIP_OK;
 }

@@ -318,10 +318,11 @@ def test_fused_decode_tile_edges(gpu, oracle, n_in, n_out, tokens, splits):
     assert rel_l2(z.sum(0).cpu().numpy(), ref) < 5e-6
 
 
-@pytest.mark.parametrize("n_in,n_out", [(32, 32), (288, 64), (480, 160), (224, 32 * 601), (8224, 96)])
+@pytest.mark.parametrize("n_in,n_out", [(32, 32), (288, 64), (480, 160), (224, 32 * 601), (8224, 96), (256, 32 * 444),
+                                        (256, 32 * 445), (224, 32 * 592), (32, 32 * 593), (288, 32 * 518), (480, 32 * 519)])
 def test_decode_matrix_strip_edges(gpu, oracle, n_in, n_out):
-    """Strips of 256 columns: rows that end inside a strip, fewer strips than the groups of one CTA, and more than one round
-    of strips over all SMs (601 block-rows)."""
+    """Strips of 256 columns: rows that end inside a strip, a handful of strips, more than one round of strips over all SMs
+    (601 block-rows), and both sides of the lines between the two kernels (three, four and seven strips an SM)."""
     w, tr, su, sv, tl = make_linear(gpu, n_in, n_out, 300 + n_in)
     out = torch.full((n_out, n_in), float("nan"), dtype=torch.bfloat16, device="cuda")
     gpu.linear.qtip_decode_matrix(w, out)
