@@ -510,7 +510,6 @@ static int gemm_attrs() {
   return gemm_attr<2, false, PUSH, 4>(gemm_smem(2, false, 0));
 }
 int decode_device_setup(DeviceInfo*) {
-  QB_CUDA(cudaFuncSetAttribute(decode_matrix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kDecSmem)));
   int rc = gemm_attrs<false>();
   return rc ? rc : gemm_attrs<true>();
 }
@@ -631,18 +630,21 @@ extern "C" int qtip_decode_matrix(qtip_matrix w, uint16_t* out_d, void* stream) 
   if (rc) return rc;
   QB_REQUIRE(out_d, QTIP_E_ARG, "qtip_decode_matrix: null output");
   QB_REQUIRE(w.out / 32 <= 65535, QTIP_E_GEOMETRY, "qtip_decode_matrix: out = %d too large", w.out);  // grid.y of the strips
-  const DeviceInfo* info = device_info();
-  if (!info) return QTIP_E_DEVICE;
+  // Needs no qtip_init: the persistent kernel is given its shared memory at each call (3.7 us of host time with and without).
+  int dev = 0, sms = 0;
+  QB_CUDA(cudaGetDevice(&dev));
+  QB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const long strips = long(w.out / 32) * blocks_for(w.in, kDecCols);
   // Which of the two, by strips per SM (strip kernel against persistent, us): up to three the table costs more than it saves
   // (24 strips 3.0 / 4.2, 128 3.1 / 4.6, 288 3.8 / 4.7, 384 4.3 / 4.7); with four every group of a CTA has its strip (448 4.7 /
   // 4.3, 560 4.9 / 4.9); five to seven are a second round for some (640 5.3 / 6.2, 896 6.1 / 6.3); above that the persistent
   // kernel gains (1,120 6.8 / 6.4; 86,016 of 57344 x 12288 371 / 298).
-  const long per_sm = (strips + info->sm_count - 1) / info->sm_count;
+  const long per_sm = (strips + sms - 1) / sms;
   if (per_sm <= 7 && per_sm != 4) {
     decode_strip_kernel<<<dim3(blocks_for(w.in, kDecCols), w.out / 32), 256, 0, as_stream(stream)>>>(w, out_d);
   } else {
-    const int grid = int(min(long(info->sm_count), (strips + kDecGroups - 1) / kDecGroups));
+    const int grid = int(min(long(sms), (strips + kDecGroups - 1) / kDecGroups));
+    QB_CUDA(cudaFuncSetAttribute(decode_matrix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kDecSmem)));
     decode_matrix_kernel<<<grid, kDecGroups * 256, kDecSmem, as_stream(stream)>>>(w, out_d);
   }
   QB_LAUNCHED();
