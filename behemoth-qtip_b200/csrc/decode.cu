@@ -326,10 +326,13 @@ __global__ __launch_bounds__(kGemmThreads, 1) void trellis_gemm_kernel(qtip_matr
   // A last round that has work for at most half of the CTAs goes out in half block-rows, one per CTA: they read all of the
   // code bytes for half of the decode work, so the round costs well under a unit (57344 x 12288, 12 units and 16 items: 94.7
   // -> 90.8 us). More than one round of them is no gain (12288 x 28672 in two splits, 352 halves for 176 items: 55.8 -> 56.9).
+  // Nor are they where a warp has no more than a block of the item to decode, unless they are few: with 48 items left, 12
+  // blocks an item 5.28 -> 5.63 us (20480 x 384), 32 6.70 -> 6.86, 48 8.50 both, 112 14.2 -> 13.7; with 16 or 24 left from 8
+  // blocks on (2560 x 1024 in four splits 4.86 -> 4.72).
   if constexpr (XS) {
-    if (2 * rest <= grid) {
-      for (int u = blockIdx.x; u < 2 * rest; u += grid)  // at most one
-        run_item<NT, XS, PUSH, true>(c, push, n_grouped + (u >> 1), kGemmThreads / 32, warp, 0, red, u & 1);
+    if (2 * rest <= grid && (2 * c.n2 >= 3 * splits * (kGemmThreads / 32) || 6 * rest <= grid)) {
+      if (int(blockIdx.x) < 2 * rest)
+        run_item<NT, XS, PUSH, true>(c, push, n_grouped + (blockIdx.x >> 1), kGemmThreads / 32, warp, 0, red, blockIdx.x & 1);
       n_items = n_grouped;
     }
   }

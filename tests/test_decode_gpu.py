@@ -329,11 +329,14 @@ def test_decode_matrix_strip_edges(gpu, oracle, n_in, n_out):
     assert np.array_equal(out.float().cpu().numpy(), oracle.decode_rows(tr, n_in, n_out, tl, 0, n_out, True))
 
 
-@pytest.mark.parametrize("n_in,n_out,splits", [(384, 32 * 608, 1), (96, 32 * 306, 1), (1152, 32 * 153, 2), (384, 32 * 666, 1)])
+@pytest.mark.parametrize("n_in,n_out,splits", [(384, 32 * 608, 1), (96, 32 * 306, 1), (1152, 32 * 153, 2), (384, 32 * 666, 1),
+                                             (1504, 32 * 666, 1), (1536, 32 * 666, 1), (384, 32 * 616, 1),
+                                             (384, 32 * 617, 1)])
 def test_one_token_short_last_round(gpu, oracle, n_in, n_out, splits):
-    """One token where the work items leave a last round for at most half of the SMs (16 of 608 items beyond a full round of
-    592, 10 of 306 beyond 296, the same in K-splits, 74 beyond 592): that round runs in half block-rows. Every row against
-    float64 on the decoded weights (1e-5, at most 1,152 fp32 terms in two orders), and the same bits when run again."""
+    """One token where the work items leave a last round for at most half of the SMs: 16 of 608 items beyond a full round of
+    592, 10 of 306 beyond 296, the same in K-splits, 74 beyond 592 of 12, 47 and 48 blocks, 24 and 25 beyond 592. That round
+    runs in half block-rows where they pay. Every row against float64 on the decoded weights (1e-5, at most 1,536 fp32 terms
+    in two orders), and the same bits when run again."""
     w, tr, su, sv, tl = make_linear(gpu, n_in, n_out, 500 + n_out % 97)
     xb = gpu.synth.f32_to_bf16_bits(np.random.default_rng(n_out).standard_normal((1, n_in)).astype(np.float32))
     z = torch.full((splits, n_out), float("nan"), dtype=torch.float32, device="cuda")
