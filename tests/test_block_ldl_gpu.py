@@ -93,3 +93,40 @@ def test_block_ldl_panel_edges(gpu, oracle, n):
         bad[at, at] = -1.0
         with pytest.raises(gpu.QtipError, match="positive definite"):
             gpu.codec.block_ldl(dev(bad))
+
+
+def block_ldl_80(H32):
+    """The factor in 80-bit arithmetic on the CPU: Cholesky column by column, then C[:, b] inv(C[b, b]) by back substitution."""
+    C = H32.astype(np.longdouble)
+    n = C.shape[0]
+    C = (C + C.T) / 2
+    for j in range(n):
+        C[j, j] = np.sqrt(C[j, j])
+        C[j + 1:, j] /= C[j, j]
+        C[j + 1:, j + 1:] -= np.outer(C[j + 1:, j], C[j + 1:, j])
+    L = np.zeros_like(C)
+    for b in range(0, n, 16):
+        D, X = C[b:b + 16, b:b + 16], L[b + 16:, b:b + 16]
+        for j in range(15, -1, -1):
+            X[:, j] = (C[b + 16:, b + j] - X[:, j + 1:] @ D[j + 1:, j]) / D[j, j]
+    return L
+
+
+@pytest.mark.parametrize("n,damping,scale", [(272, 1e-6, 1.0), (272, 1e-6, 1e-2), (400, 1e-5, 1e-3)])
+def test_block_ldl_of_an_ill_conditioned_hessian(gpu, n, damping, scale):
+    """Half as many activations as columns, a small damping, columns scaled over up to three decades (condition 1e6 to 1e11):
+    the panel solve multiplies by inverses of diagonal blocks, and its factor stays as close to the 80-bit one as fp64
+    substitution does (LAPACK's on the CPU; twice its distance is allowed, two orders of summation)."""
+    assert np.finfo(np.longdouble).nmant >= 63
+    rng = np.random.default_rng(n)
+    X = rng.standard_normal((n // 2, n))
+    d = np.geomspace(1.0, scale, n)[rng.permutation(n)]
+    H = X.T @ X / n
+    H = (H + damping * H.diagonal().mean() * np.eye(n)) * d * d[:, None]
+    H32 = H.astype(np.float32)
+    H32 = np.tril(H32) + np.tril(H32, -1).T
+    ref = block_ldl_80(H32)
+    dist = lambda L: float(np.linalg.norm((L - ref).astype(np.float64)) / np.linalg.norm(ref.astype(np.float64)))  # noqa: E731
+    _, L64 = gpu.codec.block_ldl(dev(H32), want_f64=True)
+    substituted = block_ldl_f64(torch.from_numpy(H32.astype(np.float64)))
+    assert dist(L64.cpu().numpy()) < 2 * dist(substituted.numpy())

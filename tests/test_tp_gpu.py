@@ -109,3 +109,39 @@ def test_two_processes_over_peer_memory():
     out = subprocess.run(cmd, env=env, capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stdout[-2000:] + out.stderr[-2000:]
     assert out.stdout.count("tp worker ok") == 2
+
+
+class DeviceArray:
+    """A device address as something torch can look at."""
+
+    def __init__(self, address, shape):
+        self.__cuda_array_interface__ = {"data": (address, False), "shape": shape, "typestr": "<f4", "version": 3}
+
+
+@pytest.mark.parametrize("rows,splits", [(32 * 153, 2), (32 * 306, 1), (32 * 608, 1)])
+def test_push_with_a_short_last_round(gpu, rows, splits):
+    """One token, two ranks whose shards leave a last round for a few CTAs (10 or 16 work items beyond the full rounds of 148
+    SMs), which goes out in half block-rows: every product arrives in both ranks' buffers. Against float64 on the decoded
+    weights (1e-5, at most 768 fp32 terms in two orders); the slot holds NaN before."""
+    n_in, n_out = 768, 2 * rows
+    w, *_ = make_linear(gpu, n_in, n_out, 23 + splits)
+    x = torch.randn(1, n_in, generator=torch.Generator(device="cuda").manual_seed(rows), device="cuda").to(torch.bfloat16)
+    dense = torch.empty(n_out, n_in, dtype=torch.bfloat16, device="cuda")
+    gpu.linear.qtip_decode_matrix(w, dense)
+    ref = (x.double() @ dense.double().T)[0]
+    group = gpu.tp.Exchange.local_group(2, n_out, max_splits=splits)
+    try:
+        z = [torch.as_tensor(DeviceArray(ex.gathered(0), (splits, n_out)), device="cuda") for ex in group]
+        for t in z:
+            t.fill_(float("nan"))
+        for r in range(2):
+            group[r].multiply_push(w.rows(r * rows, rows), x, 0, n_out, r * rows, splits)
+        for r in range(2):
+            assert group[r].gather_wait(0) == group[r].gathered(0)
+            group[r].check()
+            assert float((z[r].double().sum(0) - ref).norm() / ref.norm()) < 1e-5
+            assert float((z[r].double().sum(0) - ref).abs().max()) < 1e-4 * float(ref.square().mean().sqrt())
+    finally:
+        torch.cuda.synchronize()
+        for ex in group:
+            ex.close(free_local=True)
