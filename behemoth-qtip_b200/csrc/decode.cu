@@ -2,7 +2,7 @@
 // 2-bit trellis codes (kernel layout: one 32x32 block = 128 uint16 = 256 contiguous bytes; word c of the four 16x16 tiles
 // of a block sits at uint16 index 4c + 2 j1 + i1).
 //
-// trellis_gemm_kernel (1..8 tokens per pass): a warp streams 32x32 blocks of one 32-row block-row. Lane l loads the 8
+// trellis_gemm_kernel (up to 16 tokens per pass): a warp streams 32x32 blocks of one 32-row block-row. Lane l loads the 8
 // bytes holding word l of the four tiles (one fully coalesced 256-byte request per warp), gets word l+1 from its
 // neighbour by shuffle, cuts the four 16-bit states of each window and looks their bf16x2 pairs up in shared memory.
 // Those four words are exactly the lane's A fragment of an m16n8k16 bf16 MMA for that tile, so the dot products run on
@@ -81,25 +81,6 @@ __device__ __forceinline__ void item_run(const ItemCtx& c, int item, int nw, int
   const int span = k_hi - k_lo;
   b_lo = k_lo + int(long(span) * wi / nw), b_hi = k_lo + int(long(span) * (wi + 1) / nw);
 }
-// Optional (off): asks the memory system to bring a warp's run of code blocks (256 bytes each, contiguous) into the L2
-// ahead of the loads that will read it: one bulk prefetch issued by one lane, no destination, no completion to wait
-// for. Measured on 57344 x 12288: same duration with and without, but 30 % more DRAM reads with it (229.8 MB against
-// the 176.4 MB of codes: a whole round of next items is 58 MB, part of it is evicted before its turn), so it stays off.
-#ifndef QB_GEMV_PREFETCH
-#define QB_GEMV_PREFETCH 0
-#endif
-__device__ __forceinline__ void prefetch_run(const ItemCtx& c, int item, int n_items, int nw, int wi) {
-#if QB_GEMV_PREFETCH
-  if (item >= n_items || (threadIdx.x & 31) != 0) return;
-  int br, sp, b_lo, b_hi;
-  item_run(c, item, nw, wi, br, sp, b_lo, b_hi);
-  if (b_hi <= b_lo) return;
-  const uint2* at = c.codes + (size_t(br) * size_t(c.n2) + size_t(b_lo)) * 32u;
-  const uint32_t bytes = uint32_t(b_hi - b_lo) * 256u;
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(at), "r"(bytes) : "memory");
-#endif
-}
-
 // One work item = one 32-row block-row x one K-split, shared by `nw` warps (this is warp `wi` of them): each warp takes
 // a contiguous run of 32x32 blocks, then the partial sums are added in warp order through `red` and written to z.
 // HALF (one token): only the 16 rows `half` of the block-row, at half the decode work for all of its code bytes.
@@ -315,12 +296,8 @@ __global__ __launch_bounds__(kGemmThreads, 1) void trellis_gemm_kernel(qtip_matr
   const int slots = gridDim.x * ipc;
   const int n_grouped = n_items / slots * slots;
   const int grp = warp / wpi, wi = warp % wpi;
-  prefetch_run(c, blockIdx.x * ipc + grp, n_grouped, wpi, wi);  // the first item's codes
-  for (int item = blockIdx.x * ipc + grp; item < n_grouped; item += slots) {
-    prefetch_run(c, item + slots, n_grouped, wpi, wi);  // the next item's codes travel while this one is decoded
+  for (int item = blockIdx.x * ipc + grp; item < n_grouped; item += slots)
     run_item<NT, XS, PUSH>(c, push, item, wpi, wi, grp + 1, red + size_t(grp) * wpi * RT * 32);
-  }
-  prefetch_run(c, n_grouped + blockIdx.x, n_items, kGemmThreads / 32, warp);
   __syncthreads();
   const int rest = n_items - n_grouped, grid = gridDim.x;
   // A last round that has work for at most half of the CTAs goes out in half block-rows, one per CTA: they read all of the
@@ -392,7 +369,8 @@ __global__ __launch_bounds__(256) void decode_strip_kernel(qtip_matrix w, uint16
         const uint32_t u = __byte_perm(j1 ? own.y : own.x, j1 ? peer.y : peer.x, i1 ? 0x3276 : 0x1054);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          tile[(i1 * 16 + (k & 1) * 8 + A) * kDecLd + warp * 16 + j1 * 8 + (k >> 1) * 4 + B] = lut_s[lut_entry(u >> (16 - 4 * k))];
+          tile[(i1 * 16 + (k & 1) * 8 + A) * kDecLd + warp * 16 + j1 * 8 + (k >> 1) * 4 + B] =
+              lut_s[lut_entry(u >> (16 - 4 * k))];
       }
   }
   __syncthreads();

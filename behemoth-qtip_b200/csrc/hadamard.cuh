@@ -585,6 +585,8 @@ constexpr int kChunkRowsBelow = 32;  // fewer rows than this: K CTAs per row
 enum class Path { Chunk, Cluster, Row };
 template <int K>
 constexpr bool kHasCluster = K == 28;
+template <int K, bool T, Mode M>  // the input side transforms by the transposed factor, the output side by the factor
+constexpr bool kHasClusterMode = kHasCluster<K> && M != Mode::F32Inplace && T == kIsPrepare<M>;
 // Few splits are little to read 28 times, and the residual's read and write of the state is the cluster kernel's to wait for:
 // where the chunk kernel transforms in registers (P of 1,024 and 2,048) it stays faster for the residual (16 rows of 28,672 in
 // one split 11.2 / 15.2, two splits 14.0 / 16.0, three 16.7 / 16.8; of 57,344 in one split 23.3 / 26.4, in two 33.2 / 28.0), and
@@ -612,7 +614,7 @@ static int configure() {
   QB_CUDA(cudaFuncSetAttribute(had_row_kernel<K, T, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (M == Mode::PrepareNorm ? kMaxRowFloats - 1024 : kMaxRowFloats) * 4));
   QB_CUDA(cudaFuncSetAttribute(had_chunk_kernel<K, T, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * 4));
-  if constexpr (kHasCluster<K> && M != Mode::F32Inplace)
+  if constexpr (kHasClusterMode<K, T, M>)
     QB_CUDA(cudaFuncSetAttribute(had_cluster_kernel<K, T, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxRowFloats));
   return QTIP_OK;
 }
@@ -621,7 +623,7 @@ static int launch(const HadArgs& a, long rows, bool force_row, cudaStream_t s) {
   const int threads = a.P >= 1024 ? 1024 : (a.P < 64 ? 64 : a.P);
   constexpr int kRoom = M == Mode::PrepareNorm ? kMaxRowFloats - 1024 : kMaxRowFloats;  // 4 KiB of static slots
   const Path path = force_row ? Path::Row : had_path(M, K, a.n, a.P, a.splits, rows, kRoom);
-  if constexpr (kHasCluster<K> && M != Mode::F32Inplace)
+  if constexpr (kHasClusterMode<K, T, M>)
     if (path == Path::Cluster) {
       QB_CUDA(launch_cluster(had_cluster_kernel<K, T, M>, rows, size_t(a.n), s, a));
       return QTIP_OK;

@@ -18,31 +18,15 @@ extern __shared__ __align__(16) uint32_t gemm_smem_words[];
 // state of the low tile is `o` itself), doubled, hashed with one multiply-add (2 v (v + 1), entry in bits 7..16) and
 // turned into the byte address of the lane's own copy (entry e, copy l at byte 128 e + 4 l) with one three-input logic
 // operation: shift, add, multiply-add, and-or, load per state.
-#ifndef QB_GEMV_DECODE
-#define QB_GEMV_DECODE 1
-#endif
 __device__ __forceinline__ uint32_t lut_word(uint32_t v, uint32_t lane4) {
-#if QB_GEMV_DECODE == 1
   const uint32_t v2 = v + v;
   uint32_t y2;
   asm("mad.lo.u32 %0, %1, %2, %2;" : "=r"(y2) : "r"(v), "r"(v2));
   const uint32_t at = (y2 & 0x1ff80u) | lane4;
-#elif QB_GEMV_DECODE == 2
-  const uint32_t y = v * v + v;
-  const uint32_t at = ((y << 1) & 0x1ff80u) | lane4;
-#else
-  const uint32_t y = v * v + v;
-  const uint32_t at = (((y >> 6) & 1023u) << 7) + lane4;
-#endif
   return *reinterpret_cast<const uint32_t*>(reinterpret_cast<const unsigned char*>(gemm_smem_words) + at);
 }
 __device__ __forceinline__ void decode_pair(uint32_t o, uint32_t p, uint32_t lane4, uint32_t (&lo)[4],
                                             uint32_t (&hi)[4]) {
-#if QB_GEMV_DECODE == 0
-  const uint32_t u0 = __byte_perm(o, p, 0x1054), u1 = __byte_perm(o, p, 0x3276);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) lo[k] = lut_word(u0 >> (16 - 4 * k), lane4), hi[k] = lut_word(u1 >> (16 - 4 * k), lane4);
-#else
   const uint32_t pl = p << 16, oh = o >> 16;
   lo[0] = lut_word(o, lane4);
   hi[0] = lut_word(oh, lane4);
@@ -51,7 +35,6 @@ __device__ __forceinline__ void decode_pair(uint32_t o, uint32_t p, uint32_t lan
     lo[k] = lut_word(__funnelshift_l(pl, o, 4 * k), lane4);
     hi[k] = lut_word(__funnelshift_l(p, oh, 4 * k), lane4);
   }
-#endif
 }
 // One of the two windows only: `upper` (the same for the whole warp) takes the tile i1 = 1.
 __device__ __forceinline__ void decode_half(uint32_t o, uint32_t p, bool upper, uint32_t lane4, uint32_t (&v)[4]) {

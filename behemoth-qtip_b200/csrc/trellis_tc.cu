@@ -46,8 +46,8 @@ struct FtSmem {
 // Where the K-splits are cut is part of the result: it decides which sums are chains of their own. Up to 64 tokens the cuts
 // lie between 128 columns (where those divide the row), above between 64. With 128-column steps a cut may then fall into a
 // step (`halves`): both splits run it, and the MMA thread leaves out the half that is not theirs. A kernel of its own, because
-// the test in the MMA thread costs every other shape 4 %; 12288 x 28672 in three splits at 65 / 128 tokens: 65 / 80 us, 91 / 96 with
-// 64-column steps.
+// the test in the MMA thread costs every other shape 4 %; 12288 x 28672 in three splits at 65 / 128 tokens: 65 / 80 us, 91 / 96
+// with 64-column steps.
 struct FtConfig {
   int ksub;     // 64-column slices per K step
   bool halves;  // some cut is in the middle of a step

@@ -271,7 +271,9 @@ int qtip_finish_b16(qtip_matrix w, const uint16_t* z_d, uint16_t* y_d, float* sc
 int qtip_forward(qtip_matrix w, const uint16_t* x_d, uint16_t* y_d, float* scratch_d, uint16_t* rotated_d,
                  float* z_d, int round_z, void* stream, int splits);
 /* Token-major activations, split-major fp32 products. runtime/cuda/batch_kernels.cu:701-736 (qtip_multiply_batch).
- * `implementation` is accepted for signature compatibility and ignored (one code path per batch regime). */
+ * `implementation`: 0 = the MMA-fragment kernel, 16 tokens a pass; 2 = the fused tensor-core product (qtip_multiply_tc); any
+ * other value = by batch size and shape: the fused product above 16 tokens, and from 9 tokens for up to 16,384 rows, where
+ * in % 64 == 0, out % 128 == 0 and x_d is 16-byte aligned, else the MMA-fragment kernel. */
 int qtip_multiply_batch(qtip_matrix w, const uint16_t* x_d, float* z_d, int stride, int splits, int tokens,
                         void* stream, int implementation);
 /* Dense bf16 decode of the whole matrix, row-major [out][in]. runtime/cuda/batch_kernels.cu:23-46,737-740. */
