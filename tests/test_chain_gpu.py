@@ -49,6 +49,27 @@ def test_chained_launches_give_the_bits_of_plain_ones(gpu, tmp_path):
             assert torch.equal(decode_steps(gpu, tokens).cpu(), plain[tokens]), tokens
 
 
+@pytest.mark.parametrize("tokens", [9, 96, 144])
+def test_surplus_splits_under_capture(gpu, tokens):
+    """More K-splits than cuts: the zero fill of the surplus slices and the chained product behind it, recorded and replayed."""
+    lin, gen = gpu.linear, torch.Generator(device="cuda").manual_seed(tokens)
+    n_in, n_out, splits = 128, 256, 4
+    trellis = torch.randint(-32768, 32768, (n_in * n_out // 256 * 32,), generator=gen, device="cuda", dtype=torch.int16)
+    one = torch.ones(n_out, device="cuda")
+    w = lin.Matrix(trellis, one[:n_in], one, lin.runtime_lut(gpu.synth.seeded_tlut(1)), n_in, n_out)
+    x = torch.randn(tokens, n_in, generator=gen, device="cuda").to(torch.bfloat16)
+    want, z = torch.empty(splits, tokens, n_out, device="cuda"), torch.empty(splits, tokens, n_out, device="cuda")
+    lin.qtip_multiply_tc(w, x, want, n_out, splits, tokens)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        lin.qtip_multiply_tc(w, x, z, n_out, splits, tokens)
+        lin.qtip_multiply_tc(w, x, z, n_out, splits, tokens)
+    for _ in range(3):
+        z.fill_(float("nan"))
+        graph.replay()
+        assert torch.equal(z, want) and not bool(want[2:].any())
+
+
 if __name__ == "__main__":
     sys.path.insert(0, ROOT)
     import __graft_entry__
