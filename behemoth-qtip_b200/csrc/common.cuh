@@ -31,7 +31,8 @@ inline cudaStream_t as_stream(void* s) { return static_cast<cudaStream_t>(s); }
 struct DeviceInfo {
   bool ready = false;
   int sm_count = 0;
-  int max_clusters = 0;  // co-resident 8-CTA clusters of the Viterbi kernel
+  int max_clusters = 0;  // co-resident 8-CTA clusters of the Viterbi kernel with back-pointers
+  int max_clusters4 = 0, max_clusters8 = 0;  // of the 4- and 8-CTA kernels of the fused path
 };
 DeviceInfo* device_info();  // for the current device; nullptr + error set if qtip_init() has not run there
 int viterbi_device_setup(DeviceInfo* info);  // viterbi.cu

@@ -12,40 +12,12 @@
 //    exchanged between the 8 SMs through distributed shared memory (each minimum is pushed with st.async to the one CTA
 //    that reads it next step and counted on that CTA's mbarrier); the two 4-sequence halves of a batch alternate so that one half computes while
 //    the other half's minima are in flight. Back-pointers go to global memory as one 32-bit word per (8 steps, group).
-#include <cooperative_groups.h>
-
+#include <algorithm>
 #include <mutex>
 
-#include "common.cuh"
-
-namespace cg = cooperative_groups;
+#include "viterbi.cuh"
 
 namespace qb {
-
-// ------------------------------------------------------------------------------------------------- shared device code
-
-__device__ __forceinline__ float state_cost(float l0, float l1, float nrm, float mp, float m0, float m1) {
-  return __fmaf_rn(l1, m1, __fmaf_rn(l0, m0, __fadd_rn(nrm, mp)));
-}
-__device__ __forceinline__ float min3(float a, float b, float c) {
-  float r;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-// (bits & mask) | d in one LOP3. With the mask as an immediate the compiler needs two instructions (an immediate AND and
-// an immediate OR) on the half-rate integer pipe, which is the busiest pipe of the inner loop; the kernels therefore
-// take the mask (0xfffffff0) as a run-time argument so that it lives in a register and only d is an immediate.
-__device__ __forceinline__ float tag_cost(float c, uint32_t mask, int d) {
-  uint32_t r;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(__float_as_uint(c)), "r"(mask), "r"(uint32_t(d)));
-  return __uint_as_float(r);
-}
-constexpr uint32_t kTagMask = 0xfffffff0u;
-
-// (cost, state) candidates of the last step order by cost, then by state.
-__device__ __forceinline__ void take_better(float& bv, uint32_t& bs, float ov, uint32_t os) {
-  if (ov < bv || (ov == bv && os < bs)) bv = ov, bs = os;
-}
 
 // ------------------------------------------------------------------------------------------------- backtraces
 
@@ -63,20 +35,6 @@ __global__ void vit_overlap_u16_kernel(const uint16_t* __restrict__ A, const uin
   uint32_t s = final_state[b];
   for (int i = 126; i >= 64; --i) s = prev_state_u16(Ab, i, s);
   overlap[b] = int(s >> 4);
-}
-__device__ __forceinline__ void emit_state(int i, uint32_t s, uint16_t* q, float* hatWT, long m, long row0, int col0,
-                                           float* hat, const uint32_t* lut_h2) {
-  if (q) q[i] = uint16_t(s);
-  if (hatWT || hat) {
-    const uint32_t u = lut_h2[s];
-    const float v0 = half_lo(u), v1 = half_hi(u);
-    if (hat) hat[2 * i] = v0, hat[2 * i + 1] = v1;
-    if (hatWT) {
-      const int t0 = perm_fwd(2 * i), t1 = perm_fwd(2 * i + 1);
-      hatWT[long(col0 + (t0 & 15)) * m + row0 + (t0 >> 4)] = v0;
-      hatWT[long(col0 + (t1 & 15)) * m + row0 + (t1 >> 4)] = v1;
-    }
-  }
 }
 __global__ void vit_finish_u16_kernel(const uint16_t* __restrict__ A, const uint16_t* __restrict__ final_state, int B,
                                       int b0, uint16_t* __restrict__ Q, int nblk, int blk, float* __restrict__ hatWT,
@@ -110,7 +68,6 @@ constexpr int kTG = 4;          // sequences per half-batch (one float4 of minim
 constexpr int kNG = QB_VIT_GROUPS;  // groups of kTG sequences in flight: one computes while the others' minima travel
 constexpr int kTB = kTG * kNG;  // sequences per cluster batch
 constexpr int kBufs = 3;        // exchange buffers per half-batch (see the hazard note in the kernel)
-constexpr long long kWaitCycles = 2000000000LL;  // give up a hand-shake after about a second
 constexpr uint32_t kBufBytes = 16 * 32 * kTG * 4;  // one exchange buffer
 
 struct __align__(16) ClusterSmem {
@@ -127,65 +84,6 @@ struct __align__(16) ClusterSmem {
   int ov[kTB];
   int abort_flag;
 };
-
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
-  return r;
-}
-// 16-byte store into a peer CTA's shared memory that, on delivery, counts 16 bytes on that CTA's mbarrier: data and
-// signal travel together, no fence on the sending side.
-__device__ __forceinline__ void st_async_v4(uint32_t addr, float a, float b, float c, float d, uint32_t bar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
-               "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float a) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(a) : "memory");
-}
-__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t a) {
-  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(a) : "memory");
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-// Arms the next phase of a local mbarrier: one arrival (this one) plus `bytes` of incoming st.async traffic.
-__device__ __forceinline__ void mbar_arm(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// Waits for phase `parity` of a local mbarrier. Never spins forever: after kWaitCycles it raises the CTA's abort flag and
-// the launch's status word, after which every wait in the CTA falls through (results are then garbage and the host
-// reports QTIP_E_KERNEL).
-__device__ __forceinline__ void wait_full(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status) {
-  if (mbar_try_wait(bar, parity)) return;
-  const long long start = clock64();
-  for (;;) {
-#pragma unroll 1
-    for (int spin = 0; spin < 256; ++spin)
-      if (mbar_try_wait(bar, parity)) return;
-    if (*abort_flag) return;
-    if (clock64() - start > kWaitCycles) {
-      *abort_flag = 1;
-      atomicExch(status, 1);
-      return;
-    }
-  }
-}
 
 // Back-pointers of eight steps (one 32-bit word per thread, oldest step in the top nibble) written in the layout of the
 // reference's k_viterbi_fwd: A[step][j >> 2] uint16, nibble j & 3. The four lanes of a quad own j & 3 = 0..3; lane q
@@ -561,18 +459,22 @@ int viterbi_device_setup(DeviceInfo* info) {
   QB_CUDA(cudaOccupancyMaxActiveClusters(&n, vit_fwd_cluster_kernel<false>, &cfg));
   QB_REQUIRE(n > 0, QTIP_E_DEVICE, "the device cannot co-schedule an %d-CTA cluster of the Viterbi kernel", kCl);
   info->max_clusters = n;
-  return QTIP_OK;
+  return viterbi_minima_device_setup(info);
 }
 
-// Workspace of the fused path: [status (256 B)] [final_state u16 x cap] [overlap i32 x cap] [bp 256 KiB x cap].
+// Workspace of the fused path: [status (256 B)] [final_state u16 x cap] [overlap i32 x cap] [scratch 256 KiB x cap], the
+// scratch being back-pointer words (256 KiB a sequence) or stored minima (1,008 KiB).
 struct QuantWorkspace {
   int* status;
   uint16_t* fs;
   int* ov;
   uint32_t* bp;
-  int cap;
+  int cap;         // sequences whose back-pointers fit
+  int cap_minima;  // sequences whose minima fit
 };
 constexpr size_t kWsHeader = 256, kBpBytes = size_t(16) * 4096 * 4;
+// Capacity beyond which more minima gain nothing: two lanes of four full rounds of 33 clusters (2.2 GB).
+constexpr size_t kMinimaCap = 2 * 4 * 33 * kTB;
 static size_t ws_bytes_for(size_t cap) {
   size_t o = kWsHeader + ((cap * 2 + 255) / 256) * 256 + ((cap * 4 + 255) / 256) * 256;
   return o + cap * kBpBytes;
@@ -593,6 +495,7 @@ static bool carve_workspace(void* ws, size_t bytes, QuantWorkspace* out) {
   p += ((cap * 4 + 255) / 256) * 256;
   out->bp = reinterpret_cast<uint32_t*>(p);
   out->cap = int(cap);
+  out->cap_minima = int(cap * kBpBytes / kMinSeqBytes / kTB * kTB);
   return true;
 }
 
@@ -644,7 +547,14 @@ int quantize_tiles_impl(const float* X, int B, int b0, const uint32_t* lut, uint
   QB_REQUIRE(carve_workspace(ws, ws_bytes, &w), QTIP_E_WORKSPACE,
              "workspace of %zu bytes is too small (need at least %zu)", ws_bytes, ws_bytes_for(kTB));
   if (reset_status) QB_CUDA(cudaMemsetAsync(w.status, 0, kWsHeader, s));
-  const int half = w.cap / 2 / kTB * kTB;
+  // The passes that store minima are the faster ones (1.43 x) where the workspace holds the call's sequences or a round of
+  // clusters of them; a smaller workspace (the built-in one, or one sized for another version) takes the back-pointers'
+  // four times as many sequences per launch instead.
+  const int round = info->max_clusters4 * kTB;
+  const bool minima = w.cap_minima >= std::min((B + kTB - 1) / kTB * kTB, round) && reinterpret_cast<uintptr_t>(ws) % 16 == 0;
+  const int ws_cap = minima ? w.cap_minima : w.cap;
+  int half = ws_cap / 2 / kTB * kTB;
+  if (minima && half > round) half = half / round * round;  // whole rounds
   two_lanes = two_lanes && half >= 16 * kTB && B > half;  // worth it only with several chunks of a useful size
   LaneStreams* ls = nullptr;
   if (two_lanes) {
@@ -653,7 +563,7 @@ int quantize_tiles_impl(const float* X, int B, int b0, const uint32_t* lut, uint
     QB_CUDA(cudaEventRecord(ls->fork, s));
     QB_CUDA(cudaStreamWaitEvent(ls->side, ls->fork, 0));
   }
-  const int cap = two_lanes ? half : w.cap;
+  const int cap = two_lanes ? half : ws_cap;
   // The chunk loop as a function, so that every way out of it passes the join below: a failed launch must not leave the
   // side stream un-joined (it may still be writing the outputs, and an open fork would invalidate a stream capture).
   auto chunks = [&]() -> int {
@@ -663,6 +573,13 @@ int quantize_tiles_impl(const float* X, int B, int b0, const uint32_t* lut, uint
       const float* xc = X + size_t(c0) * 256;
       const int o = (two_lanes && lane) ? half : 0;  // this lane's part of the scratch arrays
       cudaStream_t st = (two_lanes && lane) ? ls->side : s;
+      float* hc = hat ? hat + size_t(c0) * 256 : nullptr;
+      if (minima) {
+        const int rc = viterbi_minima_chunk(info, xc, nb, lut, reinterpret_cast<float*>(w.bp) + size_t(o) * (kMinSeqBytes / 4),
+                                            w.fs + o, w.ov + o, w.status, b0 + c0, Q, nblk, blk, hc, hatWT, m, col0, st);
+        if (rc) return rc;
+        continue;
+      }
       uint32_t* bp = w.bp + size_t(o) * (kBpBytes / 4);
       int rc = launch_cluster_fwd(info, xc, nullptr, 1, nb, bp, 8, w.fs + o, lut, w.status, st);
       if (rc) return rc;
@@ -674,7 +591,6 @@ int quantize_tiles_impl(const float* X, int B, int b0, const uint32_t* lut, uint
       QB_LAUNCHED();
       rc = launch_cluster_fwd(info, xc, w.ov + o, 0, nb, bp, 0, w.fs + o, lut, w.status, st);
       if (rc) return rc;
-      float* hc = hat ? hat + size_t(c0) * 256 : nullptr;
       if (nb <= kBtMaxBatch)
         vit_backtrace_staged_kernel<true><<<nb, kBtThreads, kBtSmem, st>>>(bp, w.fs + o, nullptr, b0 + c0, Q, nblk, blk, hc,
                                                                           hatWT, m, col0, lut);
@@ -770,7 +686,9 @@ extern "C" int qtip_k_viterbi_finish_words(const uint32_t* bp_d, const uint16_t*
 
 extern "C" size_t qtip_quantize_workspace_bytes(int max_tiles) {
   size_t cap = max_tiles < kTB ? size_t(kTB) : size_t((max_tiles + kTB - 1) / kTB * kTB);
-  return ws_bytes_for(cap);
+  const size_t minima = cap < kMinimaCap ? cap : kMinimaCap;
+  const size_t words = (minima * kMinSeqBytes + kBpBytes - 1) / kBpBytes;  // the same scratch in back-pointer units
+  return ws_bytes_for(std::max(cap, (words + kTB - 1) / kTB * kTB));
 }
 extern "C" int qtip_quantize_tiles(const float* X_d, int B, const uint32_t* lut_h2_d, uint16_t* states_d, float* hat_d,
                                    void* workspace_d, size_t workspace_bytes, void* stream) {

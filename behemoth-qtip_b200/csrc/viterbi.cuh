@@ -1,0 +1,117 @@
+// What the Viterbi kernels share: the cost of a state, tags, the exchange between the CTAs of a cluster, the output of a
+// path. Included by viterbi.cu (back-pointer kernels, entry points) and viterbi_minima.cu (the fused path's kernels).
+#pragma once
+#include <cooperative_groups.h>
+
+#include "common.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace qb {
+
+__device__ __forceinline__ float state_cost(float l0, float l1, float nrm, float mp, float m0, float m1) {
+  return __fmaf_rn(l1, m1, __fmaf_rn(l0, m0, __fadd_rn(nrm, mp)));
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+// (bits & mask) | d in one LOP3. With the mask as an immediate the compiler needs two instructions (an immediate AND and
+// an immediate OR) on the half-rate integer pipe, which is the busiest pipe of the inner loop; the kernels therefore
+// take the mask (0xfffffff0) as a run-time argument so that it lives in a register and only d is an immediate.
+__device__ __forceinline__ float tag_cost(float c, uint32_t mask, int d) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(__float_as_uint(c)), "r"(mask), "r"(uint32_t(d)));
+  return __uint_as_float(r);
+}
+constexpr uint32_t kTagMask = 0xfffffff0u;
+
+// (cost, state) candidates of the last step order by cost, then by state.
+__device__ __forceinline__ void take_better(float& bv, uint32_t& bs, float ov, uint32_t os) {
+  if (ov < bv || (ov == bv && os < bs)) bv = ov, bs = os;
+}
+
+__device__ __forceinline__ void emit_state(int i, uint32_t s, uint16_t* q, float* hatWT, long m, long row0, int col0,
+                                           float* hat, const uint32_t* lut_h2) {
+  if (q) q[i] = uint16_t(s);
+  if (hatWT || hat) {
+    const uint32_t u = lut_h2[s];
+    const float v0 = half_lo(u), v1 = half_hi(u);
+    if (hat) hat[2 * i] = v0, hat[2 * i + 1] = v1;
+    if (hatWT) {
+      const int t0 = perm_fwd(2 * i), t1 = perm_fwd(2 * i + 1);
+      hatWT[long(col0 + (t0 & 15)) * m + row0 + (t0 >> 4)] = v0;
+      hatWT[long(col0 + (t1 & 15)) * m + row0 + (t1 >> 4)] = v1;
+    }
+  }
+}
+
+constexpr long long kWaitCycles = 2000000000LL;  // give up a hand-shake after about a second
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
+  return r;
+}
+// 16-byte store into a peer CTA's shared memory that, on delivery, counts 16 bytes on that CTA's mbarrier: data and
+// signal travel together, no fence on the sending side.
+__device__ __forceinline__ void st_async_v4(uint32_t addr, float a, float b, float c, float d, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
+               "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float a) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(a) : "memory");
+}
+__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t a) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(a) : "memory");
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+// Arms the next phase of a local mbarrier: one arrival (this one) plus `bytes` of incoming st.async traffic.
+__device__ __forceinline__ void mbar_arm(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Waits for phase `parity` of a local mbarrier. Never spins forever: after kWaitCycles it raises the CTA's abort flag and
+// the launch's status word, after which every wait in the CTA falls through (results are then garbage and the host
+// reports QTIP_E_KERNEL).
+__device__ __forceinline__ void wait_full(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  if (mbar_try_wait(bar, parity)) return;
+  const long long start = clock64();
+  for (;;) {
+#pragma unroll 1
+    for (int spin = 0; spin < 256; ++spin)
+      if (mbar_try_wait(bar, parity)) return;
+    if (*abort_flag) return;
+    if (clock64() - start > kWaitCycles) {
+      *abort_flag = 1;
+      atomicExch(status, 1);
+      return;
+    }
+  }
+}
+
+// viterbi_minima.cu: the fused path's passes over B sequences with minima in place of back-pointers
+constexpr size_t kMinSeqBytes = size_t(63) * 4096 * 4;  // of the minima buffer per sequence, whole batches of eight
+int viterbi_minima_device_setup(DeviceInfo* info);
+int viterbi_minima_chunk(const DeviceInfo* info, const float* X, int B, const uint32_t* lut, float* mins, uint16_t* fs,
+                         int* ov, int* status, int b0, uint16_t* Q, int nblk, int blk, float* hat, float* hatWT, long m,
+                         int col0, cudaStream_t s);
+
+}  // namespace qb

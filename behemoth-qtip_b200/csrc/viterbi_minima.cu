@@ -1,0 +1,429 @@
+// The fused path's Viterbi: forward passes that keep group minima instead of back-pointers, and the backtraces that find
+// the few back-pointers of the chosen path from them. Same arithmetic contract as viterbi.cu, same states bit for bit.
+//
+// Why: the back-pointer of a group is the tag that rides in the low four bits of its sixteen costs, one logic operation a
+// state on the half-rate integer pipe and three more a group to take it off and collect it. A path needs 127 of the
+// 4,096 x 127 back-pointers of a sequence. Truncation of the low four bits is monotone, so the truncated minimum of the
+// costs is the minimum of the truncated costs, and the forward pass can leave the tags out: add, fma, fma, half a 3-input
+// minimum. Every second step its 4,096 minima go to memory (16 KiB); the backtrace recomputes, for the state it stands
+// at, the sixteen costs of that step with their tags and the 256 of the step before, which is what the tagged pass
+// compared.
+#include <type_traits>
+
+#include "viterbi.cuh"
+
+namespace qb {
+
+constexpr int kMinThreads = 256;
+constexpr int kMinTG = 4;               // sequences per group (one float4 of minima per predecessor)
+constexpr int kMinNG = 2;               // groups in flight: one computes while the other's minima travel
+constexpr int kMinTB = kMinTG * kMinNG; // sequences per cluster batch
+constexpr int kMinBufs = 3;             // exchange buffers per group (see the hazard note of vit_fwd_cluster_kernel)
+constexpr int kMinSlots = 63;           // the predecessor minima of steps 1, 3, .., 125 are stored
+static_assert(kMinSeqBytes == size_t(kMinSlots) * 4096 * 4, "the stored minima of a sequence");
+
+// kCl CTAs own the trellis, 4096 / kCl groups each, J adjacent groups a thread.
+template <int kCl>
+struct __align__(16) MinimaSmem {
+  static constexpr int kRows = 256 / kCl;  // distinct j >> 4 of a CTA
+  // M[g][buf][d][row][t]: minimum (+ next step's xx) of predecessor group (d << 8) | (kRows * rank + row)
+  float M[kMinNG][kMinBufs][16][kRows][kMinTG];
+  struct {
+    __half m[kMinNG][2][kMinTG];  // fp16(-2 x0), fp16(-2 x1)
+    float xx[kMinNG][kMinTG];     // x0^2 + x1^2
+  } in[128];                      // per step
+  unsigned long long full[kMinNG][kMinBufs];
+  float red_c[kMinThreads / 32][kMinTB];
+  uint32_t red_s[kMinThreads / 32][kMinTB];
+  float fin_c[kCl][kMinTB];  // used in CTA 0 only: one candidate per CTA
+  uint32_t fin_s[kCl][kMinTB];
+  int ov[kMinTB];
+  int abort_flag;
+};
+
+// a * b + c with fp16 a, b: their product is exact in fp32, so this is the fp32 fma of the converted values.
+__device__ __forceinline__ float fma_f16(uint16_t a, uint16_t b, float c) {
+  float r;
+  asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(r) : "h"(a), "h"(b), "f"(c));
+  return r;
+}
+// state_cost on the packed table entry (l0 | l1 << 16): the table stays in fp16, one register for what took two.
+__device__ __forceinline__ float state_cost_h(uint32_t l, float nrm, float mp, uint16_t m0, uint16_t m1) {
+  return fma_f16(uint16_t(l >> 16), m1, fma_f16(uint16_t(l), m0, __fadd_rn(nrm, mp)));
+}
+__device__ __forceinline__ void unpack_h4(uint2 v, uint16_t (&h)[4]) {
+  h[0] = uint16_t(v.x), h[1] = uint16_t(v.x >> 16), h[2] = uint16_t(v.y), h[3] = uint16_t(v.y >> 16);
+}
+
+// Copies a finished buffer of minima from shared to global memory behind the compute (one thread; 16-byte aligned).
+__device__ __forceinline__ void bulk_store(float* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("fence.proxy.async.shared::cta;\n\t"
+               "cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\t"
+               "cp.async.bulk.commit_group;" ::"l"(dst), "r"(src), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_store_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
+// X [B][256]; overlap [B] or null; final_state [B]. mins: per group of four sequences [63 slots][kCl][d 16][rows][t 4] floats,
+// slot (i - 1) / 2 holds the buffers that the CTAs read at odd step i; steps below first_step are not stored.
+//
+// What bounds it: issue, at about 70 % of the slots (operand-port conflicts and the hand-shake take the rest; no pipe above
+// 75 %). The adjacent groups of a thread share each 16-byte load of predecessor minima: with one group a thread the
+// shared-memory return path (128 bytes a clock) alone takes four cycles a state and scheduler. With the table in fp16 four
+// SMs hold the trellis (128 registers a thread), and 33 clusters of four are resident against 15 of eight: 132 SMs for 120.
+// Four groups a thread in 256 threads spread the step's fixed work over more states than two in 512: 365 and 383 us for
+// 400 and 405 (rolled and constrained pass of one batch, kCl = 4). Minima stored by the threads that compute them: 430 us
+// for the constrained pass, 380 with none stored at all; as bulk copies from the exchange buffers 405.
+template <int kCl>
+__global__ __launch_bounds__(kMinThreads, 1) void vit_fwd_minima_kernel(
+    const float* __restrict__ X, const int* __restrict__ overlap, int roll, int B, float* __restrict__ mins,
+    int first_step, uint16_t* __restrict__ final_state, const uint32_t* __restrict__ lut_h2, int* __restrict__ status,
+    uint32_t tag_mask) {
+  using Smem = MinimaSmem<kCl>;
+  constexpr int J = 4096 / (kCl * kMinThreads), kRows = Smem::kRows;
+  static_assert(J == 2 || J == 4, "two or four adjacent groups a thread share their predecessors");
+  constexpr uint32_t kBufBytes = 16 * kRows * kMinTG * 4, kGrpBytes = kMinBufs * kBufBytes;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = cg::this_cluster().block_rank();
+  const int cluster_id = blockIdx.x / kCl, n_clusters = gridDim.x / kCl;
+  const int j0 = (int(rank) * kMinThreads + tid) * J;  // this thread's groups: j0 .. j0 + J - 1
+  const int gl = tid * J >> 4;                         // local row of the predecessors they share
+
+  // The 16 states (d << 12) | j of each group: packed LUT pair and squared norm stay in registers for the whole launch.
+  uint32_t lut[J][16];
+  float nr[J][16];
+#pragma unroll
+  for (int q = 0; q < J; ++q)
+#pragma unroll
+    for (int d = 0; d < 16; ++d) {
+      const uint32_t u = lut_h2[(d << 12) | (j0 + q)];
+      const float l0 = half_lo(u), l1 = half_hi(u);
+      lut[q][d] = u;
+      nr[q][d] = __fadd_rn(__fmul_rn(l0, l0), __fmul_rn(l1, l1));
+    }
+
+  if (tid == 0) {
+    for (int g = 0; g < kMinNG; ++g)
+      for (int b = 0; b < kMinBufs; ++b) mbar_init(smem_u32(&sm.full[g][b]), 1);
+    sm.abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    // Every phase of every barrier receives one full buffer from the kCl CTAs.
+    for (int g = 0; g < kMinNG; ++g)
+      for (int b = 0; b < kMinBufs; ++b) mbar_arm(smem_u32(&sm.full[g][b]), kBufBytes);
+  }
+  cluster_sync_all();
+
+  // Minimum of group j is read next step as predecessor (d' << 8) | g' with d' = j >> 8, g' = j & 255, i.e. by CTA
+  // g' / kRows at row (d', g' % kRows). A half-warp covers kRows consecutive j and pushes to one CTA, and every CTA is fed
+  // by some warp of every other: the hazard note of vit_fwd_cluster_kernel holds here too.
+  const uint32_t dst = uint32_t(j0 & 255) / kRows;
+  const uint32_t push_base = map_to_cta(smem_u32(&sm.M[0][0][j0 >> 8][j0 % kRows][0]), dst);
+  const uint32_t bar_base = map_to_cta(smem_u32(&sm.full[0][0]), dst);
+  volatile int* abort_flag = &sm.abort_flag;
+  const uint32_t bar_own = smem_u32(&sm.full[0][0]);
+  uint32_t parities = 0;  // bit buf: parity of the next wait on full[.][buf], the same for every group
+
+  for (int batch = cluster_id; batch * kMinTB < B; batch += n_clusters) {
+    const int t_first = batch * kMinTB;
+    // Per-step input terms of the batch's sequences (sequences past B repeat the last one).
+    bool overflow = false;
+    for (int idx = tid; idx < 128 * kMinTB; idx += kMinThreads) {
+      const int tl = idx % kMinTB, step = idx / kMinTB;
+      const float* src = X + size_t(min(t_first + tl, B - 1)) * 256;
+      const int p0 = roll ? ((2 * step + 128) & 255) : 2 * step;
+      const float x0 = round_half(src[p0]), x1 = round_half(src[p0 + 1]);
+      const __half m0 = __float2half_rn(-2.f * x0), m1 = __float2half_rn(-2.f * x1);
+      sm.in[step].m[tl / kMinTG][0][tl % kMinTG] = m0;
+      sm.in[step].m[tl / kMinTG][1][tl % kMinTG] = m1;
+      sm.in[step].xx[tl / kMinTG][tl % kMinTG] = __fadd_rn(__fmul_rn(x0, x0), __fmul_rn(x1, x1));
+      overflow |= __hisinf(m0) || __hisinf(m1);
+    }
+    if (tid < kMinTB) sm.ov[tid] = overlap ? overlap[min(t_first + tid, B - 1)] : -1;
+    // A cost can only be -inf where fp16(-2 x) is infinite. The contract's tag turns -inf into a NaN, which loses every
+    // comparison, for all d but 0, so such batches (inputs beyond 32,752) are run with the tags; all CTAs see the same.
+    const bool tagged = __syncthreads_or(overflow);
+    for (int idx = tid; idx < 16 * kRows; idx += kMinThreads) {
+      // step-0 predecessors: 0 where the start constraint allows, 1e30 elsewhere, plus xx of step 0
+      const int d = idx / kRows, row = idx % kRows;
+      const int k = (d << 8) | (int(rank) * kRows + row);
+#pragma unroll
+      for (int g = 0; g < kMinNG; ++g)
+#pragma unroll
+        for (int t = 0; t < kMinTG; ++t) {
+          const int ov = sm.ov[g * kMinTG + t];
+          sm.M[g][0][d][row][t] = __fadd_rn((ov < 0 || k == ov) ? 0.f : 1e30f, sm.in[0].xx[g][t]);
+        }
+    }
+    __syncthreads();
+
+    // One step of one group. cur / nxt: byte offsets of the buffers read and written; parity: of the wait on the former.
+    float* store = mins + ((size_t(batch) * kMinNG * kMinSlots + (first_step >> 1)) * kCl + rank) * (kBufBytes / 4);
+    constexpr size_t kSlot = size_t(kCl) * kBufBytes / 4, kGroup = kMinSlots * kSlot;
+    auto stored = [&](int i) { return (i & 1) && i >= first_step; };
+    auto group_step = [&](int i, uint32_t cur, uint32_t nxt, uint32_t parity, int g, auto with_tags) {
+      const uint32_t full = bar_own + uint32_t(g * kMinBufs) * 8u;
+      if (i > 0) {
+        wait_full(full + cur / (kBufBytes / 8), parity, abort_flag, status);
+        if (tid == 0) {
+          mbar_arm(full + cur / (kBufBytes / 8), kBufBytes);  // for this buffer's next use
+          if (stored(i)) bulk_store(store + size_t(g) * kGroup, smem_u32(&sm.M[g][0][0][0][0]) + cur, kBufBytes);
+        }
+      }
+      uint16_t m0[4], m1[4];
+      unpack_h4(*reinterpret_cast<const uint2*>(&sm.in[i].m[g][0][0]), m0);
+      unpack_h4(*reinterpret_cast<const uint2*>(&sm.in[i].m[g][1][0]), m1);
+      float best[J][4];
+#pragma unroll
+      for (int q = 0; q < J; ++q)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) best[q][t] = 3e30f;
+      const float4* Mrow = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(&sm.M[g][0][0][gl][0]) + cur);
+#pragma unroll
+      for (int d = 0; d < 16; d += 2) {
+        const float4 pa = Mrow[d * kRows], pb = Mrow[(d + 1) * kRows];
+        const float paa[4] = {pa.x, pa.y, pa.z, pa.w}, pba[4] = {pb.x, pb.y, pb.z, pb.w};
+#pragma unroll
+        for (int q = 0; q < J; ++q)
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            float ca = state_cost_h(lut[q][d], nr[q][d], paa[t], m0[t], m1[t]);
+            float cb = state_cost_h(lut[q][d + 1], nr[q][d + 1], pba[t], m0[t], m1[t]);
+            if constexpr (decltype(with_tags)::value) ca = tag_cost(ca, tag_mask, d), cb = tag_cost(cb, tag_mask, d + 1);
+            best[q][t] = min3(best[q][t], ca, cb);
+          }
+      }
+      // The copy has read the buffer before this warp's push, hence (hazard note) before any CTA's push into it again.
+      if (tid == 0 && stored(i)) bulk_store_read();
+      const float4 xn = *reinterpret_cast<const float4*>(&sm.in[i + 1].xx[g][0]);
+      const float xna[4] = {xn.x, xn.y, xn.z, xn.w};
+#pragma unroll
+      for (int q = 0; q < J; ++q) {
+        float out[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) out[t] = __fadd_rn(__uint_as_float(__float_as_uint(best[q][t]) & ~15u), xna[t]);
+        st_async_v4(push_base + nxt + uint32_t(g) * kGrpBytes + q * 16, out[0], out[1], out[2], out[3],
+                    bar_base + uint32_t(g * kMinBufs) * 8u + nxt / (kBufBytes / 8));
+      }
+    };
+    auto advance = [&](int i, uint32_t& cur, uint32_t& nxt) {
+      if (i > 0) parities ^= 1u << (cur / kBufBytes);
+      if (stored(i)) store += kSlot;
+      cur = nxt;
+      nxt = nxt == (kMinBufs - 1) * kBufBytes ? 0 : nxt + kBufBytes;
+    };
+    uint32_t cur = 0, nxt = kBufBytes;
+    if (!tagged) {
+#pragma unroll 1
+      for (int i = 0; i < 127; ++i) {
+        const uint32_t parity = (parities >> (cur / kBufBytes)) & 1u;
+#pragma unroll
+        for (int g = 0; g < kMinNG; ++g) group_step(i, cur, nxt, parity, g, std::false_type{});
+        advance(i, cur, nxt);
+      }
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < 127; ++i) {
+        const uint32_t parity = (parities >> (cur / kBufBytes)) & 1u;
+#pragma unroll 1
+        for (int g = 0; g < kMinNG; ++g) group_step(i, cur, nxt, parity, g, std::true_type{});
+        advance(i, cur, nxt);
+      }
+    }
+
+    // Last step: untagged costs over the allowed states, lowest state on ties.
+#pragma unroll 1
+    for (int g = 0; g < kMinNG; ++g) {
+      const uint32_t full = bar_own + uint32_t(g * kMinBufs) * 8u + cur / (kBufBytes / 8);
+      wait_full(full, (parities >> (cur / kBufBytes)) & 1u, abort_flag, status);
+      if (tid == 0) mbar_arm(full, kBufBytes);
+      uint16_t m0[4], m1[4];
+      unpack_h4(*reinterpret_cast<const uint2*>(&sm.in[127].m[g][0][0]), m0);
+      unpack_h4(*reinterpret_cast<const uint2*>(&sm.in[127].m[g][1][0]), m1);
+      float bv[4] = {3e30f, 3e30f, 3e30f, 3e30f};
+      uint32_t bs[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+      const float4* Mrow = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(&sm.M[g][0][0][gl][0]) + cur);
+#pragma unroll
+      for (int d = 0; d < 16; ++d) {
+        const float4 pa = Mrow[d * kRows];
+        const float paa[4] = {pa.x, pa.y, pa.z, pa.w};
+#pragma unroll
+        for (int q = 0; q < J; ++q)
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const int ov = sm.ov[g * kMinTG + t];
+            const float c = state_cost_h(lut[q][d], nr[q][d], paa[t], m0[t], m1[t]);
+            // (d, q) ascending is the state order: the lowest state wins ties
+            if (c < bv[t] && (ov < 0 || j0 + q == ov)) bv[t] = c, bs[t] = (uint32_t(d) << 12) | uint32_t(j0 + q);
+          }
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+          take_better(bv[t], bs[t], __shfl_xor_sync(0xffffffffu, bv[t], off), __shfl_xor_sync(0xffffffffu, bs[t], off));
+        if (lane == 0) sm.red_c[warp][g * kMinTG + t] = bv[t], sm.red_s[warp][g * kMinTG + t] = bs[t];
+      }
+    }
+    parities ^= 1u << (cur / kBufBytes);
+    __syncthreads();
+    if (tid < kMinTB) {
+      float bv = sm.red_c[0][tid];
+      uint32_t bs = sm.red_s[0][tid];
+      for (int w = 1; w < kMinThreads / 32; ++w) take_better(bv, bs, sm.red_c[w][tid], sm.red_s[w][tid]);
+      st_cluster_f32(map_to_cta(smem_u32(&sm.fin_c[rank][tid]), 0), bv);
+      st_cluster_u32(map_to_cta(smem_u32(&sm.fin_s[rank][tid]), 0), bs);
+    }
+    cluster_sync_all();  // also keeps a fast CTA from pushing the next batch into buffers still being read
+    if (rank == 0 && tid < kMinTB && t_first + tid < B) {
+      float bv = sm.fin_c[0][tid];
+      uint32_t bs = sm.fin_s[0][tid];
+      for (int c = 1; c < kCl; ++c) take_better(bv, bs, sm.fin_c[c][tid], sm.fin_s[c][tid]);
+      final_state[t_first + tid] = uint16_t(bs);
+    }
+  }
+  cluster_sync_all();  // no CTA leaves while a peer may still write into its shared memory
+}
+
+// One CTA per sequence, two steps at a time: from the state of step i + 1 (group j) to those of steps i and i - 1.
+// Thread (e, d): predecessor d of j at step i is group k = (d << 8) | (j >> 4) of step i - 1, whose own predecessor e is the
+// stored minimum (e << 8) | (k >> 4); the sixteen minima over e, then their costs at step i, give both back-pointers.
+// What bounds it: the chain of 32 / 64 rounds, each one trip to memory for the minima and the table entries at once and
+// some 300 cycles behind it (a warp per sequence, eight entries a lane: 56 / 129 us; this way 25 / 50 us).
+// kFinish = false: overlap[b] = group of step 64 of the rolled pass. kFinish = true: the path of the constrained pass.
+template <bool kFinish>
+__global__ __launch_bounds__(256) void vit_backtrace_minima_kernel(
+    const float* __restrict__ X, int row_bits, const float* __restrict__ mins, const uint16_t* __restrict__ final_state,
+    int* __restrict__ overlap, int b0, uint16_t* __restrict__ Q, int nblk, int blk, float* __restrict__ hat,
+    float* __restrict__ hatWT, long m, int col0, const uint32_t* __restrict__ lut_h2) {
+  __shared__ float s_m0[128], s_m1[128], s_xx[128];
+  __shared__ float s_v[2][16][16];  // [round & 1][e][d]
+  __shared__ uint32_t s_state[128];
+  const int b = blockIdx.x, tid = threadIdx.x;
+  if (tid < 128) {
+    const int p0 = kFinish ? 2 * tid : (2 * tid + 128) & 255;
+    const float x0 = round_half(X[size_t(b) * 256 + p0]), x1 = round_half(X[size_t(b) * 256 + p0 + 1]);
+    s_m0[tid] = round_half(-2.f * x0), s_m1[tid] = round_half(-2.f * x1);
+    s_xx[tid] = __fadd_rn(__fmul_rn(x0, x0), __fmul_rn(x1, x1));
+  }
+  __syncthreads();
+  const int e = tid >> 4, d = tid & 15, half = (tid >> 4) & 1;
+  const float* const base = mins + size_t(b / kMinTG) * kMinSlots * 4096 * kMinTG + (b % kMinTG);
+  auto cost = [&](uint32_t u, float mp, int i) {
+    const float l0 = half_lo(u), l1 = half_hi(u);
+    return state_cost(l0, l1, __fadd_rn(__fmul_rn(l0, l0), __fmul_rn(l1, l1)), mp, s_m0[i], s_m1[i]);
+  };
+  auto best_tag = [&](float v) {  // tag of the minimum over the sixteen d (both halves of a warp hold the same values)
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, off));
+    return __float_as_uint(fminf(v, 3e30f)) & 15u;
+  };
+  uint32_t s = final_state[b];
+  if (kFinish && tid == 0) s_state[127] = s;
+#pragma unroll 1
+  for (int i = 126; i >= (kFinish ? 2 : 64); i -= 2) {
+    const uint32_t j = s >> 4, row = (uint32_t(d) << 4) | (j >> 8);
+    const uint32_t at = (((row >> row_bits) * 16 + e) << row_bits) | (row & ((1u << row_bits) - 1));
+    const float mp = base[(size_t(i / 2 - 1) * 4096 + at) * kMinTG];
+    const uint32_t u = lut_h2[(e << 12) | (d << 8) | (j >> 4)], u_own = lut_h2[(uint32_t(d) << 12) | j];
+    float(*sv)[16] = s_v[(i >> 1) & 1];
+    sv[e][d] = tag_cost(cost(u, mp, i - 1), kTagMask, e);
+    __syncthreads();  // two buffers: a warp writes one again only behind the next round's barrier
+    float v = 3e30f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) v = fminf(v, sv[half * 8 + r][d]);
+    v = fminf(v, __shfl_xor_sync(0xffffffffu, v, 16));
+    const float in = __fadd_rn(__uint_as_float(__float_as_uint(v) & ~15u), s_xx[i]);
+    const uint32_t dd = best_tag(tag_cost(cost(u_own, in, i), kTagMask, d));
+    s = (dd << 12) | j;
+    if (!kFinish && i == 64) break;
+    const uint32_t ee = __float_as_uint(__shfl_sync(0xffffffffu, v, int(dd))) & 15u;
+    const uint32_t s1 = (ee << 12) | (s >> 4);
+    if (kFinish && tid == 0) s_state[i] = s, s_state[i - 1] = s1;
+    s = s1;
+  }
+  if (!kFinish) {
+    if (tid == 0) overlap[b] = int(s >> 4);
+    return;
+  }
+  {  // step 0: the start constraint's minima
+    const uint32_t j = s >> 4;
+    const int ov = overlap[b], k = (d << 8) | int(j >> 4);
+    const float in = __fadd_rn((ov < 0 || k == ov) ? 0.f : 1e30f, s_xx[0]);
+    const uint32_t dd = best_tag(tag_cost(cost(lut_h2[(uint32_t(d) << 12) | j], in, 0), kTagMask, d));
+    if (tid == 0) s_state[0] = (dd << 12) | j;
+  }
+  __syncthreads();
+  if (tid < 128)
+    emit_state(tid, s_state[tid], Q ? Q + (size_t(b0 + b) * nblk + blk) * 128 : nullptr, hatWT, m, long(b0 + b) * 16, col0,
+               hat ? hat + size_t(b) * 256 : nullptr, lut_h2);
+}
+
+// ------------------------------------------------------------------------------------------------- host side
+
+template <int kCl>
+static void cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int clusters) {
+  cfg->gridDim = dim3(unsigned(clusters * kCl)), cfg->blockDim = dim3(kMinThreads);
+  cfg->dynamicSmemBytes = sizeof(MinimaSmem<kCl>);
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = kCl, attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  cfg->attrs = attr, cfg->numAttrs = 1;
+}
+template <int kCl>
+static int setup(int* resident) {
+  QB_CUDA(cudaFuncSetAttribute(vit_fwd_minima_kernel<kCl>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               int(sizeof(MinimaSmem<kCl>))));
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr{};
+  cluster_config<kCl>(&cfg, &attr, 64);
+  QB_CUDA(cudaOccupancyMaxActiveClusters(resident, vit_fwd_minima_kernel<kCl>, &cfg));
+  QB_REQUIRE(*resident > 0, QTIP_E_DEVICE, "the device cannot co-schedule a %d-CTA cluster of the Viterbi kernel", kCl);
+  return QTIP_OK;
+}
+int viterbi_minima_device_setup(DeviceInfo* info) {
+  int rc = setup<4>(&info->max_clusters4);
+  return rc ? rc : setup<8>(&info->max_clusters8);
+}
+
+template <int kCl>
+static int launch_fwd(int resident, const float* X, const int* overlap, int roll, int B, float* mins, int first_step,
+                      uint16_t* fs, const uint32_t* lut, int* status, cudaStream_t s) {
+  const int batches = (B + kMinTB - 1) / kMinTB;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr{};
+  cluster_config<kCl>(&cfg, &attr, batches < resident ? batches : resident);
+  cfg.stream = s;
+  QB_CUDA(cudaLaunchKernelEx(&cfg, vit_fwd_minima_kernel<kCl>, X, overlap, roll, B, mins,
+                             first_step, fs, lut, status, kTagMask));
+  return QTIP_OK;
+}
+// One pair of passes with their backtraces over up to the buffer's capacity of sequences (mins: kMinSeqBytes each, whole
+// batches of eight).
+int viterbi_minima_chunk(const DeviceInfo* info, const float* X, int B, const uint32_t* lut, float* mins, uint16_t* fs,
+                         int* ov, int* status, int b0, uint16_t* Q, int nblk, int blk, float* hat, float* hatWT, long m,
+                         int col0, cudaStream_t s) {
+  // A cluster of eight SMs takes a batch of eight sequences through a pass in 0.56 of the time that four SMs take (211 us
+  // for 375), with fewer than half as many clusters resident: it is the faster one for the few sequences of a short LDLQ column
+  // step.
+  const int batches = (B + kMinTB - 1) / kMinTB;
+  const int rounds4 = (batches + info->max_clusters4 - 1) / info->max_clusters4;
+  const int rounds8 = (batches + info->max_clusters8 - 1) / info->max_clusters8;
+  const bool wide = 0.56 * rounds8 < rounds4;
+  auto forward = [&](const int* overlap, int roll, int first_step) {
+    return wide ? launch_fwd<8>(info->max_clusters8, X, overlap, roll, B, mins, first_step, fs, lut, status, s)
+                : launch_fwd<4>(info->max_clusters4, X, overlap, roll, B, mins, first_step, fs, lut, status, s);
+  };
+  const int row_bits = wide ? 5 : 6;
+  // The rolled pass is traced back to step 64 only: from the minima that enter step 63 on.
+  int rc = forward(nullptr, 1, 63);
+  if (rc) return rc;
+  vit_backtrace_minima_kernel<false><<<B, 256, 0, s>>>(X, row_bits, mins, fs, ov, 0, nullptr, 0, 0, nullptr, nullptr, 0, 0, lut);
+  QB_LAUNCHED();
+  if ((rc = forward(ov, 0, 1))) return rc;
+  vit_backtrace_minima_kernel<true><<<B, 256, 0, s>>>(X, row_bits, mins, fs, ov, b0, Q, nblk, blk, hat, hatWT, m, col0, lut);
+  QB_LAUNCHED();
+  return QTIP_OK;
+}
+
+}  // namespace qb

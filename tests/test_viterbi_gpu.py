@@ -216,3 +216,31 @@ def test_two_chunks_in_flight_give_the_same_codes(gpu, hyb):
     big.check()
     small.check()
     assert torch.equal(s1, s2) and torch.equal(h1, h2)
+
+
+@pytest.mark.parametrize("kind", ["normal", "overflow", "tiny", "nonfinite"])
+@pytest.mark.parametrize("B", [1, 8, 61, 130, 265, 300])
+def test_stored_minima_give_the_back_pointers_path(gpu, B, kind):
+    """The passes that store minima (workspace of the advised size) against the passes with back-pointers (a workspace too
+    small for the minima): clusters of eight and of four, partly filled batches, a second round; costs of -inf, where the
+    tags decide, among finite ones, subnormal table entries and inputs, infinities and NaN."""
+    rng = np.random.default_rng(1000 + B)
+    tl = gpu.synth.seeded_tlut(1).copy()
+    X = (rng.standard_normal((B, 256)) * 1.2).astype(np.float32)
+    if kind == "overflow":
+        X[rng.random(X.shape) < 0.05] = 40000.0  # finite in fp16, -2 x is not
+        X[::3, 7] = -65000.0
+    elif kind == "tiny":
+        tl = (tl.astype(np.float32) * 2.0 ** -17).astype(np.float16)  # subnormal in fp16
+        X *= np.float32(2.0 ** -17)
+    elif kind == "nonfinite":
+        X[0, 3], X[B // 2, 100], X[-1, 255] = np.inf, np.nan, -np.inf
+    lut_d, _ = gpu_lut(gpu, tl)
+    c = gpu.codec
+    # 17 / 80 sequences' back-pointer words: minima of none / of sixteen
+    big, small = c.quantize_workspace(B), c.Workspace((17 if B <= 16 else 80) * 16 * 4096 * 4)
+    s1, h1 = c.quantize_tiles(dev(X), lut_d, workspace=big)
+    s2, h2 = c.quantize_tiles(dev(X), lut_d, workspace=small)
+    big.check()
+    small.check()
+    assert torch.equal(s1, s2) and np.array_equal(h1.cpu().numpy(), h2.cpu().numpy(), equal_nan=True)
