@@ -8,6 +8,7 @@
 //    every element is one thread's fp32 FMA chain over k ascending, which is deterministic and at least as accurate.
 //    128 x 128 output tile per CTA, 8 x 8 per thread, the 128-deep operand panels staged through shared memory.
 //  * qtip_ldlq: the schedule of ldlq_gpu (src/quantizer.cpp:30-89) on one stream, restricted to a slice of W rows.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
@@ -18,7 +19,7 @@ namespace qb {
 
 int quantize_tiles_impl(const float* X, int B, int b0, const uint32_t* lut, uint16_t* Q, int nblk, int blk, float* hat,
                         float* hatWT, long m, int col0, void* ws, size_t ws_bytes, bool reset_status, cudaStream_t s,
-                        bool two_lanes);  // viterbi.cu
+                        bool two_lanes, int in_flight);  // viterbi.cu
 
 // Rows j in [j0, j0 + mj) of W; X is indexed from the slice start: X[(j - j0) >> 4][256].
 // A CTA owns 32 rows of W and the block's 16 columns: the (up to 112) rows of L that reach into the block and the
@@ -147,7 +148,9 @@ static int ldlq_slices(long ntr) {
     const int v = std::atoi(e);
     if (v >= 1 && v <= kMaxSlices) return ntr >= v ? v : 1;
   }
-  return ntr >= 128 ? 2 : 1;  // measured: 192 sequences per step 2.13 s -> 1.64 s, 768: 7.0 -> 5.97 s, 96: no difference
+  // Measured, ms for 64 column steps in one / two / four slices: 1,792 sequences a step (16 steps) 94 / 86 / 85, 320: 94 / 71 /
+  // 66, 192: 58 / 49 / 50, 128: 56 / 42 / 38; 96: no difference.
+  return ntr >= 128 ? kMaxSlices : 1;
 }
 static size_t slice_ws_bytes(long ntr, int slices) {  // Viterbi scratch of all slices together
   size_t total = 0;
@@ -185,7 +188,9 @@ __global__ void merge_status_kernel(int* dst, const int* src) {
 extern "C" size_t qtip_ldlq_workspace_bytes(long n, long m) {
   if (n <= 0 || m <= 0) return 0;
   const long ntr = m / 16;
-  return slice_ws_bytes(ntr, kMaxSlices) + align256(size_t(n) * m * 4) + align256(size_t(ntr) * 256 * 4);
+  size_t scratch = 0;  // whichever number of slices the call will take
+  for (int slices = 1; slices <= kMaxSlices; ++slices) scratch = std::max(scratch, slice_ws_bytes(ntr, slices));
+  return scratch + align256(size_t(n) * m * 4) + align256(size_t(ntr) * 256 * 4);
 }
 
 extern "C" int qtip_ldlq(const float* WT_d, const float* L_d, long n, long m, long j0, long mj, float* hatWT_d,
@@ -254,7 +259,7 @@ extern "C" int qtip_ldlq(const float* WT_d, const float* L_d, long n, long m, lo
                                                                    bufend, a.X);
           QB_LAUNCHED();
           int rc = quantize_tiles_impl(a.X, a.ntr, int(a.j0 / 16), lut_h2_d, Q_d, nblk, col0 / 16, nullptr, hatWT_d, m,
-                                       col0, a.vws, a.vws_bytes, false, a.st, false);
+                                       col0, a.vws, a.vws_bytes, false, a.st, false, slices > 1 ? ntr : 0);
           if (rc) return rc;
         }
       }

@@ -537,10 +537,11 @@ static int lane_streams(LaneStreams** out) {
 // Shared body of the fused entry points. The sequences are processed in chunks that fit the workspace: forward (rolled),
 // overlap, forward (constrained), finish. two_lanes: the workspace is halved and consecutive chunks alternate between
 // the caller's stream and a side stream, so that one chunk's backtrace kernels (one thread per sequence) and the partly
-// filled last round of its forward launches run under the other chunk's forward pass.
+// filled last round of its forward launches run under the other chunk's forward pass. in_flight: sequences of this call and
+// of the ones that run beside it (0: it runs by itself).
 int quantize_tiles_impl(const float* X, int B, int b0, const uint32_t* lut, uint16_t* Q, int nblk, int blk, float* hat,
                         float* hatWT, long m, int col0, void* ws, size_t ws_bytes, bool reset_status, cudaStream_t s,
-                        bool two_lanes) {
+                        bool two_lanes, int in_flight) {
   const DeviceInfo* info = device_info();
   if (!info) return QTIP_E_DEVICE;
   QuantWorkspace w;
@@ -576,7 +577,7 @@ int quantize_tiles_impl(const float* X, int B, int b0, const uint32_t* lut, uint
       float* hc = hat ? hat + size_t(c0) * 256 : nullptr;
       if (minima) {
         const int rc = viterbi_minima_chunk(info, xc, nb, lut, reinterpret_cast<float*>(w.bp) + size_t(o) * (kMinSeqBytes / 4),
-                                            w.fs + o, w.ov + o, w.status, b0 + c0, Q, nblk, blk, hc, hatWT, m, col0, st);
+                                            w.fs + o, w.ov + o, w.status, b0 + c0, Q, nblk, blk, hc, hatWT, m, col0, in_flight, st);
         if (rc) return rc;
         continue;
       }
@@ -695,7 +696,7 @@ extern "C" int qtip_quantize_tiles(const float* X_d, int B, const uint32_t* lut_
   if (B == 0) return QTIP_OK;
   QB_REQUIRE(X_d && lut_h2_d && B > 0, QTIP_E_ARG, "qtip_quantize_tiles: bad argument");
   return quantize_tiles_impl(X_d, B, 0, lut_h2_d, states_d, 1, 0, hat_d, nullptr, 0, 0, workspace_d, workspace_bytes,
-                             true, as_stream(stream), true);
+                             true, as_stream(stream), true, 0);
 }
 extern "C" int qtip_quantize_tiles_scatter(const float* X_d, int B, int b0, const uint32_t* lut_h2_d, uint16_t* Q_d,
                                            int nblk, int blk, float* hatWT_d, long m, int col0, void* workspace_d,
@@ -706,7 +707,7 @@ extern "C" int qtip_quantize_tiles_scatter(const float* X_d, int B, int b0, cons
              "qtip_quantize_tiles_scatter: m = %ld does not cover %d row blocks", m, b0 + B);
   if (B == 0) return QTIP_OK;
   return quantize_tiles_impl(X_d, B, b0, lut_h2_d, Q_d, nblk, blk, nullptr, hatWT_d, m, col0, workspace_d,
-                             workspace_bytes, true, as_stream(stream), true);
+                             workspace_bytes, true, as_stream(stream), true, 0);
 }
 // ---- allocation-free variant of qtip_quantize_tiles
 // Some hosts of this library may not allocate device memory at all: a serving process whose memory pool is sized once at
@@ -743,7 +744,7 @@ extern "C" int qtip_quantize_tiles_noalloc(const float* X_d, int B, const uint32
   // status word is NOT cleared here, so that a time-out of any call since the last qtip_kernel_status (which reads and
   // clears it) is still reported.
   return quantize_tiles_impl(X_d, B, 0, lut_h2_d, states_d, 1, 0, hat_d, nullptr, 0, 0, scratch, kNoAllocBytes, false,
-                             as_stream(stream), false);  // one lane: this entry point creates no streams or events
+                             as_stream(stream), false, 0);  // one lane: this entry point creates no streams or events
 }
 
 extern "C" int qtip_workspace_status(const void* workspace_d, void* stream) {

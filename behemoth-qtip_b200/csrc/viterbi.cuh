@@ -112,6 +112,6 @@ constexpr size_t kMinSeqBytes = size_t(63) * 4096 * 4;  // of the minima buffer 
 int viterbi_minima_device_setup(DeviceInfo* info);
 int viterbi_minima_chunk(const DeviceInfo* info, const float* X, int B, const uint32_t* lut, float* mins, uint16_t* fs,
                          int* ov, int* status, int b0, uint16_t* Q, int nblk, int blk, float* hat, float* hatWT, long m,
-                         int col0, cudaStream_t s);
+                         int col0, int in_flight, cudaStream_t s);
 
 }  // namespace qb

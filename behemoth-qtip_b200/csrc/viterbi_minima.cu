@@ -8,6 +8,7 @@
 // minimum. Every second step its 4,096 minima go to memory (16 KiB); the backtrace recomputes, for the state it stands
 // at, the sixteen costs of that step with their tags and the 256 of the step before, which is what the tagged pass
 // compared.
+#include <algorithm>
 #include <type_traits>
 
 #include "viterbi.cuh"
@@ -402,17 +403,19 @@ static int launch_fwd(int resident, const float* X, const int* overlap, int roll
 // batches of eight).
 int viterbi_minima_chunk(const DeviceInfo* info, const float* X, int B, const uint32_t* lut, float* mins, uint16_t* fs,
                          int* ov, int* status, int b0, uint16_t* Q, int nblk, int blk, float* hat, float* hatWT, long m,
-                         int col0, cudaStream_t s) {
+                         int col0, int in_flight, cudaStream_t s) {
   // A cluster of eight SMs takes a batch of eight sequences through a pass in 0.56 of the time that four SMs take (211 us
-  // for 375), with fewer than half as many clusters resident: it is the faster one for the few sequences of a short LDLQ column
-  // step.
-  const int batches = (B + kMinTB - 1) / kMinTB;
-  const int rounds4 = (batches + info->max_clusters4 - 1) / info->max_clusters4;
-  const int rounds8 = (batches + info->max_clusters8 - 1) / info->max_clusters8;
-  const bool wide = 0.56 * rounds8 < rounds4;
+  // for 375), with fewer than half as many clusters resident: it is the faster one for the few sequences of a short LDLQ
+  // column step. A call by itself counts whole rounds of clusters; chains in flight beside each other (in_flight sequences
+  // in all) fill each other's rounds, so that rates count: 24 batches in four chains 0.78 ms a column step with eight SMs
+  // (0.90 with four), 40 batches 1.21 with eight and 1.03 with four.
+  const int batches = (B + kMinTB - 1) / kMinTB, all = (in_flight + kMinTB - 1) / kMinTB;
+  const int c4 = info->max_clusters4, c8 = info->max_clusters8;
+  const bool wide = in_flight > B ? 0.56 * all / c8 < std::max(1.0, double(all) / c4)
+                                  : 0.56 * ((batches + c8 - 1) / c8) < (batches + c4 - 1) / c4;
   auto forward = [&](const int* overlap, int roll, int first_step) {
-    return wide ? launch_fwd<8>(info->max_clusters8, X, overlap, roll, B, mins, first_step, fs, lut, status, s)
-                : launch_fwd<4>(info->max_clusters4, X, overlap, roll, B, mins, first_step, fs, lut, status, s);
+    return wide ? launch_fwd<8>(c8, X, overlap, roll, B, mins, first_step, fs, lut, status, s)
+                : launch_fwd<4>(c4, X, overlap, roll, B, mins, first_step, fs, lut, status, s);
   };
   const int row_bits = wide ? 5 : 6;
   // The rolled pass is traced back to step 64 only: from the minima that enter step 63 on.
