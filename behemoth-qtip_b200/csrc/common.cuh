@@ -1,5 +1,6 @@
 // Shared helpers of the qtip_b200 library: status/error plumbing, per-device state, small device functions.
 #pragma once
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -52,10 +53,7 @@ int had_order(long n);
 
 // ---- device helpers
 __device__ __forceinline__ float bf16_to_f32(uint16_t x) { return __uint_as_float(uint32_t(x) << 16); }
-__device__ __forceinline__ uint16_t f32_to_bf16(float x) {  // round to nearest even, finite inputs
-  uint32_t u = __float_as_uint(x);
-  return uint16_t((u + 0x7fffu + ((u >> 16) & 1u)) >> 16);
-}
+__device__ __forceinline__ uint16_t f32_to_bf16(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ float half_lo(uint32_t u) { return __half2float(__ushort_as_half(uint16_t(u))); }
 __device__ __forceinline__ float half_hi(uint32_t u) { return __half2float(__ushort_as_half(uint16_t(u >> 16))); }
 __device__ __forceinline__ float round_half(float x) { return __half2float(__float2half_rn(x)); }

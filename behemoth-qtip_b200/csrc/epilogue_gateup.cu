@@ -44,18 +44,19 @@ int hadamard_output_gateup(const float* z, int splits, long split_stride, int ro
              "gate/up rows of 2 x %d floats do not fit a CTA", F);
   QB_REQUIRE(rows <= 65535, QTIP_E_GEOMETRY, "too many rows");
   const int threads = a.P >= 1024 ? 1024 : (a.P < 64 ? 64 : a.P);
-  const size_t chunk_smem = (size_t(a.P > 1024 ? a.P : 1024) + a.P) * 4, row_smem = size_t(F) * 8;
+  const size_t chunk_smem = (size_t(a.P > 1024 ? a.P : 1024) + a.P) * 4, row_smem = size_t(had_room(K, a.P)) * 4;
+  const int row_threads = had_row_threads(rows, row_smem, false);
   // few rows: a link of a decode step's kernel chain (programmatic dependent launch, like the other chunk kernels)
 #define QB_GATEUP(K_)                                                                                                  \
   if (path == Path::Chunk)                                                                                             \
     QB_CUDA(launch_chained(had_chunk_gateup_kernel<K_>, dim3(K_, unsigned(rows)), dim3(threads), chunk_smem, s, a, sv_up)); \
-  else had_row_gateup_kernel<K_><<<unsigned(rows), 1024, row_smem, s>>>(a, sv_up)
+  else QB_CUDA(launch_row(had_row_gateup_kernel<K_>, rows, row_threads, row_smem, s, a, sv_up))
   switch (K) {
-    case 1: had_row_gateup_kernel<1><<<unsigned(rows), 1024, row_smem, s>>>(a, sv_up); break;
+    case 1: QB_CUDA(launch_row(had_row_gateup_kernel<1>, rows, row_threads, row_smem, s, a, sv_up)); break;
     case 12: QB_GATEUP(12); break;
     default:
       if (path == Path::Cluster) {
-        QB_CUDA(launch_cluster(had_cluster_gateup_kernel<28>, rows, size_t(F) * 3, s, a, sv_up));
+        QB_CUDA(launch_cluster(had_cluster_gateup_kernel<28>, rows, size_t(had_room(28 / kHadCluster, a.P)) * 12, s, a, sv_up));
         break;
       }
       QB_GATEUP(28);

@@ -11,8 +11,9 @@ static int configure_in() {
   int rc;
   if ((rc = configure<K, K != 1, Mode::PrepareNorm>())) return rc;
   if ((rc = configure<K, false, Mode::FinishResidual>())) return rc;
-  QB_CUDA(cudaFuncSetAttribute(had_row_residual_input_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (kMaxRowFloats - 1024) * 4));
+  if constexpr (K != 28)
+    QB_CUDA(cudaFuncSetAttribute(had_row_residual_input_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (kMaxRowFloats - 1024) * 4));
   return QTIP_OK;
 }
 int epilogue_residual_device_setup() {
@@ -43,8 +44,11 @@ int hadamard_output_residual(const float* z, int splits, long split_stride, int 
   a.round_z = round_z, a.ranks = ranks;
   return dispatch_epilogue<Mode::FinishResidual>(a, rows, false, s);
 }
-// state += epilogue(z), then u = input transform of the updated state (same width). One kernel per row when the batch
-// is large enough for the whole-row kernels, else the two separate launches: identical results either way.
+// state += epilogue(z), then u = input transform of the updated state (same width): one kernel per row, or the two separate
+// launches, with identical results. The launches are the faster way for few rows, which have the chunk kernels (12,288
+// columns, 24 rows: 11.3 us against 12.5, one row 6.0 against 12.4), and for order 28, whose two transforms in one kernel
+// leave the registers short (3,584 columns, 72 rows 17 us against 20, 2,048 rows 95 against 106; 28,672 columns, 64 rows in four
+// splits 21 against 33).
 int hadamard_output_residual_input(const float* z, int splits, long split_stride, int round_z, int ranks, const float* sv,
                                    int n, int rows, uint16_t* state, const uint16_t* norm, float eps, const float* su,
                                    uint16_t* u, long ldu, uint16_t* xn, cudaStream_t s) {
@@ -56,8 +60,8 @@ int hadamard_output_residual_input(const float* z, int splits, long split_stride
   QB_REQUIRE(K != 20, QTIP_E_GEOMETRY, "the fused epilogues carry the Hadamard orders 1, 12 and 28 (n = %d needs 20)", n);
   if (rows == 0) return QTIP_OK;
   if (fin.ranks > 1) QB_REQUIRE(n % fin.ranks == 0, QTIP_E_GEOMETRY, "n = %d is not divisible by %d ranks", n, fin.ranks);
-  const bool chunks = K > 1 && rows < kChunkRowsBelow && fin.P <= 8192;
-  if (chunks || n > kMaxRowFloats - 1024) {
+  const bool separate = K == 28 || (K > 1 && rows * K <= 2 * 148);
+  if (separate || n > kMaxRowFloats - 1024) {
     int rc = hadamard_output_residual(z, splits, split_stride, round_z, ranks, sv, n, rows, state, s);
     if (rc) return rc;
     return hadamard_input_transform(state, n, norm, eps, su, n, rows, u, ldu, xn, s);
@@ -65,11 +69,10 @@ int hadamard_output_residual_input(const float* z, int splits, long split_stride
   HadArgs prep{};
   prep.dst = u, prep.sign = su, prep.ld_dst = ldu, prep.n = n, prep.splits = 1, prep.P = fin.P, prep.rows = fin.rows;
   prep.scale = fin.scale, prep.norm = norm, prep.eps = eps, prep.xn = xn, prep.factor = 1.f;
-  switch (K) {
-    case 1: had_row_residual_input_kernel<1><<<unsigned(rows), 1024, size_t(n) * 4, s>>>(fin, prep); break;
-    case 12: had_row_residual_input_kernel<12><<<unsigned(rows), 1024, size_t(n) * 4, s>>>(fin, prep); break;
-    default: had_row_residual_input_kernel<28><<<unsigned(rows), 1024, size_t(n) * 4, s>>>(fin, prep); break;
-  }
+  const size_t smem = size_t(had_room(K, fin.P)) * 4;
+  const int threads = had_row_threads(rows, smem + 4096, false);
+  if (K == 1) QB_CUDA(launch_row(had_row_residual_input_kernel<1>, rows, threads, smem, s, fin, prep));
+  else QB_CUDA(launch_row(had_row_residual_input_kernel<12>, rows, threads, smem, s, fin, prep));
   QB_LAUNCHED();
   return QTIP_OK;
 }

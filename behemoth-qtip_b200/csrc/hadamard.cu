@@ -8,7 +8,7 @@
 //    once. Used for the quantizer's fp32 matrices and for prefill-sized token batches.
 //  * had_chunk_kernel: K CTAs per row, each mixing its own chunk from the full row (served by L2) and transforming it.
 //    No inter-CTA step; used for a few tokens where latency, not traffic, decides.
-//  * had_cluster_kernel: a cluster of four CTAs per row for 16 to 64 rows of order 28 (see had_path).
+//  * had_cluster_kernel: a cluster of four CTAs per row for up to 64 rows of order 28 (see had_path).
 //
 // Sources/destinations (Mode): fp32 in place (quantizer); bf16 x times SU -> bf16 (operator input); fp32 partial
 // products summed over K-splits, optionally rounded to bf16 -> times SV -> bf16 (operator output); bf16 z -> same.

@@ -64,9 +64,14 @@ struct SignMasks {
 //   FinishResidual  state = bf16(state + bf16(SV (.) hadU(z)))
 //   FinishGateUp    the gate/up epilogue in two phases of the same code: phase 0 keeps g = bf16(SVg (.) hadU(zg)) in
 //                   shared memory, phase 1 stores h = bf16(silu(g) * bf16(SVu (.) hadU(zu)))
-enum class Mode { F32Inplace, Prepare, Finish, FinishB16, PrepareNorm, PrepareSmem, FinishResidual, FinishGateUp };
+//   FinishGateUpRow the same with g kept in h
+enum class Mode {
+  F32Inplace, Prepare, Finish, FinishB16, PrepareNorm, PrepareSmem, FinishResidual, FinishGateUp, FinishGateUpRow
+};
 template <Mode M>
-constexpr bool kIsFinish = M == Mode::Finish || M == Mode::FinishResidual || M == Mode::FinishGateUp;
+constexpr bool kIsGateUp = M == Mode::FinishGateUp || M == Mode::FinishGateUpRow;
+template <Mode M>
+constexpr bool kIsFinish = M == Mode::Finish || M == Mode::FinishResidual || kIsGateUp<M>;
 template <Mode M>
 constexpr bool kIsPrepare = M == Mode::Prepare || M == Mode::PrepareNorm || M == Mode::PrepareSmem;
 
@@ -86,11 +91,17 @@ struct HadArgs {
   const uint16_t* norm;  // PrepareNorm / PrepareSmem: RMSNorm weight (bf16) or null
   uint16_t* xn;          // PrepareNorm / PrepareSmem: normalised row out [rows][n] (bf16) or null
   float eps, factor;     // factor = rsqrt(mean(x^2) + eps), computed per row inside the kernel
-  float* aux;            // shared-memory row: FinishResidual / FinishGateUp (phase 0) write it, phase 1 / PrepareSmem read it
+  float* aux;            // shared memory: FinishResidual leaves the updated row there for PrepareSmem (at had_row_place), FinishGateUp the gate
   int phase;             // FinishGateUp: 0 = gate, 1 = up
   int aux_base;          // element index of aux[0] within the row (chunk kernels hold one chunk)
   bool write_xn;         // this CTA writes xn (one CTA per row does)
 };
+
+// Place of element i of a chunk: the eight float4 of each run of 32 are permuted by the run's number, so that 32 lanes may
+// read a run each in 16-byte pieces (bits 0..4) or an element of one run each (bits 5..9) without bank conflicts.
+__device__ __forceinline__ int had_place(int i) { return (i & ~28) | (((i >> 2 ^ i >> 5) & 7) << 2); }
+// The same for element j of a row of chunks of P.
+__device__ __forceinline__ int had_row_place(int j, int P) { return P >= 32 ? (j & -P) | had_place(j & (P - 1)) : j; }
 
 // Element offset of column element j of `row` relative to the source base: row-major, or [rank][row][n / ranks] when
 // the source was gathered from `ranks` ranks.
@@ -104,24 +115,57 @@ __device__ __forceinline__ float load_one(const void* src, long at) {
   if constexpr (M == Mode::F32Inplace || kIsFinish<M> || M == Mode::PrepareSmem) return static_cast<const float*>(src)[at];
   else return bf16_to_f32(static_cast<const uint16_t*>(src)[at]);
 }
-// The K source values of column i (elements k P + i), loaded as one batch: the K loads of a pass are independent
-// straight-line code, so they are all in flight together (per-element control flow around each load would serialise
-// them on memory latency). K-split partials are added in split order, then optionally rounded to bf16.
-template <int K, Mode M>
+// v = the sums of S partials in split order, kFlight loads in flight at a time (all of them for S = 1).
+template <int K, int S, int kFlight>
+__device__ __forceinline__ void load_partials(const float* z, size_t split_stride, int P, float (&v)[K]) {
+  constexpr int B = S == 1 ? K : (kFlight / S < K ? kFlight / S : K);
+#pragma unroll
+  for (int k0 = 0; k0 < K; k0 += B) {
+    float part[S][B];
+#pragma unroll
+    for (int p = 0; p < S; ++p)
+#pragma unroll
+      for (int k = 0; k < B; ++k)
+        if (k0 + k < K) part[p][k] = z[p * split_stride + (k0 + k) * P];
+#pragma unroll
+    for (int k = 0; k < B; ++k)
+      if (k0 + k < K) {
+        v[k0 + k] = part[0][k];
+#pragma unroll
+        for (int p = 1; p < S; ++p) v[k0 + k] += part[p][k];
+      }
+    if constexpr (S > 1) asm volatile("" ::: "memory");  // the next batch's loads stay behind: bounds register use
+  }
+}
+// The K source values of column i (elements k P + i), loaded in batches of independent straight-line code, so that the loads
+// of a batch are in flight together (per-element control flow around each load would serialise them on memory latency).
+// K-split partials are added in split order, then optionally rounded to bf16. kFlight: partials in flight per thread, 32
+// where few threads wait for them, 16 in the whole-row kernel, which has 64 registers (gate/up of 64 rows of 28,672 in four
+// splits 25.5 us with the splits loaded one after another, 18.4 so).
+template <int K, Mode M, int kFlight = 16>
 __device__ __forceinline__ void load_column(const HadArgs& a, long row, int i, int P, float (&v)[K]) {
   if (a.ranks <= 1) {
-    const long base = row * a.ld + i;
-#pragma unroll
-    for (int k = 0; k < K; ++k) v[k] = load_one<M>(a.src, base + k * P);
+    const long base = M == Mode::PrepareSmem ? had_row_place(i, P) : row * a.ld + i;
     if constexpr (kIsFinish<M>) {
-      for (int p = 1; p < a.splits; ++p) {
-        const float* zp = static_cast<const float*>(a.src) + size_t(p) * a.split_stride + base;
+      const float* z = static_cast<const float*>(a.src) + base;
+      const size_t stride = size_t(a.split_stride);
+      switch (a.splits) {
+        case 1: load_partials<K, 1, kFlight>(z, stride, P, v); break;
+        case 2: load_partials<K, 2, kFlight>(z, stride, P, v); break;
+        case 3: load_partials<K, 3, kFlight>(z, stride, P, v); break;
+        default: load_partials<K, 4, kFlight>(z, stride, P, v); break;
+      }
+      for (int p = 4; p < a.splits; ++p) {
+        const float* zp = z + p * stride;
 #pragma unroll
         for (int k = 0; k < K; ++k) {
           v[k] += zp[k * P];
-          if (k % 8 == 7) asm volatile("" ::: "memory");  // at most 8 partial loads in flight: bounds register use
+          if (k % 8 == 7) asm volatile("" ::: "memory");
         }
       }
+    } else {
+#pragma unroll
+      for (int k = 0; k < K; ++k) v[k] = load_one<M>(a.src, base + k * P);
     }
   } else {
     // gathered source: a chunk never straddles two ranks' parts (n / ranks is a multiple of P), so one offset per chunk
@@ -147,7 +191,7 @@ __device__ __forceinline__ void load_column(const HadArgs& a, long row, int i, i
   }
   if constexpr (kIsPrepare<M>) {
 #pragma unroll
-    for (int k = 0; k < K; ++k) v[k] *= a.sign[k * P + i];
+    for (int k = 0; k < K; ++k) v[k] *= __ldg(a.sign + k * P + i);
   }
   if constexpr (kIsFinish<M>) {
     if (a.round_z) {
@@ -156,46 +200,67 @@ __device__ __forceinline__ void load_column(const HadArgs& a, long row, int i, i
     }
   }
 }
-template <Mode M>
-__device__ __forceinline__ void store_dst(const HadArgs& a, long row, int j, float v) {
+// Elements j, j + step, .. of the result. What they are combined with is loaded before the first store: behind a store, which
+// may alias for all the compiler knows, every load would wait out its own latency (residual of 2,048 rows of 12,288: 143 us
+// one by one).
+template <Mode M, int N>
+__device__ __forceinline__ void store_run(const HadArgs& a, long row, int j, int step, const float* v) {
   const long at = row * (a.ld_dst ? a.ld_dst : a.ld) + j;
+  uint16_t* dst = static_cast<uint16_t*>(a.dst) + at;
+  float sign[N];
+  if constexpr (M != Mode::F32Inplace && !kIsPrepare<M>) {
+#pragma unroll
+    for (int r = 0; r < N; ++r) sign[r] = __ldg(a.sign + j + r * step);
+  }
+  auto value = [&](int r) { return f32_to_bf16(v[r] * a.scale * sign[r]); };
   if constexpr (M == Mode::F32Inplace) {
-    static_cast<float*>(a.dst)[at] = v * a.scale;
+#pragma unroll
+    for (int r = 0; r < N; ++r) static_cast<float*>(a.dst)[at + r * step] = v[r] * a.scale;
   } else if constexpr (kIsPrepare<M>) {
-    static_cast<uint16_t*>(a.dst)[at] = f32_to_bf16(v * a.scale);
+#pragma unroll
+    for (int r = 0; r < N; ++r) dst[r * step] = f32_to_bf16(v[r] * a.scale);
   } else if constexpr (M == Mode::FinishResidual) {
-    uint16_t* st = static_cast<uint16_t*>(a.dst) + at;
-    const float t = bf16_to_f32(f32_to_bf16(v * a.scale * a.sign[j]));
-    const uint16_t nb = f32_to_bf16(bf16_to_f32(*st) + t);
-    *st = nb;
-    if (a.aux) a.aux[j - a.aux_base] = bf16_to_f32(nb);  // the updated row, for a fused next-input transform
-  } else if constexpr (M == Mode::FinishGateUp) {
-    const float t = bf16_to_f32(f32_to_bf16(v * a.scale * a.sign[j]));
+    uint16_t old[N];
+#pragma unroll
+    for (int r = 0; r < N; ++r) old[r] = dst[r * step];
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+      const uint16_t nb = f32_to_bf16(bf16_to_f32(old[r]) + bf16_to_f32(value(r)));
+      dst[r * step] = nb;
+      if (a.aux) a.aux[had_row_place(j + r * step, a.P)] = bf16_to_f32(nb);  // for a fused next-input transform
+    }
+  } else if constexpr (kIsGateUp<M>) {
+    float* aux = a.aux + (j - a.aux_base);  // FinishGateUp only
     if (a.phase == 0) {
-      a.aux[j - a.aux_base] = t;
+#pragma unroll
+      for (int r = 0; r < N; ++r) {
+        if constexpr (M == Mode::FinishGateUp) aux[r * step] = bf16_to_f32(value(r));
+        else dst[r * step] = value(r);
+      }
     } else {
-      const float g = a.aux[j - a.aux_base];
-      static_cast<uint16_t*>(a.dst)[at] = f32_to_bf16(g / (1.f + expf(-g)) * t);
+      float g[N];
+#pragma unroll
+      for (int r = 0; r < N; ++r) {
+        if constexpr (M == Mode::FinishGateUp) g[r] = aux[r * step];
+        else g[r] = bf16_to_f32(dst[r * step]);
+      }
+#pragma unroll
+      for (int r = 0; r < N; ++r) dst[r * step] = f32_to_bf16(g[r] / (1.f + expf(-g[r])) * bf16_to_f32(value(r)));
     }
   } else {
-    static_cast<uint16_t*>(a.dst)[at] = f32_to_bf16(v * a.scale * a.sign[j]);
+#pragma unroll
+    for (int r = 0; r < N; ++r) dst[r * step] = value(r);
   }
 }
-
-// rsqrt(mean(x^2) + eps) of one row, the same bits whatever the CTA's thread count: 1,024 slots (slot i adds the
-// squares of elements i, i + 1024, ... in ascending order), then one warp adds the slots 32 apart in ascending order
-// and folds its 32 lanes with a butterfly. `slots` is shared memory for 1,024 floats. All threads must call it.
 template <Mode M>
-__device__ __forceinline__ float row_norm_factor(const HadArgs& a, long row, float* slots) {
+__device__ __forceinline__ void store_dst(const HadArgs& a, long row, int j, float v) {
+  store_run<M, 1>(a, row, j, 0, &v);
+}
+
+// The sum of the slots of a row's squares (one warp adds the slots 32 apart in ascending order and folds its 32 lanes with a
+// butterfly), as rsqrt(mean + eps). All threads must call it; `slots` may be overwritten afterwards.
+__device__ __forceinline__ float fold_norm_slots(const HadArgs& a, float* slots) {
   const int ns = a.n < 1024 ? a.n : 1024;
-  for (int i = threadIdx.x; i < ns; i += blockDim.x) {
-    float ss = 0.f;
-    for (int e = i; e < a.n; e += 1024) {
-      const float x = M == Mode::PrepareSmem ? a.aux[e] : bf16_to_f32(static_cast<const uint16_t*>(a.src)[row * a.ld + e]);
-      ss = fmaf(x, x, ss);
-    }
-    slots[i] = ss;
-  }
   __syncthreads();
   float total = 0.f;
   if (threadIdx.x < 32) {
@@ -208,6 +273,59 @@ __device__ __forceinline__ float row_norm_factor(const HadArgs& a, long row, flo
   total = slots[0];
   __syncthreads();
   return rsqrtf(total / float(a.n) + a.eps);
+}
+// rsqrt(mean(x^2) + eps) of one row, the same bits whatever the CTA's thread count: 1,024 slots (slot i adds the
+// squares of elements i, i + 1024, ... in ascending order), then one warp adds the slots 32 apart in ascending order
+// and folds its 32 lanes with a butterfly. `slots` is shared memory for 1,024 floats. All threads must call it.
+template <Mode M>
+__device__ __forceinline__ float row_norm_factor(const HadArgs& a, long row, float* slots) {
+  const int ns = a.n < 1024 ? a.n : 1024;
+  for (int i = threadIdx.x; i < ns; i += blockDim.x) {
+    float ss = 0.f;
+    for (int e0 = i; e0 < a.n; e0 += 8 * 1024) {
+      float x[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {  // eight loads in flight; what lies behind the row adds zero, which changes no sum of squares
+        const int e = e0 + q * 1024;
+        x[q] = 0.f;
+        if (e < a.n)
+          x[q] = M == Mode::PrepareSmem ? a.aux[had_row_place(e, a.P)]
+                                        : bf16_to_f32(static_cast<const uint16_t*>(a.src)[row * a.ld + e]);
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) ss = fmaf(x[q], x[q], ss);
+    }
+    slots[i] = ss;
+  }
+  return fold_norm_slots(a, slots);
+}
+// A column of a row of K chunks of 1,024 in a CTA of 1,024 threads: its K elements are the ones that the thread's slot adds, so
+// one trip to memory serves the norm and the transform, and (where the registers hold them) brings the weights and signs
+// along.
+template <int K>
+__device__ __forceinline__ void norm_column_1024(HadArgs& a, long row, float* slots, float (&v)[K]) {
+  constexpr bool kAhead = K <= 12;
+  const int i = threadIdx.x;
+  const uint16_t* x = static_cast<const uint16_t*>(a.src) + row * a.ld + i;
+  float sign[kAhead ? K : 1];
+  uint16_t w[kAhead ? K : 1];
+#pragma unroll
+  for (int k = 0; k < K; ++k) v[k] = bf16_to_f32(x[k * 1024]);
+  if constexpr (kAhead) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) w[k] = __ldg(a.norm + k * 1024 + i), sign[k] = __ldg(a.sign + k * 1024 + i);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < K; ++k) ss = fmaf(v[k], v[k], ss);
+  slots[i] = ss;
+  a.factor = fold_norm_slots(a, slots);
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const uint16_t xb = f32_to_bf16(v[k] * a.factor * bf16_to_f32(kAhead ? w[kAhead ? k : 0] : __ldg(a.norm + k * 1024 + i)));
+    if (a.xn && a.write_xn) a.xn[row * a.n + k * 1024 + i] = xb;
+    v[k] = bf16_to_f32(xb) * (kAhead ? sign[kAhead ? k : 0] : __ldg(a.sign + k * 1024 + i));
+  }
 }
 
 // Natural-order FWHT on `count` contiguous chunks of P floats in shared memory (any power-of-two P). All threads of the
@@ -268,7 +386,7 @@ __device__ __forceinline__ void fwht_regs(float (&v)[R], float* buf) {
       }
 }
 
-// Mixed value of chunk r at column i: sum over k (ascending) of +-v[k].
+// Mixed value of chunk r at column i: sum over k (ascending) of +-v[k], by a mask known at run time / at compile time.
 template <int K>
 __device__ __forceinline__ float mix_row(const float (&v)[K], uint32_t mask) {
   float s = 0.f;
@@ -276,111 +394,170 @@ __device__ __forceinline__ float mix_row(const float (&v)[K], uint32_t mask) {
   for (int k = 0; k < K; ++k) s += __uint_as_float(__float_as_uint(v[k]) ^ (((mask >> k) & 1u) << 31));
   return s;
 }
-
-// Natural-order FWHT of 1,024 floats by ONE warp, no block-level synchronisation: v[r] is element 32 r + lane. Index
-// bits 0..4 (the lane) are butterflied with shuffles, bits 5..9 (r) between the registers of a thread. Same stage order
-// as fwht_shared / fwht_regs, therefore the same bits.
-__device__ __forceinline__ void fwht_warp_1024(float (&v)[32]) {
-  const int lane = threadIdx.x & 31;
+template <int K>
+__device__ __forceinline__ float mix_fixed(const float (&v)[K], uint32_t mask) {
+  float s = 0.f;
 #pragma unroll
-  for (int h = 1; h < 32; h <<= 1) {
-    const bool upper = lane & h;
-#pragma unroll
-    for (int r = 0; r < 32; ++r) {
-      const float p = __shfl_xor_sync(0xffffffffu, v[r], h);
-      v[r] = upper ? p - v[r] : v[r] + p;
-    }
-  }
-#pragma unroll
-  for (int h = 1; h < 32; h <<= 1)
-#pragma unroll
-    for (int r = 0; r < 32; ++r)
-      if ((r & h) == 0) {
-        const float x = v[r], y = v[r + h];
-        v[r] = x + y;
-        v[r + h] = x - y;
-      }
+  for (int k = 0; k < K; ++k) s = (mask >> k) & 1u ? s - v[k] : s + v[k];
+  return s;
 }
 
-// FWHT of K chunks (P = 1024 H floats each, H = 1 or 2; the row's chunks chunk0, chunk0 + 1, ...) of a mixed row in shared
-// memory, one 1,024-float unit per warp at a time, results straight to the destination (H = 1) or after one more stage
-// across the two halves (H = 2).
-template <int H, Mode M>
-__device__ __forceinline__ void row_chunks_warp(const HadArgs& a, long row, float* row_s, int K, int chunk0 = 0) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  for (int u = warp; u < K * H; u += nwarps) {
+// ---- the FWHT of whole chunks in shared memory, 32 values a thread at a time
+template <int H>
+__device__ __forceinline__ void butterflies(float (&v)[H], int below = H) {
+#pragma unroll
+  for (int h = 1; h < H; h <<= 1)
+    if (h < below) {
+#pragma unroll
+      for (int r = 0; r < H; ++r)
+        if ((r & h) == 0) {
+          const float x = v[r], y = v[r + h];
+          v[r] = x + y;
+          v[r + h] = x - y;
+        }
+    }
+}
+// Bits 10 and up of chunks of several units of 1,024 floats: butterflies between H units that lie `stride` units apart, to
+// the destination (kLast) or back in place.
+template <int H, bool kLast, Mode M>
+__device__ __forceinline__ void across_units(const HadArgs& a, long row, float* row_s, int units, int stride, int first) {
+  for (int j = threadIdx.x; j < units / H * 1024; j += blockDim.x) {
+    const int q = j >> 10, i = j & 1023, unit = (q & (stride - 1)) + q / stride * (stride * H);
+    float v[H];
+#pragma unroll
+    for (int t = 0; t < H; ++t) v[t] = row_s[(unit + t * stride) * 1024 + had_place(i)];
+    butterflies(v);
+    if constexpr (kLast) {
+      store_run<M, H>(a, row, first + unit * 1024 + i, stride * 1024, v);
+    } else {
+#pragma unroll
+      for (int t = 0; t < H; ++t) row_s[(unit + t * stride) * 1024 + had_place(i)] = v[t];
+    }
+  }
+}
+// Natural-order FWHT of `count` chunks of P >= 32 floats (the row's chunks chunk0, chunk0 + 1, ...) at had_place() of row_s,
+// to the destination. A warp takes 1,024 floats at a time (row_s has room for whole units; what lies behind the last
+// chunk is transformed and dropped): a run of 32 per lane, butterflies over bits 0..4 in registers, back in place; then
+// a column of 32 runs per lane, over bits 5..9 (fewer for P < 1,024). No shuffles: they cost the shared-memory pipe one
+// pass per value and stage, these two exchanges three passes per value in all. Stages ascend (h = 1, 2, 4, ...) as in
+// fwht_shared and fwht_regs, therefore the same bits.
+template <Mode M>
+__device__ __forceinline__ void chunks_fwht(const HadArgs& a, long row, float* row_s, int count, int chunk0 = 0) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
+  const int runs = a.P >> 5, total = count * runs, key = (runs - 1) & 7;
+  for (int u = warp; u * 32 < total; u += nwarps) {
     float* unit = row_s + u * 1024;
     float v[32];
+    float4* run = reinterpret_cast<float4*>(unit + lane * 32);
 #pragma unroll
-    for (int r = 0; r < 32; ++r) v[r] = unit[32 * r + lane];
-    fwht_warp_1024(v);
+    for (int q = 0; q < 8; ++q) {
+      const float4 f = run[q ^ (lane & key)];
+      v[4 * q] = f.x, v[4 * q + 1] = f.y, v[4 * q + 2] = f.z, v[4 * q + 3] = f.w;
+    }
+    butterflies(v);
 #pragma unroll
-    for (int r = 0; r < 32; ++r) {
-      if constexpr (H == 1) store_dst<M>(a, row, (chunk0 * H + u) * 1024 + 32 * r + lane, v[r]);
-      else unit[32 * r + lane] = v[r];
+    for (int q = 0; q < 8; ++q) run[q ^ (lane & key)] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    __syncwarp();
+    float* column = unit + (lane & 3);
+#pragma unroll
+    for (int r = 0; r < 32; ++r) v[r] = column[r * 32 + (((lane >> 2) ^ (r & key)) << 2)];
+    butterflies(v, runs);
+    if (a.P > 1024) {
+#pragma unroll
+      for (int r = 0; r < 32; ++r) column[r * 32 + (((lane >> 2) ^ (r & key)) << 2)] = v[r];
+    } else {
+      const int j0 = chunk0 * a.P + u * 1024 + lane, left = total - u * 32;
+      if (left >= 32) {
+#pragma unroll
+        for (int r = 0; r < 32; r += 8) store_run<M, 8>(a, row, j0 + 32 * r, 32, v + r);
+      } else {
+#pragma unroll
+        for (int r = 0; r < 32; r += 4) {
+          if (r + 4 <= left) {
+            store_run<M, 4>(a, row, j0 + 32 * r, 32, v + r);
+          } else {
+#pragma unroll
+            for (int q = r; q < r + 4; ++q)
+              if (q < left) store_dst<M>(a, row, j0 + 32 * q, v[q]);
+          }
+        }
+      }
     }
   }
-  if constexpr (H == 2) {
-    __syncthreads();
-    for (int j = threadIdx.x; j < K * 1024; j += blockDim.x) {
-      const int c = j >> 10, i = j & 1023;
-      const float x = row_s[c * 2048 + i], y = row_s[c * 2048 + 1024 + i];
-      store_dst<M>(a, row, (chunk0 + c) * 2048 + i, x + y);
-      store_dst<M>(a, row, (chunk0 + c) * 2048 + 1024 + i, x - y);
-    }
+  if (a.P <= 1024) return;
+  __syncthreads();
+  const int units = count * (a.P >> 10), first = chunk0 * a.P;
+  switch (a.P >> 10) {
+    case 2: return across_units<2, true, M>(a, row, row_s, units, 1, first);
+    case 4: return across_units<4, true, M>(a, row, row_s, units, 1, first);
+    case 8: return across_units<8, true, M>(a, row, row_s, units, 1, first);
+    default: break;  // 16,384 and 32,768, the longest powers of two that fit
   }
+  across_units<8, false, M>(a, row, row_s, units, 1, first);
+  __syncthreads();
+  if (a.P >> 10 == 16) across_units<2, true, M>(a, row, row_s, units, 8, first);
+  else across_units<4, true, M>(a, row, row_s, units, 8, first);
 }
+// Floats of shared memory for `count` chunks of P: whole units.
+inline __host__ __device__ int had_room(int count, int P) { return (count * P + 1023) & ~1023; }
 
-// One row, whole in shared memory (row_s: n floats): mix, FWHT per chunk, store. Called by every thread of the CTA.
+// One row, whole in shared memory (row_s: had_room(K, P) floats): mix, FWHT per chunk, store. Called by every thread of the CTA.
 template <int K, bool T, Mode M>
-__device__ __forceinline__ void row_transform(const HadArgs& a, long row, float* row_s) {
+__device__ __forceinline__ void row_transform(HadArgs& a, long row, float* row_s) {
   constexpr SignMasks<K, T> masks{};
   const int P = a.P;
-  if constexpr (K == 1) {
-    for (int i = threadIdx.x; i < P; i += blockDim.x) {
-      float v[1];
-      load_column<1, M>(a, row, i, P, v);
-      row_s[i] = v[0];
-    }
-  } else {
-    for (int i = threadIdx.x; i < P; i += blockDim.x) {
+  if constexpr (M == Mode::PrepareNorm && K > 1) {
+    if (a.norm && P == 1024 && blockDim.x == 1024) {
       float v[K];
-      load_column<K, M>(a, row, i, P, v);
+      norm_column_1024<K>(a, row, row_s, v);
+      float* at = row_s + had_place(threadIdx.x);
 #pragma unroll
-      for (int r = 0; r < K; ++r) row_s[r * P + i] = mix_row<K>(v, masks.m[r]);
+      for (int r = 0; r < K; ++r) at[r * P] = mix_fixed<K>(v, masks.m[r]);
+      __syncthreads();
+      return chunks_fwht<M>(a, row, row_s, K);
     }
+    if (a.norm) a.factor = row_norm_factor<M>(a, row, row_s);  // slots where the row will be: two rows of 28,672 fit an SM
+  } else if constexpr (M == Mode::PrepareNorm) {
+    if (a.norm) a.factor = row_norm_factor<M>(a, row, row_s);
+  }
+  for (int i = threadIdx.x; i < P; i += blockDim.x) {
+    float v[K];
+    load_column<K, M>(a, row, i, P, v);
+    float* at = row_s + (P >= 32 ? had_place(i) : i);
+#pragma unroll
+    for (int r = 0; r < K; ++r) at[r * P] = mix_fixed<K>(v, masks.m[r]);
   }
   __syncthreads();
-  if (P == 1024) return row_chunks_warp<1, M>(a, row, row_s, K);
-  if (P == 2048) return row_chunks_warp<2, M>(a, row, row_s, K);
+  if (P >= 32) return chunks_fwht<M>(a, row, row_s, K);
   fwht_shared(row_s, P, K);
   for (int j = threadIdx.x; j < a.n; j += blockDim.x) store_dst<M>(a, row, j, row_s[j]);
 }
 
+__device__ __forceinline__ void row_chain() {
+  if (gridDim.x < 32) chain_release();  // see launch_row
+  chain_wait();
+}
 template <int K, bool T, Mode M>
 __global__ __launch_bounds__(1024, 1) void had_row_kernel(HadArgs a) {
-  extern __shared__ float row_s[];
+  extern __shared__ __align__(16) float row_s[];
   const long row = blockIdx.x;
-  if constexpr (M == Mode::PrepareNorm) {
-    __shared__ float slots[1024];
-    a.write_xn = true;
-    if (a.norm) a.factor = row_norm_factor<M>(a, row, slots);
-  }
+  row_chain();
+  a.write_xn = true;
   row_transform<K, T, M>(a, row, row_s);
 }
 
-// Gate/up epilogue of one row: g = bf16(SVg (.) hadU(zg)) into the second half of the shared row, then the up transform
-// in the first half with h = bf16(silu(g) * u) as its store. `a` describes the gate half; the up half sits F elements
-// further in the source row and uses sign2.
+// Gate/up epilogue of one row: g = bf16(SVg (.) hadU(zg)) into h, then the up transform with h = bf16(silu(g) * u) as its
+// store; the thread that reads g back is the one that wrote it. (Kept in shared memory g would leave room for one row an
+// SM instead of two.) `a` describes the gate half; the up half sits F elements further in the source row and uses sign_up.
 template <int K>
 __global__ __launch_bounds__(1024, 1) void had_row_gateup_kernel(HadArgs a, const float* sign_up) {
-  extern __shared__ float row_s[];
+  extern __shared__ __align__(16) float row_s[];
   const long row = blockIdx.x;
-  a.aux = row_s + a.n, a.aux_base = 0;
+  row_chain();
 #pragma unroll 1
   for (int phase = 0; phase < 2; ++phase) {  // one copy of the transform code, run twice
     a.phase = phase;
-    row_transform<K, false, Mode::FinishGateUp>(a, row, row_s);
+    row_transform<K, false, Mode::FinishGateUpRow>(a, row, row_s);
     __syncthreads();
     a.src = static_cast<const float*>(a.src) + a.n;
     a.sign = sign_up;
@@ -391,10 +568,11 @@ __global__ __launch_bounds__(1024, 1) void had_row_gateup_kernel(HadArgs a, cons
 // hadU(z))), kept in shared memory as it is stored, then u = bf16(hadUt(SU (.) rmsnorm(state))) from there.
 template <int K>
 __global__ __launch_bounds__(1024, 1) void had_row_residual_input_kernel(HadArgs fin, HadArgs prep) {
-  extern __shared__ float row_s[];
+  extern __shared__ __align__(16) float row_s[];
   __shared__ float slots[1024];
   const long row = blockIdx.x;
-  fin.aux = row_s, fin.aux_base = 0;
+  row_chain();
+  fin.aux = row_s;
   row_transform<K, false, Mode::FinishResidual>(fin, row, row_s);
   __syncthreads();
   prep.src = row_s, prep.aux = row_s, prep.ld = 0, prep.write_xn = true;
@@ -403,14 +581,19 @@ __global__ __launch_bounds__(1024, 1) void had_row_residual_input_kernel(HadArgs
 }
 
 template <int K, int R, Mode M>
-__device__ __forceinline__ void chunk_regs(const HadArgs& a, long row, int r_out, uint32_t mask, float* buf) {
+__device__ __forceinline__ void chunk_regs(HadArgs& a, long row, int r_out, uint32_t mask, float* buf, float* slots) {
   const int P = 1024 * R;
   float w[R];
 #pragma unroll
   for (int q = 0; q < R; ++q) {
     const int i = threadIdx.x + 1024 * q;
     float v[K];
-    load_column<K, M>(a, row, i, P, v);
+    if constexpr (M == Mode::PrepareNorm && R == 1) {
+      if (slots) norm_column_1024<K>(a, row, slots, v);
+      else load_column<K, M, 32>(a, row, i, P, v);
+    } else {
+      load_column<K, M, 32>(a, row, i, P, v);
+    }
     w[q] = mix_row<K>(v, mask);
   }
   fwht_regs<R>(w, buf);
@@ -418,20 +601,21 @@ __device__ __forceinline__ void chunk_regs(const HadArgs& a, long row, int r_out
   for (int q = 0; q < R; ++q) store_dst<M>(a, row, r_out * P + threadIdx.x + 1024 * q, w[q]);
 }
 
-// Output chunk r of one row by one CTA (smem: P floats, or 1,024 as the transpose buffer of the register path).
+// Output chunk r of one row by one CTA (smem: P floats, or 1,024 as the transpose buffer of the register path). slots: not null
+// where the norm is yet to be taken, for rows of chunks of 1,024.
 template <int K, bool T, Mode M>
-__device__ __forceinline__ void chunk_transform(const HadArgs& a, long row, int r, float* smem) {
+__device__ __forceinline__ void chunk_transform(HadArgs& a, long row, int r, float* smem, float* slots = nullptr) {
   constexpr SignMasks<K, T> masks{};
   const int P = a.P;
   uint32_t mask = 0;
 #pragma unroll
   for (int q = 0; q < K; ++q)
     if (q == r) mask = masks.m[q];
-  if (P == 1024 && blockDim.x == 1024) return chunk_regs<K, 1, M>(a, row, r, mask, smem);
-  if (P == 2048 && blockDim.x == 1024) return chunk_regs<K, 2, M>(a, row, r, mask, smem);
+  if (P == 1024 && blockDim.x == 1024) return chunk_regs<K, 1, M>(a, row, r, mask, smem, slots);
+  if (P == 2048 && blockDim.x == 1024) return chunk_regs<K, 2, M>(a, row, r, mask, smem, slots);
   for (int i = threadIdx.x; i < P; i += blockDim.x) {
     float v[K];
-    load_column<K, M>(a, row, i, P, v);
+    load_column<K, M, 32>(a, row, i, P, v);
     smem[i] = mix_row<K>(v, mask);
   }
   __syncthreads();
@@ -441,7 +625,7 @@ __device__ __forceinline__ void chunk_transform(const HadArgs& a, long row, int 
 
 template <int K, bool T, Mode M>
 __global__ __launch_bounds__(1024, 1) void had_chunk_kernel(HadArgs a) {
-  extern __shared__ float row_s[];
+  extern __shared__ __align__(16) float row_s[];
   const int r = blockIdx.x;
   const long row = blockIdx.y;
   chain_release();
@@ -449,6 +633,7 @@ __global__ __launch_bounds__(1024, 1) void had_chunk_kernel(HadArgs a) {
   if constexpr (M == Mode::PrepareNorm) {
     __shared__ float slots[1024];
     a.write_xn = r == 0;
+    if (a.norm && a.P == 1024 && blockDim.x == 1024) return chunk_transform<K, T, M>(a, row, r, row_s, slots);
     if (a.norm) a.factor = row_norm_factor<M>(a, row, slots);
   }
   chunk_transform<K, T, M>(a, row, r, row_s);
@@ -457,7 +642,7 @@ __global__ __launch_bounds__(1024, 1) void had_chunk_kernel(HadArgs a) {
 // Gate/up epilogue, chunk r of one row: g chunk into shared memory behind the work area, then the up chunk.
 template <int K>
 __global__ __launch_bounds__(1024, 1) void had_chunk_gateup_kernel(HadArgs a, const float* sign_up) {
-  extern __shared__ float row_s[];
+  extern __shared__ __align__(16) float row_s[];
   const int r = blockIdx.x;
   const long row = blockIdx.y;
   const int work = a.P > 1024 ? a.P : 1024;
@@ -504,7 +689,7 @@ __device__ __forceinline__ void had_peer_store(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
 
-// work: K / 4 chunks of P floats in every CTA of the cluster, free in all of them when this is called.
+// work: had_room(K / 4, P) floats in every CTA of the cluster, free in all of them when this is called.
 template <int K, bool T, Mode M>
 __device__ __forceinline__ void cluster_transform(const HadArgs& a, long row, float* work, int q) {
   constexpr SignMasks<K, T> masks{};
@@ -515,34 +700,26 @@ __device__ __forceinline__ void cluster_transform(const HadArgs& a, long row, fl
   for (int o = 0; o < kHadCluster; ++o) peer[o] = had_peer(work, o);
   for (int i = q * cols + threadIdx.x; i < (q + 1) * cols; i += blockDim.x) {
     float v[K];
-    load_column<K, M>(a, row, i, P, v);
+    load_column<K, M, 32>(a, row, i, P, v);
+    const int place = P >= 32 ? had_place(i) : i;
 #pragma unroll
     for (int r = 0; r < K; ++r)
-      had_peer_store(peer[r / KC] + uint32_t((r % KC) * P + i) * 4u, mix_row<K>(v, masks.m[r]));
+      had_peer_store(peer[r / KC] + uint32_t((r % KC) * P + place) * 4u, mix_fixed<K>(v, masks.m[r]));
   }
   had_cluster_sync();
-  if (P == 1024) return row_chunks_warp<1, M>(a, row, work, KC, q * KC);
-  if (P == 2048) return row_chunks_warp<2, M>(a, row, work, KC, q * KC);
+  if (P >= 32) return chunks_fwht<M>(a, row, work, KC, q * KC);
   fwht_shared(work, P, KC);
   for (int j = threadIdx.x; j < KC * P; j += blockDim.x) store_dst<M>(a, row, q * KC * P + j, work[j]);
 }
 
 template <int K, bool T, Mode M>
 __global__ __cluster_dims__(kHadCluster, 1, 1) __launch_bounds__(kClusterThreads, 2) void had_cluster_kernel(HadArgs a) {
-  extern __shared__ float row_s[];
+  extern __shared__ __align__(16) float row_s[];
   const int q = blockIdx.x;
   const long row = blockIdx.y;
-  // The first cluster barrier: every CTA of the cluster runs before one stores into another. With a norm it also stands
-  // between the reads of the whole row for the norm and the first store of xn, which may be the row itself.
-  if constexpr (M != Mode::PrepareNorm) had_cluster_arrive();
+  had_cluster_arrive();  // every CTA of the cluster runs before one stores into another
   chain_release();
   chain_wait();
-  if constexpr (M == Mode::PrepareNorm) {
-    __shared__ float slots[1024];
-    a.write_xn = true;  // a column is mixed by one CTA only
-    if (a.norm) a.factor = row_norm_factor<M>(a, row, slots);
-    had_cluster_arrive();
-  }
   had_cluster_wait();
   cluster_transform<K, T, M>(a, row, row_s, q);
 }
@@ -552,10 +729,10 @@ __global__ __cluster_dims__(kHadCluster, 1, 1) __launch_bounds__(kClusterThreads
 template <int K>
 __global__ __cluster_dims__(kHadCluster, 1, 1) __launch_bounds__(kClusterThreads, 2) void had_cluster_gateup_kernel(
     HadArgs a, const float* sign_up) {
-  extern __shared__ float row_s[];
-  const int q = blockIdx.x, own = a.n / kHadCluster;
+  extern __shared__ __align__(16) float row_s[];
+  const int q = blockIdx.x, own = a.n / kHadCluster, room = had_room(K / kHadCluster, a.P);
   const long row = blockIdx.y;
-  a.aux = row_s + 2 * own, a.aux_base = q * own;
+  a.aux = row_s + 2 * room, a.aux_base = q * own;
   had_cluster_arrive();
   chain_release();
   chain_wait();
@@ -563,7 +740,7 @@ __global__ __cluster_dims__(kHadCluster, 1, 1) __launch_bounds__(kClusterThreads
 #pragma unroll 1
   for (int phase = 0; phase < 2; ++phase) {
     a.phase = phase;
-    cluster_transform<K, false, Mode::FinishGateUp>(a, row, row_s + phase * own, q);
+    cluster_transform<K, false, Mode::FinishGateUp>(a, row, row_s + phase * room, q);
     __syncthreads();
     a.src = static_cast<const float*>(a.src) + a.n;
     a.sign = sign_up;
@@ -571,37 +748,44 @@ __global__ __cluster_dims__(kHadCluster, 1, 1) __launch_bounds__(kClusterThreads
 }
 
 constexpr int kMaxRowFloats = 57344;  // 224 KiB of the 227 KiB a CTA may hold
-constexpr int kChunkRowsBelow = 32;  // fewer rows than this: K CTAs per row
-// Kernel of a transform by its row count and shape; `room`: longest row of the whole-row kernel. A cluster per row from 16 to
-// 64 rows of order 28. Below 16 rows the chunk kernel is the better link of a chain of launches (13 rows of 28,672 in two
-// splits: gate/up 25.1 us against 24.1, the MLP around it 265 against 299). From 72 rows the clusters, two CTAs an SM, no
-// longer run all at once. Chunk or whole-row kernel against cluster, us, 28,672 columns in four splits (one for the norm):
-//   rows              16            31            64            72            96
-//   output          18.9 / 13.4   28.8 / 14.1   20.6 / 15.0   20.6 / 25.1   21.0 / 27.5
-//   gate/up         41.1 / 28.3   63.7 / 29.9   45.5 / 33.0   47.4 / 59.1   61.9 / 71.8
-//   input + norm    31.4 / 15.7   46.2 / 17.0   22.7 / 17.4   22.7 / 29.7   22.7 / 32.1
-// The same lines hold at 3,584, 7,168 and 14,336 columns. Order 12 has less to gain from reading a row once (gate/up at 64
-// rows 27.1 / 21.8, at 200 47.9 / 64.7) and keeps the two kernels.
+// Kernel of a transform by its row count and shape; `room`: longest row of the whole-row kernel. Lines between the three, from
+// their times (us; chunk / cluster of four / whole row, splits one and four):
+//  * The chunk kernel reads a row K times, a CTA of 1,024 threads an SM from P = 1,024 on: best while its K CTAs a row
+//    run at once (28,672 columns, five rows: output 3.4 / 4.5 / 10.7, gate/up 7.6 / 11.5 / 25.2; six rows 5.8 / 4.5 / 10.9
+//    and 13.8 / 11.5 / 25.4). Two rounds still beat the whole row (12,288 columns, 24 rows: output 4.1 / - / 5.4, four
+//    splits 6.4 / - / 6.3, gate/up 8.7 / - / 11.9), three do not (31 rows 5.5 / - / 5.2), nor two of long chunks (49,152
+//    columns, 13 rows 17.9 / - / 15.0).
+//  * A cluster for order 28 up to 64 rows, from 72 its CTAs no longer run all at once (28,672 columns, 64 rows: output 30.0 /
+//    7.2 / 11.1, gate/up 78.9 / 15.8 / 25.6; 72 rows 33.7 / 10.9 / 10.9 and 86.3 / 24.9 / 25.6). The input side is short
+//    of work and gains from a few rows on (14,336 columns, one row 5.4 / 3.8 / 6.6; 28,672: 4.1 / 4.5 / 11.3). Residual and
+//    gate/up have it wait for the state or carry a second area: 7,168 columns, 13 rows 7.4 / 6.8 / 5.2 and 9.2 / 12.4 /
+//    11.3, 14,336 columns 11.6 / 6.2 / 7.2 and 16.2 / 12.7 / 15.6, 57,344 columns, six rows 12.3 / 15.2 / 23.7.
+//  * A norm is taken by every CTA of a row, in the chunk and the row kernel (P = 1,024) from the loads of the transform itself:
+//    28,672 columns, five rows 6.3 / 15.9 / 11.3, six rows 11.5 / 15.9 / 11.5; 3,072 columns, one row 6.2 / - / 4.3.
+constexpr int kChunkRowsBelow = 32;  // fewer rows than this may be longer than the whole-row kernel's limit
 enum class Path { Chunk, Cluster, Row };
 template <int K>
 constexpr bool kHasCluster = K == 28;
 template <int K, bool T, Mode M>  // the input side transforms by the transposed factor, the output side by the factor
-constexpr bool kHasClusterMode = kHasCluster<K> && M != Mode::F32Inplace && T == kIsPrepare<M>;
-// Few splits are little to read 28 times, and the residual's read and write of the state is the cluster kernel's to wait for:
-// where the chunk kernel transforms in registers (P of 1,024 and 2,048) it stays faster for the residual (16 rows of 28,672 in
-// one split 11.2 / 15.2, two splits 14.0 / 16.0, three 16.7 / 16.8; of 57,344 in one split 23.3 / 26.4, in two 33.2 / 28.0), and
-// at P = 256, where up to 21 rows of its CTAs run at once, for residual and gate/up of one split (20 rows of 7,168: 7.6 / 7.9,
-// 10.8 / 11.6). The whole-row kernel has caught up in one split from 48 rows of 28,672 (50 rows: 16.7 / 17.2).
-static bool cluster_is_slower(Mode m, int P, int splits, long rows) {
-  if (m == Mode::FinishResidual && P == 1024 && splits == 1) return rows <= 28 || rows >= 48;
-  if (m == Mode::FinishResidual && P == 1024) return splits == 2 && rows <= 21;
-  if (m == Mode::FinishResidual && P == 2048) return splits == 1 && rows <= 21;
-  return (m == Mode::FinishResidual || m == Mode::FinishGateUp) && P == 256 && splits == 1 && rows <= 21;
+constexpr bool kHasClusterMode = kHasCluster<K> && M != Mode::F32Inplace && M != Mode::PrepareNorm && T == kIsPrepare<M>;
+static bool had_cluster_pays(Mode m, int P, int splits, long rows, bool one_round) {
+  switch (m) {
+    case Mode::Prepare: return P >= 128 && !(P == 1024 && one_round);
+    case Mode::FinishResidual: return P >= 512 && !one_round && (P <= 1024 || splits > 1 || rows > 12);
+    case Mode::FinishGateUp: return P >= 512 && !one_round && (P > 512 || rows > 8);
+    case Mode::Finish:
+    case Mode::FinishB16: return P >= 256 && (P == 512 || !one_round);
+    default: return false;
+  }
 }
 static Path had_path(Mode m, int K, int n, int P, int splits, long rows, int room) {
-  if (K == 28 && rows >= 16 && rows <= 64 && P % (4 * kHadCluster) == 0 && n <= room && !cluster_is_slower(m, P, splits, rows))
+  const bool chunk = K > 1 && P <= 8192, one_round = rows * K <= 148;
+  if (n > room && chunk && rows < kChunkRowsBelow) return Path::Chunk;  // longer rows than a CTA holds, a few at a time
+  if (m == Mode::PrepareNorm) return chunk && one_round && P >= (K == 28 ? 512 : 1024) ? Path::Chunk : Path::Row;
+  if (K == 28 && rows <= 64 && P % (4 * kHadCluster) == 0 && n <= room && had_cluster_pays(m, P, splits, rows, one_round))
     return Path::Cluster;
-  return K > 1 && rows < kChunkRowsBelow && P <= 8192 ? Path::Chunk : Path::Row;
+  if (m == Mode::FinishResidual && K == 28 && P == 256 && !one_round) return Path::Row;
+  return chunk && (P > 2048 ? one_round : rows * K <= 2 * 148) ? Path::Chunk : Path::Row;
 }
 // The kernels of a cluster are a link of the decode step's chain like the chunk kernels.
 template <typename... Params, typename... Args>
@@ -618,14 +802,34 @@ static int configure() {
     QB_CUDA(cudaFuncSetAttribute(had_cluster_kernel<K, T, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxRowFloats));
   return QTIP_OK;
 }
+// Rows that leave room for several CTAs per SM run with fewer threads per row once there are rows for every SM: the load,
+// transform and store phases of different rows then overlap on each SM. Measured on 12288-wide fp32 rows: 3.3 TB/s with
+// 1,024 threads (one row per SM), 4.2 with 512 (two), 4.7 with 256 (four).
+static int had_row_threads(long rows, size_t row_bytes, bool light) {
+  static const int forced = [] { const char* e = std::getenv("QTIP_HAD_ROW_THREADS"); return e ? std::atoi(e) : 0; }();
+  if (forced == 256 || forced == 512 || forced == 1024) return forced;
+  const size_t room = size_t(224) * 1024;
+  if (light && rows >= 4 * 148 && row_bytes * 4 <= room) return 256;
+  return rows >= 148 && row_bytes * 2 <= room ? 512 : 1024;
+}
+// Up to four rows an SM the kernel may start while the one in front of it drains; it lets the next one do so (row_chain) only with
+// few rows. us a pass, plain launch / this / with the release at every count: MLP at 13 tokens 309 / 304 / 305, at 64 tokens
+// 280 / 279 / 285, at 100 tokens (7,168 / 14,336 columns) 190 / 182 / 181, q/k/v at 40 tokens 118.6 / 114.9 / 118.1; the linear
+// of 28,672 x 12,288 at 200 tokens 158.2 / 155.9; no gain at 2,048 rows.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_row(void (*kernel)(Params...), long rows, int threads, size_t smem, cudaStream_t s, Args&&... args) {
+  if (rows <= 4 * 148) return launch_chained(kernel, dim3(unsigned(rows)), dim3(threads), smem, s, args...);
+  kernel<<<unsigned(rows), threads, smem, s>>>(args...);
+  return cudaGetLastError();
+}
 template <int K, bool T, Mode M>
 static int launch(const HadArgs& a, long rows, bool force_row, cudaStream_t s) {
   const int threads = a.P >= 1024 ? 1024 : (a.P < 64 ? 64 : a.P);
-  constexpr int kRoom = M == Mode::PrepareNorm ? kMaxRowFloats - 1024 : kMaxRowFloats;  // 4 KiB of static slots
+  constexpr int kRoom = M == Mode::PrepareNorm ? kMaxRowFloats - 1024 : kMaxRowFloats;  // the fused residual + input's limit
   const Path path = force_row ? Path::Row : had_path(M, K, a.n, a.P, a.splits, rows, kRoom);
   if constexpr (kHasClusterMode<K, T, M>)
     if (path == Path::Cluster) {
-      QB_CUDA(launch_cluster(had_cluster_kernel<K, T, M>, rows, size_t(a.n), s, a));
+      QB_CUDA(launch_cluster(had_cluster_kernel<K, T, M>, rows, size_t(had_room(K / kHadCluster, a.P)) * 4, s, a));
       return QTIP_OK;
     }
   if (path == Path::Chunk) {
@@ -635,18 +839,8 @@ static int launch(const HadArgs& a, long rows, bool force_row, cudaStream_t s) {
     QB_CUDA(launch_chained(had_chunk_kernel<K, T, M>, dim3(K, unsigned(rows)), dim3(threads), size_t(a.P) * 4, s, a));
   } else {
     QB_REQUIRE(a.n <= kRoom, QTIP_E_GEOMETRY, "Hadamard rows longer than %d are not supported (n = %d)", kRoom, a.n);
-    // Rows that leave room for several CTAs per SM run with fewer threads per row once there are rows for every SM:
-    // the load, transform and store phases of different rows then overlap on each SM. Measured on 12288-wide fp32 rows:
-    // 3.3 TB/s with 1,024 threads (one row per SM), 4.2 with 512 (two), 4.7 with 256 (four); the output transforms
-    // (several partial sums per element) and 28,672-wide rows are best with 512.
-    static const int forced = [] { const char* e = std::getenv("QTIP_HAD_ROW_THREADS"); return e ? std::atoi(e) : 0; }();
-    constexpr bool kLight = M == Mode::F32Inplace || M == Mode::Prepare;
-    const size_t row_bytes = size_t(a.n) * 4, room = size_t(224) * 1024;
-    int row_threads = 1024;
-    if (rows >= 148 && row_bytes * 2 <= room) row_threads = 512;
-    if (kLight && rows >= 4 * 148 && row_bytes * 4 <= room) row_threads = 256;
-    if (forced == 256 || forced == 512 || forced == 1024) row_threads = forced;
-    had_row_kernel<K, T, M><<<unsigned(rows), row_threads, size_t(a.n) * 4, s>>>(a);
+    const int row_threads = had_row_threads(rows, size_t(had_room(K, a.P)) * 4, M == Mode::F32Inplace || M == Mode::Prepare);
+    QB_CUDA(launch_row(had_row_kernel<K, T, M>, rows, row_threads, size_t(had_room(K, a.P)) * 4, s, a));
   }
   QB_LAUNCHED();
   return QTIP_OK;

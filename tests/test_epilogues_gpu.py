@@ -250,3 +250,42 @@ def test_rows_of_order_28_normalised_in_place(gpu, n, rows):
         lin.input_transform(x, norm, 1e-5, su, n, rows, u, xn)
         lin.input_transform(x, norm, 1e-5, su, n, rows, u2, x)
         assert torch.equal(x, xn) and torch.equal(u, u2)
+
+
+@pytest.mark.parametrize("n,rows", [(12288, 12), (12288, 13), (12288, 25), (12288, 150), (3072, 13), (3072, 25), (49152, 13),
+                                    (896, 11), (3584, 11), (7168, 6), (14336, 4), (14336, 9), (28672, 6), (28672, 65), (24576, 25)])
+@pytest.mark.parametrize("splits", [1, 3, 5])
+def test_stages_at_the_lines_between_kernels_match_single_rows(gpu, n, rows, splits):
+    """Row counts on both sides of the lines between the chunk, cluster and whole-row kernels, and K-splits on both sides of the
+    batched loads: each stage gives the bits of the same rows taken one at a time."""
+    lin, bits = gpu.linear, lambda t: t.view(torch.int16)  # noqa: E731
+    gen = torch.Generator(device="cuda").manual_seed(n + rows)
+    su, sv, sv2 = (torch.randint(0, 2, (n,), generator=gen, device="cuda").float() * 2 - 1 for _ in range(3))
+    x, norm = bf16_rows(rows, n, 5), (1 + 0.1 * torch.randn(n, generator=gen, device="cuda")).to(torch.bfloat16)
+    z = torch.randn(splits, rows, 2 * n, generator=gen, device="cuda")
+    half = z[:, :, :n].contiguous()
+    w = lin.Matrix(None, su, sv, None, n, n)
+
+    def stages(lo, hi):
+        r, out = hi - lo, {}
+        new = lambda: torch.empty(r, n, dtype=torch.bfloat16, device="cuda")  # noqa: E731
+        zs, xs = half[:, lo:hi].contiguous(), x[lo:hi].contiguous()
+        out["finish"], out["prepare"], out["u"], out["xn"] = new(), new(), new(), new()
+        lin.qtip_finish(w, zs, out["finish"], None, True, splits, r)
+        lin.qtip_prepare(w, xs, None, out["prepare"], r)
+        lin.input_transform(xs, norm, EPS, su, n, r, out["u"], out["xn"])
+        out["residual"] = xs.clone()
+        lin.output_residual(zs, splits, r, sv, n, out["residual"])
+        out["state"], out["next_u"] = xs.clone(), new()
+        lin.output_residual_input(zs, splits, r, sv, n, out["state"], norm, EPS, su, out["next_u"])
+        if 2 * n <= 57344:
+            out["h"] = new()
+            lin.output_gateup(z[:, lo:hi].contiguous(), splits, r, sv, sv2, n, out["h"])
+        return out
+
+    many = stages(0, rows)
+    for r in {0, rows // 2, rows - 1}:
+        one = stages(r, r + 1)
+        for key in many:
+            assert torch.equal(bits(many[key][r]), bits(one[key][0])), (key, r)
+    assert torch.equal(bits(many["residual"]), bits(many["state"]))

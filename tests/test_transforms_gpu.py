@@ -253,3 +253,19 @@ def test_rotate_hessian_as_one_call(gpu):
     a, ca = gpu.codec.rotate_hessian(dev(H), dev(su))
     b, cb = gpu.codec.rotate_hessian_fused(dev(H), dev(su))
     assert ca == cb and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n", [96, 256, 32, 64, 384, 512, 640, 896, 1536, 3072, 3584, 5120, 2048, 4096, 8192, 16384, 32768, 24576,
+                               40960, 49152])
+def test_hadamard_rows_of_every_chunk_length(gpu, oracle, n):
+    """Orders 1, 12, 20 and 28 with chunks from 8 to 32,768: units of 1,024 partly filled, whole, and several a chunk. Each value
+    is K - 1 + log2 P additions deep, each of at most half a unit in the last place (2^-24) of a partial sum, whose root mean
+    square is at most the result's."""
+    x = np.random.default_rng(n).standard_normal((3, n)).astype(np.float32)
+    K = next((k for k in (28, 20, 12) if n % k == 0 and (n // k) & (n // k - 1) == 0), 1)
+    bound = (K - 1 + np.log2(n // K) + 1) * 2.0 ** -24  # and the scale
+    for t in (0, 1):
+        X = dev(x)
+        gpu.codec.k_hadamard_rows(X, 3, n, n, t)
+        ref = oracle.hadamard_rows(x.astype(np.float64), bool(t))
+        assert np.linalg.norm(X.cpu().numpy() - ref) <= bound * np.linalg.norm(ref)
