@@ -369,6 +369,28 @@ def test_wide_batches_keep_their_partial_sums(gpu, n_in, n_out, tokens):
     assert torch.equal(z, z0)
 
 
+@pytest.mark.parametrize("n_in,n_out,splits,tokens", [(12288, 128, 1, 13), (12288, 16512, 2, 16), (3072, 20480, 4, 9),
+                                                      (128, 256, 1, 1), (384, 384, 3, 16), (640, 256, 2, 7)])
+def test_eight_chains_of_the_fused_product(gpu, n_in, n_out, splits, tokens):
+    """Up to 16 tokens the fused product adds each K-split in eight chains, one for each 16 columns of a 128-column step. A
+    step drops less than 2^-23 of its chain's running sum: the products stay within the length of a chain times half of that
+    of float64 on the decoded weights (one chain is 1.4e-5 off at 12,288 columns, the bound there 5.7e-6). From 9 tokens wide
+    matrices in several splits take it by themselves."""
+    w, *_ = make_linear(gpu, n_in, n_out, 900 + tokens)
+    x = torch.randn(tokens, n_in, generator=torch.Generator(device="cuda").manual_seed(n_in), device="cuda").to(torch.bfloat16)
+    z = torch.full((splits, tokens, n_out), float("nan"), device="cuda")
+    gpu.linear.qtip_multiply_tc(w, x, z, n_out, splits, tokens)
+    gpu.linear.kernel_status()
+    dense = torch.empty(n_out, n_in, dtype=torch.bfloat16, device="cuda")
+    gpu.linear.qtip_decode_matrix(w, dense)
+    ref = x.double() @ dense.double().T
+    assert float((z.double().sum(0) - ref).norm() / ref.norm()) < max(8, n_in // 128 / splits) * 2.0 ** -24
+    if tokens > 8 and n_in >= 3072:
+        own = torch.full_like(z, float("nan"))
+        gpu.linear.qtip_multiply_batch(w, x, own, n_out, splits, tokens)
+        assert torch.equal(own, z)
+
+
 @pytest.mark.parametrize("n_in,n_out,splits", [(128, 128, 2), (384, 256, 4), (384, 256, 6), (640, 384, 3), (896, 128, 7),
                                                (3584, 1536, 3), (128, 20480, 2)])
 def test_cuts_inside_a_step_of_the_fused_product(gpu, n_in, n_out, splits):
