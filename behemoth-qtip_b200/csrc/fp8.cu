@@ -1,7 +1,6 @@
 // W8A16 projection for the FP8 (e4m3, OCP "fn": 0x7f / 0xff are NaN) K/V weights that sit beside the QTIP linears of a
 // layer: y[t][o] = bf16( (sum_i fp8(w[o][i]) * bf16(x[t][i])) * scale[o] ), fp32 accumulation.
-// HBM-bound (one byte per weight): four warps share an output row, each lane streams 16 weights per 16-byte load (two
-// loads in flight), keeps one fp32 accumulator per token (up to 8 tokens per pass); shuffles and shared memory reduce.
+// One byte per weight from HBM, two per activation and CTA from the L2 (see fp8_gemv_kernel); up to 8 tokens per pass.
 #include <cuda_fp8.h>
 
 #include "common.cuh"
@@ -15,73 +14,91 @@ __device__ __forceinline__ float2 fp8x2_to_float2(uint16_t v) {
   return __half22float2(*reinterpret_cast<const __half2*>(&h));
 }
 
-// Four warps share a row (a quarter of K each), two rows per 256-thread CTA; partial sums meet in shared memory.
-constexpr int kFp8Split = 4;
-__global__ __launch_bounds__(256) void fp8_gemv_kernel(const uint8_t* __restrict__ w, const float* __restrict__ scale,
-                                                       const uint16_t* __restrict__ x, uint16_t* __restrict__ y, int in,
-                                                       int out, int tokens) {
-  __shared__ float part[8][kFp8Tokens];
+// A CTA owns four rows; its eight warps take every eighth run of 256 columns, eight columns a lane, for all four rows and NT
+// tokens, so that an activation is loaded and unpacked once for four rows. The weights of the next runs are on their way
+// meanwhile; partial sums meet in shared memory, in warp order. Two CTAs an SM: 1,024 rows are one round. Bound by latency
+// (a few runs a warp) and the multiply-adds. 1024 x 12288, 5 tokens: 17.8 us with two rows a CTA, four warps a row and the
+// activations loaded and unpacked anew for each row, now 7.
+constexpr int kFp8Rows = 4, kFp8Warps = 8, kFp8Ahead = 4;
+template <int NT>
+__global__ __launch_bounds__(32 * kFp8Warps, 2) void fp8_gemv_kernel(const uint8_t* __restrict__ w,
+                                                                     const float* __restrict__ scale,
+                                                                     const uint16_t* __restrict__ x, uint16_t* __restrict__ y,
+                                                                     int in, int out, int tokens) {
+  __shared__ float part[kFp8Warps][kFp8Rows * NT];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int row = blockIdx.x * 2 + (warp >> 2), quarter = warp & 3;
-  const int t0 = blockIdx.y * kFp8Tokens, nt = min(kFp8Tokens, tokens - t0);
-  float acc[kFp8Tokens];
+  // The last pass ends with the last token: where it overlaps the one before, both store the same bits.
+  const int row0 = blockIdx.x * kFp8Rows, t0 = min(int(blockIdx.y) * NT, tokens - NT);
+  float acc[kFp8Rows][NT];
 #pragma unroll
-  for (int t = 0; t < kFp8Tokens; ++t) acc[t] = 0.f;
+  for (int r = 0; r < kFp8Rows; ++r)
+#pragma unroll
+    for (int t = 0; t < NT; ++t) acc[r][t] = 0.f;
   chain_release();
   chain_wait();  // x may come from the kernel before this one, y may still be read by it
-  if (row < out) {
-    const int chunks = in / 16, c_lo = chunks * quarter / kFp8Split, c_hi = chunks * (quarter + 1) / kFp8Split;
-    const uint4* wr = reinterpret_cast<const uint4*>(w + size_t(row) * in);
-    for (int c0 = c_lo + lane; c0 < c_hi; c0 += 64) {
-      // two independent 16-byte weight loads in flight per lane
-      const int c1 = c0 + 32;
-      const uint4 wa = wr[c0];
-      const uint4 wb = c1 < c_hi ? wr[c1] : make_uint4(0, 0, 0, 0);
+  const int chunks = in / 8;  // of eight columns; in is a multiple of 16
+  const uint2* wr[kFp8Rows];
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const uint4 wv = half ? wb : wa;
-        const int c = half ? c1 : c0;
-        if (c >= c_hi) break;
-        const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
-        float wf[16];
+  for (int r = 0; r < kFp8Rows; ++r)  // rows past the end repeat the last one and are not stored
+    wr[r] = reinterpret_cast<const uint2*>(w + size_t(min(row0 + r, out - 1)) * in);
+  constexpr int kStep = 32 * kFp8Warps;
+  uint2 next[kFp8Ahead][kFp8Rows];
+  auto fetch = [&](uint2(&dst)[kFp8Rows], int c) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float2 a = fp8x2_to_float2(uint16_t(ww[q])), b = fp8x2_to_float2(uint16_t(ww[q] >> 16));
-          wf[4 * q] = a.x, wf[4 * q + 1] = a.y, wf[4 * q + 2] = b.x, wf[4 * q + 3] = b.y;
+    for (int r = 0; r < kFp8Rows; ++r) dst[r] = c < chunks ? wr[r][c] : make_uint2(0u, 0u);
+  };
+  const int c_first = warp * 32 + lane;
+#pragma unroll
+  for (int q = 0; q < kFp8Ahead; ++q) fetch(next[q], c_first + q * kStep);
+  for (int c0 = c_first; c0 < chunks; c0 += kFp8Ahead * kStep) {
+#pragma unroll
+    for (int q = 0; q < kFp8Ahead; ++q) {
+      const int c = c0 + q * kStep;
+      if (c >= chunks) break;
+      float wf[kFp8Rows][8];
+#pragma unroll
+      for (int r = 0; r < kFp8Rows; ++r) {
+        const uint32_t ww[2] = {next[q][r].x, next[q][r].y};
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          const float2 a = fp8x2_to_float2(uint16_t(ww[p])), b = fp8x2_to_float2(uint16_t(ww[p] >> 16));
+          wf[r][4 * p] = a.x, wf[r][4 * p + 1] = a.y, wf[r][4 * p + 2] = b.x, wf[r][4 * p + 3] = b.y;
         }
+      }
+      fetch(next[q], c + kFp8Ahead * kStep);
 #pragma unroll
-        for (int t = 0; t < kFp8Tokens; ++t) {
-          if (t < nt) {
-            const uint4* xr = reinterpret_cast<const uint4*>(x + size_t(t0 + t) * in) + 2 * c;
-            const uint4 x0 = __ldg(xr), x1 = __ldg(xr + 1);
-            const uint32_t xx[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+      for (int t = 0; t < NT; ++t) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(x + size_t(t0 + t) * in) + c);
+        const uint32_t xx[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              acc[t] = fmaf(wf[2 * q], __uint_as_float(xx[q] << 16), acc[t]);
-              acc[t] = fmaf(wf[2 * q + 1], __uint_as_float(xx[q] & 0xffff0000u), acc[t]);
-            }
-          }
+        for (int k = 0; k < 4; ++k) {
+          const float lo = __uint_as_float(xx[k] << 16), hi = __uint_as_float(xx[k] & 0xffff0000u);
+#pragma unroll
+          for (int r = 0; r < kFp8Rows; ++r) acc[r][t] = fmaf(wf[r][2 * k + 1], hi, fmaf(wf[r][2 * k], lo, acc[r][t]));
         }
       }
     }
   }
 #pragma unroll
-  for (int t = 0; t < kFp8Tokens; ++t) {
-    float s = acc[t];
+  for (int r = 0; r < kFp8Rows; ++r)
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (lane == 0) part[warp][t] = s;
-  }
+    for (int t = 0; t < NT; ++t) {
+      float s = acc[r][t];
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+      if (lane == 0) part[warp][r * NT + t] = s;
+    }
   __syncthreads();
-  if (threadIdx.x < 2 * kFp8Tokens) {
-    const int r = threadIdx.x / kFp8Tokens, t = threadIdx.x % kFp8Tokens, orow = blockIdx.x * 2 + r;
-    if (orow < out && t < nt) {
-      const float s = ((part[4 * r][t] + part[4 * r + 1][t]) + part[4 * r + 2][t]) + part[4 * r + 3][t];
-      y[size_t(t0 + t) * out + orow] = f32_to_bf16(s * scale[orow]);
+  if (threadIdx.x < kFp8Rows * NT) {
+    const int row = row0 + threadIdx.x / NT, t = threadIdx.x % NT;
+    if (row < out) {
+      float s = part[0][threadIdx.x];
+#pragma unroll
+      for (int q = 1; q < kFp8Warps; ++q) s += part[q][threadIdx.x];
+      y[size_t(t0 + t) * out + row] = f32_to_bf16(s * scale[row]);
     }
   }
 }
-
 // Exact bf16 value of every e4m3 byte (e4m3 has 3 mantissa bits: bf16 holds it exactly); 16 bytes per thread.
 __global__ void fp8_to_bf16_kernel(const uint8_t* __restrict__ in, uint16_t* __restrict__ out, size_t n16) {
   const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -117,9 +134,25 @@ extern "C" int qtip_fp8_forward(const uint8_t* w_d, const float* scale_d, const 
                                 int out, int tokens, void* stream) {
   QB_REQUIRE(w_d && scale_d && x_d && y_d && tokens >= 1, QTIP_E_ARG, "qtip_fp8_forward: bad argument");
   QB_REQUIRE(in > 0 && out > 0 && in % 16 == 0, QTIP_E_GEOMETRY, "qtip_fp8_forward: in = %d must be a multiple of 16", in);
-  const dim3 grid(blocks_for(out, 2), blocks_for(tokens, kFp8Tokens));
-  QB_REQUIRE(grid.y <= 65535, QTIP_E_GEOMETRY, "qtip_fp8_forward: too many tokens (%d)", tokens);
-  QB_CUDA(launch_chained(fp8_gemv_kernel, grid, dim3(256), 0, as_stream(stream), w_d, scale_d, x_d, y_d, in, out, tokens));
+  // Passes of even size in one launch
+  const unsigned passes = blocks_for(tokens, kFp8Tokens);
+  QB_REQUIRE(passes <= 65535, QTIP_E_GEOMETRY, "qtip_fp8_forward: too many tokens (%d)", tokens);
+  const dim3 grid(blocks_for(out, kFp8Rows), passes), block(32 * kFp8Warps);
+#define QB_FP8(NT_)                                                                                                     \
+  case NT_:                                                                                                             \
+    QB_CUDA(launch_chained(fp8_gemv_kernel<NT_>, grid, block, 0, as_stream(stream), w_d, scale_d, x_d, y_d, in, out, tokens)); \
+    break
+  switch ((tokens + passes - 1) / passes) {
+    QB_FP8(1);
+    QB_FP8(2);
+    QB_FP8(3);
+    QB_FP8(4);
+    QB_FP8(5);
+    QB_FP8(6);
+    QB_FP8(7);
+    QB_FP8(8);
+  }
+#undef QB_FP8
   QB_LAUNCHED();
   return QTIP_OK;
 }

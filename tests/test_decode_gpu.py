@@ -369,6 +369,25 @@ def test_wide_batches_keep_their_partial_sums(gpu, n_in, n_out, tokens):
     assert torch.equal(z, z0)
 
 
+@pytest.mark.parametrize("n_in,n_out,tokens", [(16, 1, 1), (256, 5, 2), (2064, 6, 3), (8192, 7, 9), (8208, 130, 12),
+                                               (12288, 64, 6), (1040, 3, 17), (4096, 33, 8)])
+def test_fp8_rows_runs_and_passes(gpu, n_in, n_out, tokens):
+    """Rows that are no multiple of a CTA's four, columns around the eight warps' runs of 256 and the four runs in flight,
+    tokens around a pass. A lane adds n_in / 2048 runs of eight products, then 5 + 8 partial sums: fp32 is that many halves
+    of 2^-23 off the sum of magnitudes at most, beside one bf16 rounding of the result."""
+    gen = torch.Generator(device="cuda").manual_seed(n_in + tokens)
+    w = torch.randint(0, 256, (n_out, n_in), generator=gen, device="cuda", dtype=torch.uint8)
+    w[(w & 127) == 127] = 0  # no NaN codes
+    scale = torch.rand(n_out, generator=gen, device="cuda") + 0.5
+    x = torch.randn(tokens, n_in, generator=gen, device="cuda").to(torch.bfloat16)
+    y = torch.full((tokens, n_out), float("nan"), dtype=torch.bfloat16, device="cuda")
+    gpu.linear.fp8_forward(w, scale, x, y, n_in, n_out, tokens)
+    wd = w.view(torch.float8_e4m3fn).double()
+    ref, size = (x.double() @ wd.T) * scale.double(), (x.double().abs() @ wd.abs().T) * scale.double()
+    bound = (8 * (n_in // 2048 + 1) + 13 + 1) * 2.0 ** -24 * size + 2.0 ** -8 * ref.abs()
+    assert bool(((y.double() - ref).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("n_in,n_out,splits,tokens", [(12288, 128, 1, 13), (12288, 16512, 2, 16), (3072, 20480, 4, 9),
                                                       (128, 256, 1, 1), (384, 384, 3, 16), (640, 256, 2, 7)])
 def test_eight_chains_of_the_fused_product(gpu, n_in, n_out, splits, tokens):
