@@ -14,27 +14,27 @@ kSeq, kSteps, kWordsPerTrellis = 256, 128, 32
 _initialised = set()
 
 
+# A one-token linear is 11 us of kernels: torch.cuda's wrappers of the two look-ups below (3 to 5 us together, for lazy
+# initialisation, device arguments and stream objects) and pointer objects would be a third of its host time.
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def init():
     """Per-device set-up (qtip_init) for the current device; idempotent."""
-    dev = torch.cuda.current_device()
+    dev = torch._C._cuda_getDevice() if _initialised else torch.cuda.current_device()  # the first call initialises CUDA
     if dev not in _initialised:
         lib().call("qtip_init")
         _initialised.add(dev)
 
 
 def _p(t, dtype=None):
-    if t is None:
-        return None
-    if isinstance(t, int):  # a raw device address (a slot of a tensor-parallel exchange buffer)
-        return C.c_void_p(t)
+    if t is None or isinstance(t, int):  # a raw device address (a slot of a tensor-parallel exchange buffer)
+        return t
     assert t.is_cuda and t.is_contiguous(), "device-resident contiguous tensor expected"
     if dtype is not None:
         assert t.dtype == dtype, "expected %s, got %s" % (dtype, t.dtype)
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def device_lut(tlut_f16):
