@@ -47,101 +47,151 @@ __global__ void ldl_symmetrise_kernel(const float* __restrict__ H, double* __res
   }
 }
 
-// Cholesky of a kb x kb block (kb a multiple of 16, at most 128) in shared memory, packed lower triangle, by 256 threads. Sixteen
+__device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+// Cholesky of a kb x kb block (kb a multiple of 16, at most 128) in shared memory, packed lower triangle, by eight warps. Sixteen
 // columns at a time: one warp factors the 16 x 16 diagonal block with a row per lane in registers and inverts it (a column
-// per lane), then all warps take the rows below it through the inverse and update what is right of it. The inverses, which
-// the panel kernel and the final block scaling need as well, go to `inv` (256 values a block, row-major, zeros above the
-// diagonal).
+// per lane), then all warps take the rows below it through the inverse, a 16 x 16 block a warp on the fp64 tensor cores. What
+// is right of them is updated by warps 1 to 7 while warp 0 updates, factors and inverts the next diagonal block. The
+// inverses, which the panel kernel and the final block scaling need as well, go to `inv` (256 values a block, row-major,
+// zeros above the diagonal).
+// Bound by latency: the square roots of the pivots, one after another. 48 us a block of 128 where it was 127 (inverse 69,000, by
+// divisions that each wait for the one before; factor 47,000; trailing updates 34,000 and the rows 19,000 in scalar
+// multiply-adds behind the factor; the block's way in and out of shared memory, an element a thread at a time, the rest of
+// 221,000 cycles). It is the floor of an update: 138 -> 70 us, which half of the panels of n = 12,288 and all of n = 4,096 met.
 constexpr int kLd = kNb + 1;  // L11 in the panel kernel
 constexpr int kInvLd = 17;
 __device__ __forceinline__ int tri(int i) { return i * (i + 1) / 2; }  // first word of row i of a packed lower triangle
+
+// c (2 x 2 fragments of 8 x 8) += x y^T over 16 columns; x(i, p) and y(j, p) read element p of row i / j of the two blocks.
+template <typename X, typename Y>
+__device__ __forceinline__ void chol_block_product(double (&c)[2][2][2], X x, Y y) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+#pragma unroll
+  for (int p = 0; p < 16; p += 4) {
+    const double a[2] = {x(g, p + q), x(g + 8, p + q)}, b[2] = {y(g, p + q), y(g + 8, p + q)};
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) dmma_8x8x4(c[i][j], a[i], b[j]);
+  }
+}
+// Block (ra, rb) of 16 x 16 (rb <= ra): minus the product of the two row blocks' columns base .. base + 15. One warp.
+__device__ __forceinline__ void chol_block_update(double* __restrict__ S, int ra, int rb, int base) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  double c[2][2][2] = {};
+  chol_block_product(c, [&](int i, int p) { return S[tri(ra + i) + base + p]; },
+                     [&](int j, int p) { return S[tri(rb + j) + base + p]; });
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = ra + 8 * i + g, col = rb + 8 * j + 2 * q + h;
+        if (col <= r) S[tri(r) + col] -= c[i][j][h];
+      }
+}
+// The 16 x 16 diagonal block at `base` and its inverse, by one warp.
+__device__ __forceinline__ void chol_factor16(double* __restrict__ S, double* __restrict__ inv_s, int base,
+                                              double* __restrict__ inv, int* status) {
+  const int lane = threadIdx.x & 31, i = lane & 15;
+  double a[16], own = 1.0;  // own: one over the diagonal element of the lane's row
+#pragma unroll
+  for (int c = 0; c < 16; ++c) a[c] = c <= i ? S[tri(base + i) + base + c] : 0.0;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const double d = __shfl_sync(0xffffffffu, a[j], j);
+    const bool ok = d > 0.0;
+    if (!ok && lane == 0) atomicOr(status, 1);
+    // a failed pivot is reported; the factor is then meaningless but finite
+    const double dj = ok ? sqrt(d) : 1.0, rj = 1.0 / dj;
+    if (i == j) own = rj;
+    a[j] = i == j ? dj : a[j] * rj;
+#pragma unroll
+    for (int c = j + 1; c < 16; ++c) a[c] = fma(-a[j], __shfl_sync(0xffffffffu, a[j], c), a[c]);
+  }
+  double col[16];  // column i of the inverse
+#pragma unroll
+  for (int r = 0; r < 16; ++r) {
+    double t = r == i ? 1.0 : 0.0;
+#pragma unroll
+    for (int q = 0; q < 16; ++q)
+      if (q < r) t = fma(-__shfl_sync(0xffffffffu, a[q], r), col[q], t);
+    col[r] = t * __shfl_sync(0xffffffffu, own, r);
+  }
+  if (lane < 16) {
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      if (c <= i) S[tri(base + i) + base + c] = a[c];
+      inv_s[c * kInvLd + i] = col[c];
+      inv[(base / 16) * 256 + c * 16 + i] = col[c];
+    }
+  }
+}
 __device__ __forceinline__ void chol_factor(double* __restrict__ S, double* __restrict__ inv_s, int kb,
                                             double* __restrict__ inv, int* status) {
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  for (int base = 0; base < kb; base += 16) {
-    if (tid < 32) {
-      const int i = tid & 15;
-      double a[16];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  if (warp == 0) chol_factor16(S, inv_s, 0, inv, status);
+  __syncthreads();
+  for (int base = 0; base + 16 < kb; base += 16) {
+    const int next = base + 16, blocks = (kb - next) / 16;
+    if (warp < blocks) {  // rows below: x = a inv^T, in place (the warp has read its rows before it writes them)
+      const int r0 = next + 16 * warp;
+      double c[2][2][2] = {};
+      chol_block_product(c, [&](int i, int p) { return S[tri(r0 + i) + base + p]; },
+                         [&](int j, int p) { return inv_s[j * kInvLd + p]; });
+      __syncwarp();
 #pragma unroll
-      for (int c = 0; c < 16; ++c) a[c] = c <= i ? S[tri(base + i) + base + c] : 0.0;
+      for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const double d = __shfl_sync(0xffffffffu, a[j], j);
-        const bool ok = d > 0.0;
-        if (!ok && tid == 0) atomicOr(status, 1);
-        const double dj = ok ? sqrt(d) : 1.0;  // a failed pivot is reported; the factor is then meaningless but finite
-        a[j] = i == j ? dj : a[j] / dj;
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int c = j + 1; c < 16; ++c) a[c] = fma(-a[j], __shfl_sync(0xffffffffu, a[j], c), a[c]);
-      }
-      double col[16];  // column i of the inverse
-#pragma unroll
-      for (int r = 0; r < 16; ++r) {
-        double t = r == i ? 1.0 : 0.0;
-#pragma unroll
-        for (int q = 0; q < 16; ++q)
-          if (q < r) t = fma(-__shfl_sync(0xffffffffu, a[q], r), col[q], t);
-        col[r] = t / __shfl_sync(0xffffffffu, a[r], r);
-      }
-      if (tid < 16) {
-#pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          if (c <= i) S[tri(base + i) + base + c] = a[c];
-          inv_s[c * kInvLd + i] = col[c];
-          inv[(base / 16) * 256 + c * 16 + i] = col[c];
-        }
-      }
+          for (int h = 0; h < 2; ++h) S[tri(r0 + 8 * i + g) + base + 8 * j + 2 * q + h] = c[i][j][h];
     }
     __syncthreads();
-    // rows below: x = a inv^T
-    const int below = kb - base - 16;
-    double x[7];
-#pragma unroll
-    for (int a = 0; a < 7; ++a) {
-      const int r = ty + 16 * a;
-      double t = 0.0;
-      if (r < below) {
-#pragma unroll
-        for (int p = 0; p < 16; ++p) t = fma(S[tri(base + 16 + r) + base + p], inv_s[tx * kInvLd + p], t);
-      }
-      x[a] = t;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int a = 0; a < 7; ++a)
-      if (ty + 16 * a < below) S[tri(base + 16 + ty + 16 * a) + base + tx] = x[a];
-    __syncthreads();
-    // right of it: a[i][c] -= sum_p x[i][p] x[c][p], 16 x 16 blocks on and below the diagonal
-    for (int a = 0; 16 * a < below; ++a) {
-      double* row = S + tri(base + 16 + ty + 16 * a) + base;
-      double xi[16];
-#pragma unroll
-      for (int p = 0; p < 16; ++p) xi[p] = row[p];
-      for (int b = 0; b <= a; ++b) {
-        const double* xc = S + tri(base + 16 + tx + 16 * b) + base;
-        double t0 = 0.0, t1 = 0.0;
-#pragma unroll
-        for (int p = 0; p < 16; p += 2) t0 = fma(xi[p], xc[p], t0), t1 = fma(xi[p + 1], xc[p + 1], t1);
-        if (b < a || tx <= ty) row[16 + tx + 16 * b] -= t0 + t1;
-      }
+    if (warp == 0) {
+      chol_block_update(S, next, next, base);
+      __syncwarp();
+      chol_factor16(S, inv_s, next, inv, status);
+    } else {
+      int at = 0;  // the other blocks, dealt to warps 1 .. 7
+      for (int ra = 1; ra < blocks; ++ra)
+        for (int rb = 0; rb <= ra; ++rb, ++at)
+          if (at % 7 == warp - 1) chol_block_update(S, next + 16 * ra, next + 16 * rb, base);
     }
     __syncthreads();
   }
 }
-// The diagonal block at (k, k): loaded, factored, stored by a CTA of 256 threads.
+// The diagonal block at (k, k): loaded, factored, stored by a CTA of 256 threads, a row a warp, four rows in flight.
 __device__ __forceinline__ void chol_diagonal(double* __restrict__ A, long n, long k, double* __restrict__ sm,
                                               double* __restrict__ inv, int* status) {
-  const int kb = int(min(long(kNb), n - k));
-  for (int idx = threadIdx.x; idx < kb * kb; idx += blockDim.x) {
-    const int i = idx / kb, j = idx - i * kb;
-    if (j <= i) sm[tri(i) + j] = A[(k + i) * n + k + j];
+  const int kb = int(min(long(kNb), n - k)), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i0 = warp; i0 < kb; i0 += 32) {
+    double v[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int i = i0 + 8 * r, j = lane + 32 * c;
+        v[r][c] = i < kb && j <= i ? A[(k + i) * n + k + j] : 0.0;
+      }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int i = i0 + 8 * r, j = lane + 32 * c;
+        if (i < kb && j <= i) sm[tri(i) + j] = v[r][c];
+      }
   }
   __syncthreads();
   chol_factor(sm, sm + tri(kNb), kb, inv, status);
-  for (int idx = threadIdx.x; idx < kb * kb; idx += blockDim.x) {
-    const int i = idx / kb, j = idx - i * kb;
-    if (j <= i) A[(k + i) * n + k + j] = sm[tri(i) + j];
-  }
+  for (int i = warp; i < kb; i += 8)
+    for (int j = lane; j <= i; j += 32) A[(k + i) * n + k + j] = sm[tri(i) + j];
 }
 __global__ __launch_bounds__(256) void chol_first_kernel(double* __restrict__ A, long n, double* __restrict__ inv,
                                                          int* status) {
@@ -210,15 +260,11 @@ __global__ __launch_bounds__(256) void chol_panel_kernel(double* __restrict__ A,
 // (m8n8k4). The two operand panels pass through a ring of 16-column slices (cp.async; row stride 20 doubles: the 4 x 4
 // words that a half-warp reads for a fragment lie in 16 different bank pairs). Two CTAs share an SM, so that one reads and
 // writes its part of C while the other multiplies. n = 12,288, all updates: 66 ms with scalar multiply-adds and 8 x 8
-// outputs a thread, 29.9 ms with fragments and one 128 x 128 tile per SM, 27.2 ms so (the fp64 rate gives 16.6).
+// outputs a thread, 29.9 ms with fragments and one 128 x 128 tile per SM, 27.2 ms so, 23.5 ms since the factorisation of the
+// next diagonal block is shorter than most updates (the fp64 rate gives 16.6).
 // Tile row ti has 2 ti + 2 tiles. The first CTA takes both tiles of the next diagonal block and factors it at once.
 constexpr int kTileCols = 64, kSliceLd = kKc + 4, kSlices = kNb / kKc, kUpdThreads = 256, kUpdStages = 3;
 constexpr int kStageDoubles = (kTile + kTileCols) * kSliceLd;
-__device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
 __device__ __forceinline__ void chol_update_tile(double* __restrict__ A, long n, long k, long i0, long j0, double* sm) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   const int wi = (warp >> 1) * 32, wj = (warp & 1) * 32;
