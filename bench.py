@@ -321,7 +321,7 @@ def main():
     gen.manual_seed(2 + 1000003 * b)
     W = torch.randn((e - b) * 16, N_COLS, generator=gen, device="cuda", dtype=torch.float32)
     X = codec.tiles_from_matrix(W)
-    chunk = 4608  # sequences per forward launch; the workspace holds two chunks, which alternate between two streams
+    chunk = 4608  # sequences of the launches that are timed by themselves (the passes with back-pointers)
     ws = codec.quantize_workspace(2 * chunk)
     states = torch.empty((tiles_local, 128), dtype=torch.int16, device="cuda")
     torch.cuda.synchronize()
@@ -381,7 +381,8 @@ def main():
     sm_count = torch.cuda.get_device_properties(local).multi_processor_count
     peak_ops = sm_count * 128 * peaks.get("sm_max_mhz", 1965.0) * 1e6
     achieved = lane_ops / (kern_ms * 1e-3)
-    launches_per_step = 4 * ((tiles_local + chunk - 1) // chunk)
+    fused_chunk = 4 * 33 * 8  # sequences per launch of the fused path: four full rounds of its 33 resident clusters of four
+    launches_per_step = 4 * ((tiles_local + fused_chunk - 1) // fused_chunk)
 
     # ---- end to end through the C ABI with host buffers: H2D of the fp32 matrix, tile gather, two-pass Viterbi, pack,
     # kernel-layout swizzle, D2H of the trellis words. Rank 0's share at N > 1 (every rank does the same on its rows).
@@ -445,10 +446,12 @@ def main():
                        "l2": ("inputs (%.0f MB per rank) exceed the 126 MB L2" % (tiles_local * 1024 / 1e6)) if flush is None
                        else ("inputs are %.0f MB per rank: a 256 MB buffer is overwritten between steps to flush the L2"
                              % (tiles_local * 1024 / 1e6)),
-                       "sharding": "contiguous tile rows per rank, no collective", "chunk_tiles": chunk,
-                       "chunks_in_flight": 2 if tiles_local > chunk else 1},
+                       "sharding": "contiguous tile rows per rank, no collective", "chunk_tiles": fused_chunk,
+                       "chunks_in_flight": 2 if tiles_local > fused_chunk else 1},
             "clocks": clocks, "e2e": e2e, "gpu_launches": launches_per_step * args.steps,
-            "roofline": {"bound": "fp32_issue", "kernel": "vit_fwd_cluster_kernel", "achieved": achieved / 1e12,
+            "roofline": {"bound": "fp32_issue", "kernel": "vit_fwd_cluster_kernel",
+                         "kernel_note": "the pass with back-pointers, timed by itself; the step runs vit_fwd_minima_kernel",
+                         "achieved": achieved / 1e12,
                          "peak": peak_ops / 1e12, "unit": "Tlane-op/s", "frac": achieved / peak_ops,
                          "peak_source": "%d SMs x 128 lanes x sm_max_mhz of MEASURED_PEAKS.json (%s)" % (sm_count, peak_src),
                          "ms_per_launch": kern_ms, "tiles_per_launch": nb,
